@@ -153,16 +153,38 @@ def _as_tensor(buf, shape):
     return torch.as_tensor(_Foreign(buf, shape), device="cuda").view(torch.bfloat16)
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """Every input of a case, as torch tensors on the GPU."""
     gen = torch.Generator(device="cuda")
     gen.manual_seed(int(seed))
+    if case["kind"] == "linear":
+        M, N, K = case["tokens"], case["rows"], case["columns"]
+        return dict(w=_weights(gen, case["format"], N, K), x=_normal(gen, (M, K), DTYPES[case["x"]][1]))
+    M, H, I = case["tokens"], case["hidden"], case["inner"]
+    if case["kind"] == "stack":
+        layers = []
+        for _ in range(case["layers"]):
+            w = [_weights(gen, "Q4_K", n, k) for n, k in _stack_shapes(case)]
+            layers.append((w, (0.9 + 0.2 * torch.rand(H, generator=gen, device="cuda")).bfloat16()))
+        return dict(layers=layers, x=_normal(gen, (M, H), torch.bfloat16))
+    E = case["experts"]
+    return dict(w13=_weights(gen, "Q4_K", E * 2 * I, H), w2=_weights(gen, "Q4_K", E * H, I),
+                x=_normal(gen, (M, H), torch.bfloat16), logits=_normal(gen, (M, E), torch.bfloat16))
+
+
+def _stack_shapes(case):
+    H, I, h, kv = case["hidden"], case["inner"], case["heads"], case["kv_heads"]
+    return [((h + 2 * kv) * 128, H), (H, h * 128), (2 * I, H), (H, I)]
+
+
+def prepare(case, seed):
     dev = _dev()
     st = dict(case=case, dev=dev)
+    made = _inputs(case, seed)
     if case["kind"] == "linear":
         M, N, K = case["tokens"], case["rows"], case["columns"]
         tag, (xd, xt), (yd, yt) = FORMATS[case["format"]][0], DTYPES[case["x"]], DTYPES[case["y"]]
-        st["w"] = _weights(gen, case["format"], N, K)
-        st["x"] = _normal(gen, (M, K), xt)
+        st["w"], st["x"] = made["w"], made["x"]
         st["y"] = torch.empty((M, N), dtype=yt, device="cuda")
         ws_bytes = ub.lib().ub_qmatmul_gguf_workspace_bytes(tag, M, N, K)
         if case["format"] == "Q8_0":
@@ -173,20 +195,18 @@ def prepare(case, seed):
     elif case["kind"] == "stack":
         M, H, I, h, kv = case["tokens"], case["hidden"], case["inner"], case["heads"], case["kv_heads"]
         st["layers"], st["gammas"] = [], []
-        for _ in range(case["layers"]):
-            shapes = [((h + 2 * kv) * 128, H), (H, h * 128), (2 * I, H), (H, I)]
-            w = [_resident(dev, _weights(gen, "Q4_K", n, k)) for n, k in shapes]
+        for packed, gamma in made["layers"]:
+            w = [_resident(dev, t) for t in packed]
             st["layers"].append(parallel.TPLinearStack(dev, H, I, h, kv, 128, 1, w[0], w[1], w[2], w[3], M))
-            st["gammas"].append(_resident(dev, (0.9 + 0.2 * torch.rand(H, generator=gen, device="cuda")).bfloat16()))
-        st["x"] = _resident(dev, _normal(gen, (M, H), torch.bfloat16))
+            st["gammas"].append(_resident(dev, gamma))
+        st["x"] = _resident(dev, made["x"])
         st["normed"] = dev.alloc(M * H * 2)
         st["y"] = _as_tensor(st["layers"][-1].out, (M, H))
     else:
         T, H, I, E = case["tokens"], case["hidden"], case["inner"], case["experts"]
-        w13, w2 = _weights(gen, "Q4_K", E * 2 * I, H), _weights(gen, "Q4_K", E * H, I)
-        st["layer"] = parallel.EPMoELayer(dev, T, H, I, E, case["top_k"], 64, 0, 1, _resident(dev, w13), _resident(dev, w2))
-        st["x"] = _resident(dev, _normal(gen, (T, H), torch.bfloat16))
-        st["logits"] = _resident(dev, _normal(gen, (T, E), torch.bfloat16))
+        w13, w2 = _resident(dev, made["w13"]), _resident(dev, made["w2"])
+        st["layer"] = parallel.EPMoELayer(dev, T, H, I, E, case["top_k"], 64, 0, 1, w13, w2)
+        st["x"], st["logits"] = _resident(dev, made["x"]), _resident(dev, made["logits"])
         st["y"] = _as_tensor(st["layer"].out, (T, H))
     # the inputs were made on torch's stream, the framework's calls go to the device's own
     torch.cuda.current_stream().synchronize()
@@ -248,3 +268,82 @@ def tolerance(case):
     if case["format"] in ("Q4_K", "Q8_0") and case["tokens"] > 8:
         return {"rel": 2e-2}
     return {"rel": 7e-3 if case["y"] == "bf16" else 1e-4}
+
+
+# --------------------------------------------------------------------------------------------------- 64-bit results
+def _f16(b, at):
+    return b[:, at:at + 2].contiguous().view(torch.float16).double()
+
+
+def _values(fmt, packed):
+    """Packed blocks as f64 values [blocks, values per block]."""
+    _, per, size = FORMATS[fmt]
+    b = packed.view(-1, size)
+    d = _f16(b, 208 if fmt == "Q6_K" else 0)
+    if fmt == "Q8_0":
+        return d * b[:, 2:].contiguous().view(torch.int8).double()
+    if fmt == "Q4_0":
+        q = b[:, 2:]
+        return d * (torch.cat([q & 15, q >> 4], 1).double() - 8)
+    if fmt == "Q6_K":
+        sc = b[:, 192:208].contiguous().view(torch.int8).double().repeat_interleave(16, 1)
+        q = []
+        for half in range(2):
+            lo, hi = b[:, 64 * half:64 * half + 64], b[:, 128 + 32 * half:160 + 32 * half]
+            for part in range(4):
+                nibble = lo[:, 32 * (part & 1):32 * (part & 1) + 32] >> (4 * (part >> 1)) & 15
+                q.append(nibble | (hi >> (2 * part) & 3) << 4)
+        return d * sc * (torch.cat(q, 1).double() - 32)
+    s, dmin = b[:, 4:16], _f16(b, 2)
+    sc = torch.cat([s[:, :4] & 63, s[:, 8:] & 15 | s[:, :4] >> 6 << 4], 1).double().repeat_interleave(32, 1)
+    mn = torch.cat([s[:, 4:8] & 63, s[:, 8:] >> 4 | s[:, 4:8] >> 6 << 4], 1).double().repeat_interleave(32, 1)
+    q4 = b[:, size - 128:]
+    q = []
+    for sub in range(8):
+        v = q4[:, 32 * (sub // 2):32 * (sub // 2) + 32] >> (4 * (sub & 1)) & 15
+        if fmt == "Q5_K":
+            v = v | (b[:, 16:48] >> sub & 1) << 4
+        q.append(v)
+    return d * sc * torch.cat(q, 1).double() - dmin * mn
+
+
+def _linear64(x, fmt, packed, rows):
+    """x . W^T in f64, W taken a slice of rows at a time."""
+    _, per, size = FORMATS[fmt]
+    K = x.shape[1]
+    w = packed.view(rows, K // per * size)
+    step = max(1, (1 << 26) // K)
+    return torch.cat([x @ _values(fmt, w[r:r + step].reshape(-1)).view(-1, K).T for r in range(0, rows, step)], 1)
+
+
+def _silu_up64(gu, I):
+    return torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+
+
+def exact(case, seed):
+    made = _inputs(case, seed)
+    x = made["x"].double()
+    if case["kind"] == "linear":
+        return _linear64(x, case["format"], made["w"], case["rows"])
+    H, I = case["hidden"], case["inner"]
+    if case["kind"] == "stack":
+        for w, gamma in made["layers"]:
+            x = x * torch.rsqrt(x.square().mean(1, keepdim=True) + 1e-5) * gamma.double()
+            for i, (packed, (rows, _)) in enumerate(zip(w, _stack_shapes(case))):
+                x = _linear64(x, "Q4_K", packed, rows)
+                if i == 0:
+                    x = x[:, :case["heads"] * 128]
+                elif i == 2:
+                    x = _silu_up64(x, I)
+        return x
+    E, k = case["experts"], case["top_k"]
+    p, chosen = torch.softmax(made["logits"].double(), 1).sort(dim=1, descending=True, stable=True)  # ties: lowest
+    p, chosen = p[:, :k] / p[:, :k].sum(1, keepdim=True), chosen[:, :k]
+    w13, w2 = made["w13"].view(E, -1), made["w2"].view(E, -1)
+    y = torch.zeros_like(x)
+    for e in range(E):
+        t, slot = (chosen == e).nonzero(as_tuple=True)
+        if len(t):
+            act = _silu_up64(_linear64(x[t], "Q4_K", w13[e], 2 * I), I)
+            y.index_add_(0, t, p[t, slot, None] * _linear64(act, "Q4_K", w2[e], H))
+    return y
