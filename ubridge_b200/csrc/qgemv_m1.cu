@@ -36,6 +36,8 @@
 
 #include <string.h>
 
+#include <type_traits>
+
 #include "ar_epilogue.cuh"
 #include "common.cuh"
 
@@ -521,7 +523,7 @@ int launch_m1(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype
 
 
 // =====================================================================================================
-// The same kernel for longer rows (K a multiple of 2048: the 8192-wide projections of a 70B-shaped stack in one
+// The same kernel for other rows (K a multiple of 256: the 8192-wide projections of a 70B-shaped stack in one
 // pass, its 28672-wide down projection in four).  A stage is 16 rows x 8 super-blocks (18 KB), a tile takes K / 2048 stages and warp w owns
 // super-block 8c + w of every stage c.  The activation fragments no longer fit the register file: each warp
 // writes those of its own super-blocks to shared memory once per launch (one word per MMA and lane: the
@@ -531,18 +533,63 @@ int launch_m1(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype
 constexpr int kFragBytesPerSb = 1024 + 48;  // 8 words x 32 lanes, then {S_t, S_4+t} x 4 and the block scale
 constexpr int kMaxChunks = 6;
 
+// Rows that are not whole 128-byte lines (ODD: K a multiple of 256, not of 2048) cannot be viewed as lines and
+// swizzled.  Their stage is four boxes of [16 rows][288 bytes = two super-blocks], 288 bytes apart from row to row:
+// that is 32 modulo 128, so the 8-byte reads of four rows x 32 bytes by a half-warp fall into all banks once.  A row's
+// last stage has fewer boxes (an odd super-block's box is filled up with zeros) and the warps beyond it idle.  Measured on
+// B200, one token, against the kernel of one CTA per SM (qgemv_imma.cu) that had these rows before: 15360x5120 12.3 us
+// (15.5), 27648x5120 18.2 us (26.4), 5120x13824 15.0 us (18.8).
+constexpr int kOddRow = 2 * UB_Q4K_BYTES, kOddBox = 16 * kOddRow;
+// byte of super-block w (0-7) of row r inside a stage
+template <bool ODD>
+__device__ __forceinline__ uint32_t stage_at(int r, int w) {
+  return ODD ? static_cast<uint32_t>((w >> 1) * kOddBox + r * kOddRow + (w & 1) * UB_Q4K_BYTES)
+             : static_cast<uint32_t>(r * (8 * UB_Q4K_BYTES) + w * UB_Q4K_BYTES);
+}
+// the copies of one stage: rows row0 .. row0 + 15 (GU: eight gate rows from row0, eight up rows from row1), stage c of
+// the rows; a stage behind the row's end only arrives
+template <bool ODD, bool GU, bool PAD>
+__device__ __forceinline__ void stage_copy(const CUtensorMap& w_map, uint32_t dst, uint32_t full, int c, int nsb, int row0,
+                                           int row1) {
+  constexpr int kBytes = 16 * 8 * UB_Q4K_BYTES;
+  if (!ODD) {
+    mb_expect_tx(full, !PAD || 8 * c < nsb ? kBytes : 0);
+    if (PAD && 8 * c >= nsb) return;
+#pragma unroll
+    for (int h = 0; h < (GU ? 2 : 1); h++)  // GU: the tensor map's box is 8 rows tall
+      asm volatile(
+          "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
+              "r"(dst + h * (kBytes / 2)),
+          "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(full), "r"(0), "r"(c * (8 * UB_Q4K_BYTES >> 7)),
+          "r"(h ? row1 : row0)
+          : "memory");
+  } else {
+    const int boxes = min(4, (nsb - 8 * c + 1) >> 1);
+    mb_expect_tx(full, boxes > 0 ? boxes * kOddBox : 0);
+    for (int b = 0; b < boxes; b++)
+#pragma unroll
+      for (int h = 0; h < (GU ? 2 : 1); h++)
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+                dst + b * kOddBox + h * (kOddBox / 2)),
+            "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(full), "r"((8 * c + 2 * b) * (UB_Q4K_BYTES / 2)),
+            "r"(h ? row1 : row0)
+            : "memory");
+  }
+}
+
 // GU: the matrix is [gate rows; up rows] (2 N rows) and y[r] = silu(gate_r . x) * (up_r . x): a stage holds gate
 // rows 8T..8T+7 in its rows 0-7 and the matching up rows in its rows 8-15 (two 8-row copies), so that the two
 // halves of every MMA row pair meet in one thread of the epilogue.  Gate and up are rounded to the output type
 // before the activation, which gives the bits of the two-kernel sequence (matmul, then ub_silu_and_mul).
 // MULTI: K is consumed in `npass` passes (rows too long for all activation fragments to be resident at once).
-template <typename XT, bool GU, bool MULTI>
+template <typename XT, bool GU, bool MULTI, bool ODD>
 __global__ void __launch_bounds__(kThreadsM1, 2)
-qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nch, int npass, int y_dtype, int S,
+qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nsb, int npass, int y_dtype, int S,
                          int early, int* err_word, const XT* __restrict__ gamma, float eps, const ArParams ar,
                          const __grid_constant__ CUtensorMap w_map) {
-  constexpr int kRowStride = 8 * UB_Q4K_BYTES;  // 1152 = 9 lines
-  constexpr int kStageBytes = 16 * kRowStride;
+  constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;  // a row's piece: 1152 bytes = 9 lines
+  const int nch = (nsb + 7) >> 3;
   extern __shared__ __align__(128) unsigned char m1_smem_raw[];
   unsigned char* const sm =
       m1_smem_raw + ((1024u - (static_cast<uint32_t>(__cvta_generic_to_shared(m1_smem_raw)) & 1023u)) & 1023u);
@@ -585,20 +632,8 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       const int cn = min(cpp, nch - p * cpp);
       tile = r / cn, c = p * cpp + (r - tile * cn);
     }
-    const uint32_t full = bars_s + 8 * (n % S);
     const int row0 = kTileRows * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x));
-    mb_expect_tx(full, kStageBytes);
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
-            "r"(ring_s + (n % S) * kStageBytes),
-        "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(full), "r"(0), "r"(c * (kRowStride >> 7)), "r"(row0)
-        : "memory");
-    if (GU)  // the tensor map's box is 8 rows tall: the up rows follow N rows further down
-      asm volatile(
-          "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
-              "r"(ring_s + (n % S) * kStageBytes + 8 * kRowStride),
-          "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(full), "r"(0), "r"(c * (kRowStride >> 7)), "r"(N + row0)
-          : "memory");
+    stage_copy<ODD, GU, false>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), c, nsb, row0, N + row0);
   };
   const int n_early = min(min(early, S), my_items);
   if (threadIdx.x == 0)
@@ -612,16 +647,17 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   // behind a warp-level barrier.
   // (Fetching the next pass's activations into shared memory with asynchronous copies while the current pass
   // computes was measured and is no faster: 37.0 against 35.7 us at 8192 x 28672; it costs a ring stage.)
+  auto here = [&](int c) { return !ODD || 8 * c + warp < nsb; };  // this warp has a super-block in stage c
   auto quantise = [&](int c0, int cn, bool first) {
     Raw8<XT> raw[kMaxChunks];
 #pragma unroll
     for (int c = 0; c < kMaxChunks; c++)
-      if (c < cn) raw[c].load(x + static_cast<size_t>(8 * (c0 + c) + warp) * 256 + 8 * lane);
+      if (c < cn && here(c0 + c)) raw[c].load(x + static_cast<size_t>(8 * (c0 + c) + warp) * 256 + 8 * lane);
     Raw8<XT> graw[kMaxChunks];
     if (gamma)
 #pragma unroll
       for (int c = 0; c < kMaxChunks; c++)
-        if (c < cn) graw[c].load(gamma + static_cast<size_t>(8 * (c0 + c) + warp) * 256 + 8 * lane);
+        if (c < cn && here(c0 + c)) graw[c].load(gamma + static_cast<size_t>(8 * (c0 + c) + warp) * 256 + 8 * lane);
     if (first && threadIdx.x == 0)
       for (int n = n_early; n < min(S, my_items); n++) issue_item(n);
     float scale = 1.f;
@@ -629,17 +665,17 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       float ss = 0.f;
 #pragma unroll
       for (int c = 0; c < kMaxChunks; c++) {
-        if (c >= cn) break;
+        if (c >= cn || !here(c0 + c)) break;
         float v[8];
         raw[c].unpack(v);
 #pragma unroll
         for (int e = 0; e < 8; e++) ss = fmaf(v[e], v[e], ss);
       }
-      scale = rms_scale(ss, ssq, warp, lane, 2048 * nch, eps);
+      scale = rms_scale(ss, ssq, warp, lane, 256 * nsb, eps);
     }
 #pragma unroll
     for (int c = 0; c < kMaxChunks; c++) {
-      if (c >= cn) break;
+      if (c >= cn || !here(c0 + c)) break;
       float v[8];
       raw[c].unpack(v);
       if (gamma) {
@@ -691,8 +727,8 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
 
   uint32_t off_h, off_q[4];
   {
-    auto swz = [](uint32_t L) { return L ^ (((L >> 7) & 7u) << 4); };
-    const uint32_t L0 = static_cast<uint32_t>(g * kRowStride + warp * UB_Q4K_BYTES);
+    auto swz = [](uint32_t L) { return ODD ? L : L ^ (((L >> 7) & 7u) << 4); };
+    const uint32_t L0 = stage_at<ODD>(g, warp);
     off_h = swz(L0);
 #pragma unroll
     for (int G = 0; G < 4; G++) off_q[G] = swz(L0 + 16 + 32 * G + 8 * t);
@@ -716,7 +752,7 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       for (int c = 0; c < c_n; c++, item++) {
         if (ok) ok = mb_wait(bars_s + 8 * slot, round & 1);
         const unsigned char* rowA = sm + static_cast<size_t>(slot) * kStageBytes;
-        const unsigned char* rowB = rowA + 8 * kRowStride;
+        const unsigned char* rowB = rowA + stage_at<ODD>(8, 0);
         const uint4 hA = *reinterpret_cast<const uint4*>(rowA + off_h);
         const uint4 hB = *reinterpret_cast<const uint4*>(rowB + off_h);
         uint2 wA[4], wB[4];
@@ -731,6 +767,8 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
           if (ok) ok = mb_wait(bars_s + 8 * (kMaxStagesM1 + slot), round & 1);
           if (ok && lane == 0) issue_item(item + S);
         }
+        if (++slot == S) slot = 0, round++;
+        if (!here(c_lo + c)) continue;
         const unsigned char* f = frag + static_cast<size_t>(8 * c + warp) * kFragBytesPerSb;
         const uint4 f0 = reinterpret_cast<const uint4*>(f)[lane], f1 = reinterpret_cast<const uint4*>(f + 512)[lane];
         const int2 ss = reinterpret_cast<const int2*>(f + 1024)[t];
@@ -766,7 +804,6 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
         acc0 = fmaf(-static_cast<float>(tA), dminA * xs, acc0);
         acc1 = fmaf(fB, dB * xsm, acc1);
         acc1 = fmaf(-static_cast<float>(tB), dminB * xs, acc1);
-        if (++slot == S) slot = 0, round++;
       }
       acc0 += __shfl_xor_sync(0xFFFFFFFFu, acc0, 1);
       acc1 += __shfl_xor_sync(0xFFFFFFFFu, acc1, 1);
@@ -824,12 +861,13 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
 constexpr int kWideWarps = 16;
 constexpr int kWideMaxUnits = 7;  // stages per half: rows up to 28672 values
 
-template <typename XT>
+// PAD: some warps have no super-block in some stages (ODD, or an odd number of stages).
+template <typename XT, bool ODD, bool PAD>
 __global__ void __launch_bounds__(kWideWarps * 32, 1)
-qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nch, int y_dtype, int S, int early,
+qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nsb, int y_dtype, int S, int early,
                          int* err_word, const __grid_constant__ CUtensorMap w_map) {
-  constexpr int kRowStride = 8 * UB_Q4K_BYTES;  // 1152 = 9 lines
-  constexpr int kStageBytes = 16 * kRowStride;
+  constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;  // a row's piece: 1152 bytes = 9 lines
+  const int nch = (nsb + 15) / 16 * 2;  // stages of a row, even: an odd row ends with a stage of no bytes
   extern __shared__ __align__(128) unsigned char m1_smem_raw[];
   unsigned char* const sm =
       m1_smem_raw + ((1024u - (static_cast<uint32_t>(__cvta_generic_to_shared(m1_smem_raw)) & 1023u)) & 1023u);
@@ -860,14 +898,8 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   // item n of this CTA = (tile n / nch, stage n % nch) -> ring slot n % S
   auto issue_item = [&](int n) {
     const int tile = n / nch, c = n - tile * nch;
-    const uint32_t full = bars_s + 8 * (n % S);
-    mb_expect_tx(full, kStageBytes);
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
-            "r"(ring_s + (n % S) * kStageBytes),
-        "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(full), "r"(0), "r"(c * (kRowStride >> 7)),
-        "r"(16 * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x)))
-        : "memory");
+    stage_copy<ODD, false, PAD>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), c, nsb,
+                           16 * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x)), 0);
   };
   const int n_early = min(min(early, S), my_items);
   if (threadIdx.x == 0)
@@ -881,14 +913,14 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
 #pragma unroll
     for (int u = 0; u < kWideMaxUnits; u++) {
       const int c = 2 * u + half;
-      if (c < nch) raw[u].load(x + static_cast<size_t>(8 * c + w8) * 256 + 8 * lane);
+      if (8 * c + w8 < nsb) raw[u].load(x + static_cast<size_t>(8 * c + w8) * 256 + 8 * lane);
     }
     if (threadIdx.x == 0)
       for (int n = n_early; n < min(S, my_items); n++) issue_item(n);
 #pragma unroll
     for (int u = 0; u < kWideMaxUnits; u++) {
       const int c = 2 * u + half;
-      if (c >= nch) break;
+      if (8 * c + w8 >= nsb) break;
       float v[8];
       raw[u].unpack(v);
       float amax = 0.f;
@@ -933,8 +965,8 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
 
   uint32_t off_h, off_q[4];
   {
-    auto swz = [](uint32_t L) { return L ^ (((L >> 7) & 7u) << 4); };
-    const uint32_t L0 = static_cast<uint32_t>(g * kRowStride + w8 * UB_Q4K_BYTES);
+    auto swz = [](uint32_t L) { return ODD ? L : L ^ (((L >> 7) & 7u) << 4); };
+    const uint32_t L0 = stage_at<ODD>(g, w8);
     off_h = swz(L0);
 #pragma unroll
     for (int G = 0; G < 4; G++) off_q[G] = swz(L0 + 16 + 32 * G + 8 * t);
@@ -956,7 +988,7 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
         const uint32_t par = static_cast<uint32_t>(item / S) & 1u;
         if (ok) ok = mb_wait(bars_s + 8 * slot, par);
         const unsigned char* rowA = sm + static_cast<size_t>(slot) * kStageBytes;
-        const unsigned char* rowB = rowA + 8 * kRowStride;
+        const unsigned char* rowB = rowA + stage_at<ODD>(8, 0);
         const uint4 hA = *reinterpret_cast<const uint4*>(rowA + off_h);
         const uint4 hB = *reinterpret_cast<const uint4*>(rowB + off_h);
         uint2 wA[4], wB[4];
@@ -972,6 +1004,7 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
           if (ok) ok = mb_wait(bars_s + 8 * (kMaxStagesM1 + slot), par);
           if (ok && lane == 0) issue_item(item + S);
         }
+        if (PAD && 8 * c + w8 >= nsb) continue;
         const unsigned char* f = frag + static_cast<size_t>(8 * c + w8) * kFragBytesPerSb;
         const uint4 f0 = reinterpret_cast<const uint4*>(f)[lane], f1 = reinterpret_cast<const uint4*>(f + 512)[lane];
         const int2 ss = reinterpret_cast<const int2*>(f + 1024)[t];
@@ -1030,35 +1063,47 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   if (!ok && lane == 0) report_device_error(err_word, UB_ERR_TIMEOUT);
 }
 
+typedef CUresult (*EncodeFnM1)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// Tensor map of the stages of stage_copy: lines of 128 bytes, swizzled, or (rows that are not whole lines) boxes of two
+// super-blocks.
+bool m1_stage_map(EncodeFnM1 enc, CUtensorMap* map, const uint8_t* wq, int rows, int nsb, unsigned box_rows) {
+  const cuuint64_t row_bytes = static_cast<cuuint64_t>(nsb) * UB_Q4K_BYTES;
+  const cuuint32_t estr[3] = {1, 1, 1};
+  if (nsb % 8) {
+    const cuuint64_t dims[2] = {row_bytes / 2, static_cast<cuuint64_t>(rows)}, strides[1] = {row_bytes};
+    const cuuint32_t box[2] = {kOddRow / 2, box_rows};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<uint8_t*>(wq), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  }
+  const cuuint64_t dims[3] = {128, row_bytes / 128, static_cast<cuuint64_t>(rows)}, strides[2] = {128, row_bytes};
+  const cuuint32_t box[3] = {128, 8 * UB_Q4K_BYTES / 128, box_rows};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(wq), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <typename XT>
 int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, cudaStream_t s) {
-  typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(ub::tensor_map_encoder());
+  EncodeFnM1 enc = reinterpret_cast<EncodeFnM1>(ub::tensor_map_encoder());
   if (!enc) return UB_ERR_UNSUPPORTED;
-  constexpr int kRowStride = 8 * UB_Q4K_BYTES;
-  constexpr int kStageBytes = 16 * kRowStride;
+  constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;
   constexpr size_t kBudget = 222 * 1024;  // one CTA per SM: ring + fragments + 1 KB slack + ~4.5 KB static <= 227 KB
-  const int nch = K / 2048;
-  if (nch > 2 * kWideMaxUnits || (nch & 1)) return UB_ERR_UNSUPPORTED;
+  const int nsb = K / UB_QK_K, nch = (nsb + 7) / 8;
+  if (nch > 2 * kWideMaxUnits) return UB_ERR_UNSUPPORTED;
   const size_t frag_bytes = static_cast<size_t>(nch) * 8 * kFragBytesPerSb;
   if (frag_bytes + 4 * static_cast<size_t>(kStageBytes) + 1024 > kBudget) return UB_ERR_UNSUPPORTED;
   int S = static_cast<int>((kBudget - 1024 - frag_bytes) / kStageBytes);
   if (S > kMaxStagesM1) S = kMaxStagesM1;
   S &= ~1;  // even: a slot always serves the same half of the CTA
   CUtensorMap wmap;
-  const cuuint64_t row_bytes = static_cast<cuuint64_t>(K / UB_QK_K) * UB_Q4K_BYTES;
-  const cuuint64_t dims[3] = {128, row_bytes / 128, static_cast<cuuint64_t>(N)};
-  const cuuint64_t strides[2] = {128, row_bytes};
-  const cuuint32_t box[3] = {128, static_cast<cuuint32_t>(kRowStride / 128), 16u};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(wq), dims, strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return UB_ERR_UNSUPPORTED;
+  if (!m1_stage_map(enc, &wmap, wq, N, nsb, 16)) return UB_ERR_UNSUPPORTED;
   const size_t smem = static_cast<size_t>(S) * kStageBytes + frag_bytes + 1024;
-  auto kernel = qgemv_q4k_m1_wide_kernel<XT>;
+  auto kernel = nsb % 8    ? qgemv_q4k_m1_wide_kernel<XT, true, true>
+                : nsb % 16 ? qgemv_q4k_m1_wide_kernel<XT, false, true>
+                           : qgemv_q4k_m1_wide_kernel<XT, false, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
@@ -1075,7 +1120,7 @@ int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr, cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nch, y_dtype, S, early, ub::device_error_word(), wmap);
+  e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nsb, y_dtype, S, early, ub::device_error_word(), wmap);
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
     return ub::fail(UB_ERR_CUDA);
@@ -1086,14 +1131,10 @@ int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
 template <typename XT, bool GU>
 int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, const XT* gamma,
                    float eps, const ArParams& ar, cudaStream_t s) {
-  typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(ub::tensor_map_encoder());
+  EncodeFnM1 enc = reinterpret_cast<EncodeFnM1>(ub::tensor_map_encoder());
   if (!enc) return UB_ERR_UNSUPPORTED;
-  constexpr int kRowStride = 8 * UB_Q4K_BYTES;
-  constexpr int kStageBytes = 16 * kRowStride;
-  const int nch = K / 2048;
+  constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;
+  const int nsb = K / UB_QK_K, nch = (nsb + 7) / 8;
   const int tiles = GU ? (N + 7) / 8 : (N + 15) / 16;
   const int slots = 2 * ub::num_sms();
   const int grid = tiles < slots ? tiles : slots;
@@ -1112,17 +1153,12 @@ int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   int S = static_cast<int>((kRingBudget - frag_bytes) / kStageBytes);
   if (S > kMaxStagesM1) S = kMaxStagesM1;
   CUtensorMap wmap;
-  const cuuint64_t row_bytes = static_cast<cuuint64_t>(K / UB_QK_K) * UB_Q4K_BYTES;
-  const cuuint64_t dims[3] = {128, row_bytes / 128, static_cast<cuuint64_t>(GU ? 2 * N : N)};
-  const cuuint64_t strides[2] = {128, row_bytes};
-  const cuuint32_t box[3] = {128, static_cast<cuuint32_t>(kRowStride / 128), GU ? 8u : 16u};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(wq), dims, strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return UB_ERR_UNSUPPORTED;
+  if (!m1_stage_map(enc, &wmap, wq, GU ? 2 * N : N, nsb, GU ? 8 : 16)) return UB_ERR_UNSUPPORTED;
   const size_t smem = static_cast<size_t>(S) * kStageBytes + frag_bytes + 1024;
-  auto kernel = npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true> : qgemv_q4k_m1_long_kernel<XT, GU, false>;
+  auto kernel = nsb % 8 ? (npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true, true>
+                                     : qgemv_q4k_m1_long_kernel<XT, GU, false, true>)
+                        : (npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true, false>
+                                     : qgemv_q4k_m1_long_kernel<XT, GU, false, false>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
@@ -1136,7 +1172,7 @@ int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr, cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nch, npass, y_dtype, S, early, ub::device_error_word(), gamma, eps, ar,
+  e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nsb, npass, y_dtype, S, early, ub::device_error_word(), gamma, eps, ar,
                          wmap);
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
@@ -1150,7 +1186,7 @@ int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
 namespace ub {
 
 // y[N] = dequant(Wq) . x for one token; UB_ERR_UNSUPPORTED (without touching the thread's status) for shapes
-// these kernels do not take (K not a multiple of 2048; beyond 12288: more rows than one batch of tiles per CTA, or
+// these kernels do not take (beyond 12288 values: more rows than one batch of tiles per CTA, or
 // with the RMSNorm prologue; unaligned weights; no tensor-map encoder).
 // fresh: the weight bytes may have been written by the kernel launched just before on the same stream.
 template <typename XT>
@@ -1164,15 +1200,15 @@ int q4k_gemv_m1x(const void* wq, const XT* x, void* y, int N, int K, int y_dtype
   const XT* gamma = static_cast<const XT*>(ex.gamma);
   if (K == 4096) return launch_m1<XT, 2>(w, x, y, N, K, y_dtype, fresh, gamma, ex.eps, a, s);
   if (K == 2048) return launch_m1<XT, 1>(w, x, y, N, K, y_dtype, fresh, gamma, ex.eps, a, s);
-  if (K % 2048 == 0 && K >= 12288 && !gamma && a.world <= 1 && !a.residual) {
+  if (K >= 12288 && !gamma && a.world <= 1 && !a.residual) {
     // one pass, one CTA of sixteen warps per SM (an even number of stages per row); measured on B200 at 8192 rows:
-    // 12288 values 13.1 us against 14.1 with two CTAs per SM, 28672 values 30.0 against 35.7 in four passes;
+    // 12288 values 13.1 us against 14.1 with two CTAs per SM, 28672 values 30.0 against 35.7 in four passes; an odd number of
+    // stages (one more that carries no bytes makes it even) 10.4 against 12.0 us in two passes at 4096 rows of 14336 values;
     // at 8192 values the two-CTA kernel is the faster one (11.0 against 12.1 us at 10240 rows)
     const int st = launch_m1_wide<XT>(w, x, y, N, K, y_dtype, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
-  if (K % 2048 == 0) return launch_m1_long<XT, false>(w, x, y, N, K, y_dtype, fresh, gamma, ex.eps, a, s);
-  return UB_ERR_UNSUPPORTED;
+  return launch_m1_long<XT, false>(w, x, y, N, K, y_dtype, fresh, gamma, ex.eps, a, s);
 }
 
 template <typename XT>
@@ -1188,7 +1224,7 @@ template <typename XT>
 int q4k_gemv_m1_gate_up(const void* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, const void* gamma,
                         float eps, cudaStream_t s) {
   const uint8_t* w = static_cast<const uint8_t*>(wq);
-  if ((reinterpret_cast<uintptr_t>(w) & 15) || K % 2048) return UB_ERR_UNSUPPORTED;
+  if (reinterpret_cast<uintptr_t>(w) & 15) return UB_ERR_UNSUPPORTED;
   ArParams none;
   memset(&none, 0, sizeof(none));
   return launch_m1_long<XT, true>(w, x, y, N, K, y_dtype, fresh, static_cast<const XT*>(gamma), eps, none, s);

@@ -223,7 +223,7 @@ int ub_qmatmul_q4k_bf16(void* y, const void* x, const void* wq, int M, int N, in
 
 // ---- gate/up projection with the SiLU.up step in the matmul's epilogue ----
 // y[M, I] = silu(x . Wgate^T) * (x . Wup^T) with wq = [gate rows; up rows] (2 I rows of K), bf16 activations.
-// One token with K a multiple of 2048 up to 12288 is ONE launch; everything else is the matmul into the
+// One token with K up to 12288 is ONE launch; everything else is the matmul into the
 // workspace followed by ub_silu_and_mul (the reference's own sequence, kernels/topsaten_ops_wrapper.cpp:375-391).
 size_t ub_qmatmul_q4k_gate_up_workspace_bytes(int M, int I, int K) {
   if (M <= 0 || I <= 0 || K <= 0) return 0;
@@ -281,7 +281,7 @@ size_t ub_qmatmul_q4k_rmsnorm_workspace_bytes(int M, int N, int K, int gate_up) 
 }
 
 // y = rmsnorm(x; gamma, eps) . W^T (gate_up == 0, y [M,N]) or silu(. Wgate^T) * (. Wup^T) (gate_up != 0, y [M,N] with
-// W = [gate rows; up rows] of 2 N rows), x and gamma bf16.  One token with K a multiple of 2048 up to 12288 is one
+// W = [gate rows; up rows] of 2 N rows), x and gamma bf16.  One token with K up to 12288 is one
 // launch: every CTA of the matmul normalises the activation row in its prologue.  Other shapes run
 // topsaten_rms_norm into the workspace and then the matmul.
 int ub_qmatmul_q4k_rmsnorm_bf16(void* y, const void* x, const void* gamma, float eps, const void* wq, int M, int N,
