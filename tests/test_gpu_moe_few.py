@@ -1,0 +1,49 @@
+"""Expert layer for a few tokens: a token at a time through the one-token kernels (two launches per token)."""
+import numpy as np
+import pytest
+
+from oracle import oracle as o
+from ubridge_b200 import DTYPE_BF16, ops
+
+from _util import fetch, to_storage
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, emap=None, norm=True):
+    ws_bytes = ops.moe_layer_q4k_workspace_bytes(T, H, I, E, k, 64)
+    d = [dev.htod_sync_copy(v) for v in (to_storage(hidden, DTYPE_BF16), to_storage(logits, DTYPE_BF16), w13, w2)]
+    d_map = None if emap is None else dev.htod_sync_copy(emap)
+    d_out = dev.alloc(T * H * 2)
+    ops.moe_layer_q4k(d_out, d[0], d[1], d[2], d[3], T, H, I, E, k, 64, norm, dev.alloc(ws_bytes), ws_bytes,
+                      expert_map=d_map, stream=dev.stream)
+    return fetch(dev, d_out, DTYPE_BF16, (T, H))
+
+
+@pytest.mark.parametrize("T,H,I,E,k,norm", [
+    (1, 256, 256, 4, 1, True),      # one slot, one super-block
+    (1, 2048, 4096, 8, 2, True),    # rows of whole lines
+    (2, 768, 1280, 5, 3, False),    # boxes of two super-blocks, an odd number of stages over the slots
+    (3, 1024, 14336, 4, 2, True),   # two slots of seven stages: the longest the down launch takes
+    (4, 512, 1024, 12, 8, True),    # eight slots
+    (2, 512, 28672, 3, 2, True),    # more stages than the down launch takes: the grouped kernels
+])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_few_tokens(dev, T, H, I, E, k, norm, mapped):
+    rng = np.random.default_rng(T + H + I + E)
+    emap = None
+    local = E
+    if mapped:  # every other expert is held by another rank
+        emap = np.full(E, -1, dtype=np.int32)
+        emap[::2] = np.arange((E + 1) // 2)
+        local = (E + 1) // 2
+    w13, w2 = o.gen_q4k_weight(rng, E * 2 * I, H), o.gen_q4k_weight(rng, E * H, I)
+    hidden, logits = o.gen_activation(rng, T, H, True), o.gen_activation(rng, T, E, True)
+    got = _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, emap, norm)
+    deq13 = o.c_dequant(w13, True).reshape(E, 2 * I, H)[:local]
+    deq2 = o.c_dequant(w2, True).reshape(E, H, I)[:local]
+    want, _ = o.moe_layer_exact(hidden, logits, deq13, deq2, k, 64, norm, expert_map=emap)
+    assert o.rel_l2(got, want) < 1e-2  # activations, each slot's output (in the oracle) and the sum are rounded to bf16
+    assert dev.device_status() == 0
+
+

@@ -227,6 +227,8 @@ __global__ void bf16_to_f32_kernel(float* __restrict__ out, const __nv_bfloat16*
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+constexpr int kMoeFewTokens = 4;  // most tokens that ub_moe_layer_q4k takes one at a time
+
 }  // namespace
 
 namespace ub {
@@ -248,6 +250,8 @@ int q4k_gemm_mma(void* y, const void* x, const void* wq, int M, int N, int K, cu
 }  // namespace ub
 
 namespace ub {
+int q4k_moe_one_token(void* out, void* act, const void* x, const void* w13, const void* w2, const int32_t* idx,
+                      const void* weights, const int32_t* map, int H, int I, int E, int slots, cudaStream_t s);
 bool q4k_moe_tc_supported(int positions, int K, int N, int block);
 int moe_gather_rows(void* xg, const void* hidden, const int32_t* sorted_ids, const int32_t* num_post_pad, int positions,
                     int num_valid, int top_k, int H, cudaStream_t s);
@@ -342,6 +346,20 @@ int ub_moe_layer_q4k(void* out, const void* hidden, const void* router_logits, c
 
   int st = ub::topk_softmax_bf16_impl(router_logits, w_t, idx, T, E, top_k, norm_topk_prob != 0, s);
   if (st != UB_OK) return st;
+  // Few tokens: a token at a time through the one-token kernels, each token's experts read at streaming speed.  Beyond, the
+  // grouped kernel's cost grows with the experts touched and not with the tokens.  Measured on B200, 8 experts top-2,
+  // 4096 / 14336, us per layer: one token 54 against 206; the layer of four tokens takes four times that, 190, as the grouped
+  // kernel for the seven experts that four to eight tokens touch takes more than 300.
+  if (T <= kMoeFewTokens && !((reinterpret_cast<uintptr_t>(w13q) | reinterpret_cast<uintptr_t>(w2q) |
+                                   reinterpret_cast<uintptr_t>(hidden)) & 15)) {
+    for (int t = 0; t < T; t++) {
+      st = ub::q4k_moe_one_token(static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(t) * H, act,
+                                 static_cast<const __nv_bfloat16*>(hidden) + static_cast<size_t>(t) * H, w13q, w2q,
+                                 idx + t * top_k, w_t + t * top_k, expert_map, H, I, E, top_k, s);
+      if (st != UB_OK) break;
+    }
+    if (st != UB_ERR_UNSUPPORTED) return st;
+  }
   bf16_to_f32_kernel<<<static_cast<int>((slots + 255) / 256), 256, 0, s>>>(w_f32, w_t, static_cast<int>(slots));
   st = ub::moe_align(sorted_ids, experts_ids, npp, idx, nullptr, expert_map, E, block_size, T, top_k, s);
   if (st != UB_OK) return st;

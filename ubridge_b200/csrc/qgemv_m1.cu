@@ -546,6 +546,31 @@ __device__ __forceinline__ uint32_t stage_at(int r, int w) {
   return ODD ? static_cast<uint32_t>((w >> 1) * kOddBox + r * kOddRow + (w & 1) * UB_Q4K_BYTES)
              : static_cast<uint32_t>(r * (8 * UB_Q4K_BYTES) + w * UB_Q4K_BYTES);
 }
+// One token through the experts it is routed to (SEL).  The tensor holds E matrices of `rows` rows; slot j takes matrix
+// idx[j] (through `map`, when given: -1 = held by another rank, the slot contributes nothing).
+struct ExpertSel {
+  const int32_t* idx;           // [slots] expert of each slot
+  const __nv_bfloat16* weight;  // [slots] routed weights
+  const int32_t* map;           // [E] global expert -> matrix, or null
+  int slots, rows, experts;
+};
+constexpr int kSelMax = 16;
+// Reads the slots' experts into shared memory (all threads of the CTA).
+__device__ __forceinline__ void sel_load(const ExpertSel& sel, int* mat, float* weight, int* err_word) {
+  if (static_cast<int>(threadIdx.x) < sel.slots) {
+    int e = sel.idx[threadIdx.x];
+    if (e < 0 || e >= sel.experts) {  // the router chose nothing (logits that are not numbers)
+      report_device_error(err_word, UB_ERR_BAD_INDEX);
+      e = -1;
+    } else if (sel.map) {
+      e = sel.map[e];
+      if (e >= sel.experts) e = -1;
+    }
+    mat[threadIdx.x] = e < 0 ? 0 : e;
+    if (weight) weight[threadIdx.x] = e < 0 ? 0.f : __bfloat162float(sel.weight[threadIdx.x]);
+  }
+  __syncthreads();
+}
 // the copies of one stage: rows row0 .. row0 + 15 (GU: eight gate rows from row0, eight up rows from row1), stage c of
 // the rows; a stage behind the row's end only arrives
 template <bool ODD, bool GU, bool PAD>
@@ -583,13 +608,15 @@ __device__ __forceinline__ void stage_copy(const CUtensorMap& w_map, uint32_t ds
 // halves of every MMA row pair meet in one thread of the epilogue.  Gate and up are rounded to the output type
 // before the activation, which gives the bits of the two-kernel sequence (matmul, then ub_silu_and_mul).
 // MULTI: K is consumed in `npass` passes (rows too long for all activation fragments to be resident at once).
-template <typename XT, bool GU, bool MULTI, bool ODD>
+// SEL (with GU): N rows are the slots' gate rows one slot behind the other, act[slot][row].
+template <typename XT, bool GU, bool MULTI, bool ODD, bool SEL>
 __global__ void __launch_bounds__(kThreadsM1, 2)
 qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nsb, int npass, int y_dtype, int S,
                          int early, int* err_word, const XT* __restrict__ gamma, float eps, const ArParams ar,
-                         const __grid_constant__ CUtensorMap w_map) {
+                         const ExpertSel sel, const __grid_constant__ CUtensorMap w_map) {
   constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;  // a row's piece: 1152 bytes = 9 lines
   const int nch = (nsb + 7) >> 3;
+  __shared__ int sel_mat[SEL ? kSelMax : 1];
   extern __shared__ __align__(128) unsigned char m1_smem_raw[];
   unsigned char* const sm =
       m1_smem_raw + ((1024u - (static_cast<uint32_t>(__cvta_generic_to_shared(m1_smem_raw)) & 1023u)) & 1023u);
@@ -632,14 +659,20 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       const int cn = min(cpp, nch - p * cpp);
       tile = r / cn, c = p * cpp + (r - tile * cn);
     }
-    const int row0 = kTileRows * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x));
-    stage_copy<ODD, GU, false>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), c, nsb, row0, N + row0);
+    int row0 = kTileRows * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x)), up = N;
+    if (SEL) {  // a tile lies inside one slot (its rows are a multiple of eight); gate and up halves of sel.rows / 2
+      up = sel.rows >> 1;
+      const int slot = row0 / up;
+      row0 += sel_mat[slot] * sel.rows - slot * up;
+    }
+    stage_copy<ODD, GU, false>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), c, nsb, row0, up + row0);
   };
   const int n_early = min(min(early, S), my_items);
   if (threadIdx.x == 0)
     for (int n = 0; n < n_early; n++) issue_item(n);
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (SEL) sel_load(sel, sel_mat, nullptr, err_word);
   const uint32_t epoch = ar.world > 1 ? ar_epoch(ar) : 0;  // of the fused all-reduce, read after the wait
 
   // ---- activations of this warp's super-blocks of one pass (stages c0 .. c0 + cn - 1, super-block 8c + warp) ->
@@ -861,13 +894,23 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
 constexpr int kWideWarps = 16;
 constexpr int kWideMaxUnits = 7;  // stages per half: rows up to 28672 values
 
-// PAD: some warps have no super-block in some stages (ODD, or an odd number of stages).
-template <typename XT, bool ODD, bool PAD>
+// SEL: a row is the slots' rows one behind the other, each ncs stages long, x the slots' activations likewise; the routed
+// weight goes into the activations' block scales, so the sum over the slots is the row's sum.
+// PAD: some warps have no super-block in some stages (ODD, SEL, or an odd number of stages).
+template <typename XT, bool ODD, bool SEL, bool PAD>
 __global__ void __launch_bounds__(kWideWarps * 32, 1)
 qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nsb, int y_dtype, int S, int early,
-                         int* err_word, const __grid_constant__ CUtensorMap w_map) {
+                         int* err_word, const ExpertSel sel, const __grid_constant__ CUtensorMap w_map) {
   constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;  // a row's piece: 1152 bytes = 9 lines
-  const int nch = (nsb + 15) / 16 * 2;  // stages of a row, even: an odd row ends with a stage of no bytes
+  const int ncs = (nsb + 7) >> 3;
+  const int nch = ((SEL ? sel.slots * ncs : ncs) + 1) & ~1;  // stages of a row, even: an odd row ends with one of no bytes
+  __shared__ int sel_mat[SEL ? kSelMax : 1];
+  __shared__ float sel_w[SEL ? kSelMax : 1];
+  // stage c -> slot and the stage inside it
+  auto split = [&](int c, int& slot_j, int& cc) {
+    slot_j = SEL ? c / ncs : 0, cc = c - slot_j * ncs;
+    if (SEL && slot_j >= sel.slots) cc = ncs;  // the stage of no bytes
+  };
   extern __shared__ __align__(128) unsigned char m1_smem_raw[];
   unsigned char* const sm =
       m1_smem_raw + ((1024u - (static_cast<uint32_t>(__cvta_generic_to_shared(m1_smem_raw)) & 1023u)) & 1023u);
@@ -898,31 +941,41 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   // item n of this CTA = (tile n / nch, stage n % nch) -> ring slot n % S
   auto issue_item = [&](int n) {
     const int tile = n / nch, c = n - tile * nch;
-    stage_copy<ODD, false, PAD>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), c, nsb,
-                           16 * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x)), 0);
+    int row0 = 16 * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x)), j, cc;
+    split(c, j, cc);
+    if (SEL && cc < ncs) row0 += sel_mat[j] * sel.rows;
+    stage_copy<ODD, false, PAD>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), cc, nsb, row0, 0);
   };
   const int n_early = min(min(early, S), my_items);
   if (threadIdx.x == 0)
     for (int n = 0; n < n_early; n++) issue_item(n);
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (SEL) sel_load(sel, sel_mat, sel_w, err_word);
 
   // ---- activations of this warp's super-blocks (stages c = half, half + 2, ...; super-block 8c + w8) ----
   {
     Raw8<XT> raw[kWideMaxUnits];
 #pragma unroll
     for (int u = 0; u < kWideMaxUnits; u++) {
-      const int c = 2 * u + half;
-      if (8 * c + w8 < nsb) raw[u].load(x + static_cast<size_t>(8 * c + w8) * 256 + 8 * lane);
+      int j, cc;
+      split(2 * u + half, j, cc);
+      if (8 * cc + w8 < nsb) raw[u].load(x + (static_cast<size_t>(j) * nsb + 8 * cc + w8) * 256 + 8 * lane);
     }
     if (threadIdx.x == 0)
       for (int n = n_early; n < min(S, my_items); n++) issue_item(n);
 #pragma unroll
     for (int u = 0; u < kWideMaxUnits; u++) {
       const int c = 2 * u + half;
-      if (8 * c + w8 >= nsb) break;
+      int j, cc;
+      split(c, j, cc);
+      if (8 * cc + w8 >= nsb) continue;
       float v[8];
       raw[u].unpack(v);
+      const float slot_w = SEL ? sel_w[j] : 1.f;
+      if (SEL && slot_w == 0.f)
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = 0.f;  // an expert of another rank: whatever its activations hold
       float amax = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
@@ -958,7 +1011,7 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       }
       const int s_lo = __shfl_sync(0xFFFFFFFFu, sum, 4 * t), s_hi = __shfl_sync(0xFFFFFFFFu, sum, 16 + 4 * t);
       if (g == 0) reinterpret_cast<int2*>(f + 1024)[t] = make_int2(s_lo, s_hi);
-      if (lane == 0) *reinterpret_cast<float*>(f + 1024 + 32) = amax * (1.f / kXQMaxM1);
+      if (lane == 0) *reinterpret_cast<float*>(f + 1024 + 32) = amax * (1.f / kXQMaxM1) * slot_w;
     }
     __syncwarp();
   }
@@ -1004,7 +1057,11 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
           if (ok) ok = mb_wait(bars_s + 8 * (kMaxStagesM1 + slot), par);
           if (ok && lane == 0) issue_item(item + S);
         }
-        if (PAD && 8 * c + w8 >= nsb) continue;
+        if (PAD) {
+          int j, cc;
+          split(c, j, cc);
+          if (8 * cc + w8 >= nsb) continue;
+        }
         const unsigned char* f = frag + static_cast<size_t>(8 * c + w8) * kFragBytesPerSb;
         const uint4 f0 = reinterpret_cast<const uint4*>(f)[lane], f1 = reinterpret_cast<const uint4*>(f + 512)[lane];
         const int2 ss = reinterpret_cast<const int2*>(f + 1024)[t];
@@ -1086,12 +1143,13 @@ bool m1_stage_map(EncodeFnM1 enc, CUtensorMap* map, const uint8_t* wq, int rows,
 }
 
 template <typename XT>
-int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, cudaStream_t s) {
+int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, cudaStream_t s,
+                   const ExpertSel* sel = nullptr, int sel_rows_total = 0) {
   EncodeFnM1 enc = reinterpret_cast<EncodeFnM1>(ub::tensor_map_encoder());
   if (!enc) return UB_ERR_UNSUPPORTED;
   constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;
   constexpr size_t kBudget = 222 * 1024;  // one CTA per SM: ring + fragments + 1 KB slack + ~4.5 KB static <= 227 KB
-  const int nsb = K / UB_QK_K, nch = (nsb + 7) / 8;
+  const int nsb = K / UB_QK_K, nch = (sel ? sel->slots : 1) * ((nsb + 7) / 8);
   if (nch > 2 * kWideMaxUnits) return UB_ERR_UNSUPPORTED;
   const size_t frag_bytes = static_cast<size_t>(nch) * 8 * kFragBytesPerSb;
   if (frag_bytes + 4 * static_cast<size_t>(kStageBytes) + 1024 > kBudget) return UB_ERR_UNSUPPORTED;
@@ -1099,11 +1157,19 @@ int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   if (S > kMaxStagesM1) S = kMaxStagesM1;
   S &= ~1;  // even: a slot always serves the same half of the CTA
   CUtensorMap wmap;
-  if (!m1_stage_map(enc, &wmap, wq, N, nsb, 16)) return UB_ERR_UNSUPPORTED;
+  if (!m1_stage_map(enc, &wmap, wq, sel ? sel_rows_total : N, nsb, 16)) return UB_ERR_UNSUPPORTED;
   const size_t smem = static_cast<size_t>(S) * kStageBytes + frag_bytes + 1024;
-  auto kernel = nsb % 8    ? qgemv_q4k_m1_wide_kernel<XT, true, true>
-                : nsb % 16 ? qgemv_q4k_m1_wide_kernel<XT, false, true>
-                           : qgemv_q4k_m1_wide_kernel<XT, false, false>;
+  auto kernel = nsb % 8    ? qgemv_q4k_m1_wide_kernel<XT, true, false, true>
+                : nsb % 16 ? qgemv_q4k_m1_wide_kernel<XT, false, false, true>
+                           : qgemv_q4k_m1_wide_kernel<XT, false, false, false>;
+  ExpertSel esel;
+  memset(&esel, 0, sizeof(esel));
+  if constexpr (std::is_same<XT, __nv_bfloat16>::value) {
+    if (sel) {
+      esel = *sel;
+      kernel = nsb % 8 ? qgemv_q4k_m1_wide_kernel<XT, true, true, true> : qgemv_q4k_m1_wide_kernel<XT, false, true, true>;
+    }
+  }
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
@@ -1112,7 +1178,7 @@ int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   const int tiles = (N + 15) / 16;
   const int sms = ub::num_sms();
   const int grid = tiles < sms ? tiles : sms;
-  const int early = fresh ? 0 : 2;
+  const int early = fresh || sel ? 0 : 2;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kWideWarps * 32), cfg.dynamicSmemBytes = smem, cfg.stream = s;
@@ -1120,7 +1186,7 @@ int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr, cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nsb, y_dtype, S, early, ub::device_error_word(), wmap);
+  e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nsb, y_dtype, S, early, ub::device_error_word(), esel, wmap);
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
     return ub::fail(UB_ERR_CUDA);
@@ -1130,7 +1196,8 @@ int launch_m1_wide(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
 
 template <typename XT, bool GU>
 int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, const XT* gamma,
-                   float eps, const ArParams& ar, cudaStream_t s) {
+                   float eps, const ArParams& ar, cudaStream_t s, const ExpertSel* sel = nullptr,
+                   int sel_rows_total = 0) {
   EncodeFnM1 enc = reinterpret_cast<EncodeFnM1>(ub::tensor_map_encoder());
   if (!enc) return UB_ERR_UNSUPPORTED;
   constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;
@@ -1152,19 +1219,29 @@ int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   if (frag_bytes + 3 * static_cast<size_t>(kStageBytes) > kRingBudget) return UB_ERR_UNSUPPORTED;
   int S = static_cast<int>((kRingBudget - frag_bytes) / kStageBytes);
   if (S > kMaxStagesM1) S = kMaxStagesM1;
-  CUtensorMap wmap;
-  if (!m1_stage_map(enc, &wmap, wq, GU ? 2 * N : N, nsb, GU ? 8 : 16)) return UB_ERR_UNSUPPORTED;
   const size_t smem = static_cast<size_t>(S) * kStageBytes + frag_bytes + 1024;
-  auto kernel = nsb % 8 ? (npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true, true>
-                                     : qgemv_q4k_m1_long_kernel<XT, GU, false, true>)
-                        : (npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true, false>
-                                     : qgemv_q4k_m1_long_kernel<XT, GU, false, false>);
+  auto kernel = nsb % 8 ? (npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true, true, false>
+                                     : qgemv_q4k_m1_long_kernel<XT, GU, false, true, false>)
+                        : (npass > 1 ? qgemv_q4k_m1_long_kernel<XT, false, true, false, false>
+                                     : qgemv_q4k_m1_long_kernel<XT, GU, false, false, false>);
+  ExpertSel esel;
+  memset(&esel, 0, sizeof(esel));
+  int w_rows = GU ? 2 * N : N;
+  if constexpr (GU) {
+    if (sel) {
+      esel = *sel, w_rows = sel_rows_total;
+      kernel = nsb % 8 ? qgemv_q4k_m1_long_kernel<XT, true, false, true, true>
+                       : qgemv_q4k_m1_long_kernel<XT, true, false, false, true>;
+    }
+  }
+  CUtensorMap wmap;
+  if (!m1_stage_map(enc, &wmap, wq, w_rows, nsb, GU ? 8 : 16)) return UB_ERR_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
     return ub::fail(UB_ERR_CUDA);
   }
-  const int early = fresh ? 0 : 2;  // 36 KB per CTA ahead of the dependency wait, as in the short-row kernel
+  const int early = fresh || sel ? 0 : 2;  // 36 KB per CTA ahead of the dependency wait, as in the short-row kernel
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kThreadsM1), cfg.dynamicSmemBytes = smem, cfg.stream = s;
@@ -1173,7 +1250,7 @@ int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr, cfg.numAttrs = 1;
   e = cudaLaunchKernelEx(&cfg, kernel, x, y, N, nsb, npass, y_dtype, S, early, ub::device_error_word(), gamma, eps, ar,
-                         wmap);
+                         esel, wmap);
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
     return ub::fail(UB_ERR_CUDA);
@@ -1228,6 +1305,27 @@ int q4k_gemv_m1_gate_up(const void* wq, const XT* x, void* y, int N, int K, int 
   ArParams none;
   memset(&none, 0, sizeof(none));
   return launch_m1_long<XT, true>(w, x, y, N, K, y_dtype, fresh, static_cast<const XT*>(gamma), eps, none, s);
+}
+
+// One token through its `slots` experts: act[slots][I] = silu(gate) * up from w13 ([E][2 I rows of H]), then
+// out[H] = sum over the slots of weight * (act . w2^T), w2 [E][H rows of I].  Two launches; act is scratch.
+// UB_ERR_UNSUPPORTED (nothing launched): rows too long for one pass, more slots or stages than the kernels keep.
+int q4k_moe_one_token(void* out, void* act, const void* x, const void* w13, const void* w2, const int32_t* idx,
+                      const void* weights, const int32_t* map, int H, int I, int E, int slots, cudaStream_t s) {
+  const int stages = slots * ((I / UB_QK_K + 7) / 8);
+  if (slots > kSelMax || H % UB_QK_K || I % UB_QK_K || (H / UB_QK_K + 7) / 8 > kMaxChunks || stages > 2 * kWideMaxUnits ||
+      !ub::tensor_map_encoder())
+    return UB_ERR_UNSUPPORTED;
+  ArParams none;
+  memset(&none, 0, sizeof(none));
+  ExpertSel sel = {idx, static_cast<const __nv_bfloat16*>(weights), map, slots, 2 * I, E};
+  int st = launch_m1_long<__nv_bfloat16, true>(static_cast<const uint8_t*>(w13), static_cast<const __nv_bfloat16*>(x), act,
+                                               slots * I, H, UB_DTYPE_BF16, false, nullptr, 0.f, none, s, &sel, E * 2 * I);
+  if (st != UB_OK) return st;
+  sel.rows = H;
+  st = launch_m1_wide<__nv_bfloat16>(static_cast<const uint8_t*>(w2), static_cast<const __nv_bfloat16*>(act), out, H, I,
+                                     UB_DTYPE_BF16, false, s, &sel, E * H);
+  return st == UB_ERR_UNSUPPORTED ? ub::fail(st) : st;
 }
 
 template int q4k_gemv_m1x<float>(const void*, const float*, void*, int, int, int, bool, const M1Extras&, cudaStream_t);
