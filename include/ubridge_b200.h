@@ -284,6 +284,9 @@ void topsaten_release_graph_workspace_pool(void* stream);
 /* ------------------------------------------------------------------ MoE: new fused entry points */
 /* out[t, :D] = silu(in[t, :D]) * in[t, D:2D]  (kernels/topsaten_ops_wrapper.cpp:375-391) */
 int ub_silu_and_mul(void* out, const void* in, int rows, int D, int dtype, void* stream);
+/* dst[height][width] = src[height][width] (bytes) at the given row pitches, device memory */
+int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t height,
+                 void* stream);
 /* out[t,:] = sum_j in[t,j,:]  (the reference's caller uses topsaten_sum, src/ffi.rs:841-849) */
 int ub_topk_sum(void* out, const void* in, int T, int topk, int H, int dtype, void* stream);
 

@@ -1,0 +1,52 @@
+"""The row-wise kernels between the matmuls with 16-byte accesses: RMSNorm, SiLU.up, strided copy."""
+import numpy as np
+import pytest
+
+from oracle import oracle as o
+from ubridge_b200 import DTYPE_BF16, DTYPE_F16, DTYPE_F32, ops
+from ubridge_b200._lib import check, lib
+
+from _util import ESIZE, fetch, to_storage
+
+pytestmark = pytest.mark.gpu
+ODT = {DTYPE_F32: o.UB_F32, DTYPE_F16: o.UB_F16, DTYPE_BF16: o.UB_BF16}
+
+
+@pytest.mark.parametrize("dtype", sorted(ODT))
+# one piece; less and more than a round of the CTA; the registers' capacity and beyond; rows that are not whole pieces
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 2040), (5, 2056), (2, 8192), (3, 8200), (1, 20000), (4, 1001)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_rms_norm_rows(dev, dtype, T, H, in_place):
+    rng = np.random.default_rng(T + H)
+    x = o.round_through(rng.standard_normal((T, H)).astype(np.float32) * 3, ODT[dtype])
+    g = o.round_through(rng.uniform(0.5, 1.5, size=H).astype(np.float32), ODT[dtype])
+    d_x = dev.htod_sync_copy(to_storage(x, dtype))
+    d_out = d_x if in_place else dev.alloc(T * H * ESIZE[dtype])
+    ops.rms_norm(d_out, d_x, dev.htod_sync_copy(to_storage(g, dtype)), T, H, 1e-5, dtype, stream=dev.stream)
+    # f32 vs f64 mean and rsqrt: a value on a rounding boundary may fall the other way, by one unit of the type
+    assert o.rel_l2(fetch(dev, d_out, dtype, (T, H)), o.rms_norm(x, g, 1e-5, ODT[dtype])) < {
+        DTYPE_F32: 1e-6, DTYPE_F16: 1e-3, DTYPE_BF16: 4e-3}[dtype]
+
+
+@pytest.mark.parametrize("dtype", sorted(ODT))
+@pytest.mark.parametrize("rows,D", [(1, 8), (33, 72), (3, 2056), (2, 14336), (5, 77), (40000, 8)])
+def test_silu_and_mul_rows(dev, dtype, rows, D):
+    rng = np.random.default_rng(rows + D)
+    x = o.round_through(rng.standard_normal((rows, 2 * D)).astype(np.float32) * 4, ODT[dtype])
+    d_o = dev.alloc(rows * D * ESIZE[dtype])
+    ops.silu_and_mul(d_o, dev.htod_sync_copy(to_storage(x, dtype)), rows, D, dtype, stream=dev.stream)
+    got, want = fetch(dev, d_o, dtype, (rows, D)), o.silu_and_mul(x, ODT[dtype])
+    # expf differs by an ulp between libm and CUDA: one unit of the type on a rounding boundary
+    assert np.allclose(got, want, rtol={DTYPE_F32: 2 ** -21, DTYPE_F16: 2 ** -10, DTYPE_BF16: 2 ** -7}[dtype], atol=1e-7)
+
+
+@pytest.mark.parametrize("rows,width,src_pitch,dst_pitch", [(1, 16, 16, 16), (3, 8192, 12288, 8192), (40000, 32, 48, 64),
+                                                            (7, 30, 64, 32), (2, 64, 66, 64)])
+def test_copy_rows(dev, rows, width, src_pitch, dst_pitch):
+    rng = np.random.default_rng(rows + width)
+    src = rng.integers(0, 256, (rows, src_pitch), dtype=np.uint8)
+    dst = rng.integers(0, 256, (rows, dst_pitch), dtype=np.uint8)
+    d_s, d_d = dev.htod_sync_copy(src), dev.htod_sync_copy(dst)
+    check(lib().ub_copy_rows(d_d.ptr, dst_pitch, d_s.ptr, src_pitch, width, rows, dev.stream), "copy_rows")
+    dst[:, :width] = src[:, :width]
+    assert np.array_equal(dev.dtoh_sync_copy(d_d, np.uint8, (rows, dst_pitch)), dst)

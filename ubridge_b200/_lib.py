@@ -140,6 +140,7 @@ _SIGS = {
     "topsaten_fused_moe_gemm": (c_int, [_P] * 8 + [c_int32] * 8 + [_P]),
     "topsaten_release_graph_workspace_pool": (None, [_P]),
     "ub_silu_and_mul": (c_int, [_P, _P, c_int, c_int, c_int, _P]),
+    "ub_copy_rows": (c_int, [_P, c_size_t, _P, c_size_t, c_size_t, c_size_t, _P]),
     "ub_topk_sum": (c_int, [_P, _P, c_int, c_int, c_int, c_int, _P]),
     "ub_fused_moe_q4k_gemm": (c_int, [_P] * 7 + [c_int] * 9 + [_P, c_size_t, _P]),
     "ub_indexed_moe_q4k": (c_int, [_P, _P, _P, _P] + [c_int] * 7 + [_P]),

@@ -38,6 +38,38 @@ __device__ __forceinline__ void report_device_error(int* err_word, int code) {
   if (err_word) atomicMax(err_word, code);
 }
 
+// ---- programmatic dependent launch ----
+// A kernel launched this way may start while the kernel in front of it on the stream still runs: it calls pdl_wait()
+// before it touches anything that one may write or read.  pdl_open() lets the next such kernel start in turn; called
+// after pdl_wait(), so that what that kernel requests ahead of its own wait (weights) is not written any more by a
+// kernel further up.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr, cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) {
+    set_cuda_error(e);
+    return fail(UB_ERR_CUDA);
+  }
+  return check_launch();
+}
+
+// ---- 16 bytes of a storage type ----
+template <typename T>
+struct Vec16 {
+  static constexpr int N = 16 / sizeof(T);
+  uint4 r;
+  __device__ __forceinline__ T at(int i) const { return reinterpret_cast<const T*>(&r)[i]; }
+  __device__ __forceinline__ void set(int i, T v) { reinterpret_cast<T*>(&r)[i] = v; }
+};
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int num_sms() {

@@ -552,6 +552,29 @@ __global__ void __launch_bounds__(256) silu_and_mul_kernel(T* __restrict__ out, 
   }
 }
 
+// The same with 16-byte accesses (D whole 16-byte pieces, everything 16-byte aligned) and overlapped with its neighbours:
+// blockIdx.y walks the rows, so no element needs a division.
+template <typename T>
+__global__ void __launch_bounds__(256) silu_and_mul_vec_kernel(T* __restrict__ out, const T* __restrict__ in, int rows,
+                                                                int D) {
+  constexpr int V = Vec16<T>::N;
+  const int c = blockIdx.x * 256 + threadIdx.x, nv = D / V;
+  pdl_wait();
+  pdl_open();
+  if (c >= nv) return;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+    const Vec16<T>* row = reinterpret_cast<const Vec16<T>*>(in + static_cast<size_t>(r) * 2 * D);
+    const Vec16<T> g = row[c], u = row[nv + c];
+    Vec16<T> o;
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+      const float gte = to_f32(g.at(e));
+      o.set(e, from_f32<T>(__fmul_rn(__fdiv_rn(gte, 1.f + expf(-gte)), to_f32(u.at(e)))));
+    }
+    reinterpret_cast<Vec16<T>*>(out + static_cast<size_t>(r) * D)[c] = o;
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) topk_sum_kernel(T* __restrict__ out, const T* __restrict__ in, size_t T_tokens,
                                                         int topk, int H) {
@@ -564,6 +587,17 @@ __global__ void __launch_bounds__(256) topk_sum_kernel(T* __restrict__ out, cons
     for (int j = 0; j < topk; j++) sacc = __fadd_rn(sacc, to_f32(in[(tk * topk + j) * H + h]));
     out[i] = from_f32<T>(sacc);
   }
+}
+
+// dst[r][c] = src[r][c] in 16-byte pieces, pitches in pieces; overlapped with its neighbours on the stream
+__global__ void __launch_bounds__(256) copy_rows_kernel(uint4* __restrict__ dst, size_t dst_pitch,
+                                                        const uint4* __restrict__ src, size_t src_pitch, unsigned nv,
+                                                        unsigned rows) {
+  const unsigned c = blockIdx.x * 256 + threadIdx.x;
+  pdl_wait();
+  pdl_open();
+  if (c >= nv) return;
+  for (unsigned r = blockIdx.y; r < rows; r += gridDim.y) dst[r * dst_pitch + c] = src[r * src_pitch + c];
 }
 
 inline int ew_grid(size_t total) {
@@ -691,9 +725,38 @@ int ub_silu_and_mul(void* out, const void* in, int rows, int D, int dtype, void*
   if (rows == 0 || D == 0) return ub::fail(UB_OK);
   if (!out || !in || rows < 0 || D < 0) return ub::fail(UB_ERR_INVALID_ARG);
   const size_t total = static_cast<size_t>(rows) * D;
+  const int esz = dtype == UB_DTYPE_F32 ? 4 : 2;
+  if (!((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in) | (static_cast<uintptr_t>(D) * esz)) & 15)) {
+    const int nv = D / (16 / esz);
+    const dim3 grid((nv + 255) / 256, rows < 32768 ? rows : 32768);
+    UB_DISPATCH_FLOAT(dtype, T, return ub::launch_pdl(silu_and_mul_vec_kernel<T>, grid, dim3(256), ub::as_stream(stream),
+                                                      static_cast<T*>(out), static_cast<const T*>(in), rows, D));
+  }
   UB_DISPATCH_FLOAT(dtype, T, (silu_and_mul_kernel<T><<<ew_grid(total), 256, 0, ub::as_stream(stream)>>>(
                                   static_cast<T*>(out), static_cast<const T*>(in), static_cast<size_t>(rows), D)));
   return ub::check_launch();
+}
+
+// dst[height][width] = src[height][width] bytes at the given row pitches, both in memory of the current device.  Rows of
+// whole 16-byte pieces go through a kernel that overlaps with its neighbours on the stream, others through the runtime.
+int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t height,
+                 void* stream) {
+  if (width == 0 || height == 0) return ub::fail(UB_OK);
+  if (!dst || !src || width > dst_pitch || width > src_pitch) return ub::fail(UB_ERR_INVALID_ARG);
+  const size_t bits = reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | dst_pitch | src_pitch | width;
+  if (!(bits & 15) && width < (1u << 30) && height < (1u << 30)) {
+    const unsigned nv = static_cast<unsigned>(width >> 4), rows = static_cast<unsigned>(height);
+    return ub::launch_pdl(copy_rows_kernel, dim3((nv + 255) / 256, rows < 32768 ? rows : 32768), dim3(256),
+                          ub::as_stream(stream), static_cast<uint4*>(dst), dst_pitch >> 4, static_cast<const uint4*>(src),
+                          src_pitch >> 4, nv, rows);
+  }
+  const cudaError_t e = cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, height, cudaMemcpyDeviceToDevice,
+                                          ub::as_stream(stream));
+  if (e != cudaSuccess) {
+    ub::set_cuda_error(e);
+    return ub::fail(UB_ERR_CUDA);
+  }
+  return ub::fail(UB_OK);
 }
 
 int ub_topk_sum(void* out, const void* in, int T_tokens, int topk, int H, int dtype, void* stream) {

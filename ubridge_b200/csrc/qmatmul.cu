@@ -76,6 +76,63 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(T* __restrict__ out, cons
     o[k] = ub::from_f32<T>(ub::to_f32(ub::from_f32<T>(ub::to_f32(x[k]) * scale)) * ub::to_f32(gamma[k]));
 }
 
+// The same with a CTA per row and 16-byte accesses: rows of whole 16-byte pieces, everything 16-byte aligned.  A row of up
+// to 8192 16-bit values stays in registers between the two passes, the rest of a longer one is read again.  Such a launch
+// moves some KB to some MB between two matmuls and is all latency: a warp per row took 8 us at 4096 values (128 dependent
+// rounds of 2-byte loads), this takes 2 us of which most is hidden, as both neighbours overlap with it (dependent launch).
+template <typename T>
+__global__ void __launch_bounds__(256) rms_norm_row_kernel(T* out, const T* in, const T* __restrict__ gamma, int H,
+                                                           float eps) {
+  using namespace ub;
+  constexpr int V = Vec16<T>::N, R = 4;
+  __shared__ float part[8];
+  const int nv = H / V, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_wait();
+  pdl_open();
+  const Vec16<T>* x = reinterpret_cast<const Vec16<T>*>(in + static_cast<size_t>(blockIdx.x) * H);
+  Vec16<T>* o = reinterpret_cast<Vec16<T>*>(out + static_cast<size_t>(blockIdx.x) * H);
+  const Vec16<T>* gm = reinterpret_cast<const Vec16<T>*>(gamma);
+  Vec16<T> xv[R], gv[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int c = threadIdx.x + 256 * i;
+    xv[i].r = c < nv ? x[c].r : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int c = threadIdx.x + 256 * i;
+    gv[i].r = c < nv ? gm[c].r : make_uint4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+  auto add = [&](const Vec16<T>& v) {
+#pragma unroll
+    for (int e = 0; e < V; e++) ss = fmaf(to_f32(v.at(e)), to_f32(v.at(e)), ss);
+  };
+#pragma unroll
+  for (int i = 0; i < R; i++) add(xv[i]);
+  for (int c = threadIdx.x + 256 * R; c < nv; c += 256) add(x[c]);
+  ss = warp_sum(ss);
+  if (lane == 0) part[warp] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; w++) ss += part[w];
+  const float scale = rsqrtf(ss / static_cast<float>(H) + eps);
+  auto norm = [&](const Vec16<T>& v, const Vec16<T>& g) {
+    Vec16<T> r;
+#pragma unroll
+    for (int e = 0; e < V; e++)
+      r.set(e, from_f32<T>(to_f32(from_f32<T>(to_f32(v.at(e)) * scale)) * to_f32(g.at(e))));
+    return r;
+  };
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int c = threadIdx.x + 256 * i;
+    if (c < nv) o[c] = norm(xv[i], gv[i]);
+  }
+  for (int c = threadIdx.x + 256 * R; c < nv; c += 256) o[c] = norm(x[c], gm[c]);
+}
+
 // y += r (bf16), the residual add behind a matmul that could not carry it in its epilogue
 __global__ void add_bf16_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ r, size_t n) {
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -265,8 +322,15 @@ int topsaten_rms_norm(void* output, const void* input, const void* gamma, int nu
                       int dtype_code, void* stream) {
   if (num_tokens == 0 || hidden_size == 0) return ub::fail(UB_OK);
   if (!output || !input || !gamma || num_tokens < 0 || hidden_size < 0) return ub::fail(UB_ERR_INVALID_ARG);
-  const int grid = (num_tokens + 7) / 8;
   cudaStream_t s = ub::as_stream(stream);
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(input) |
+                         reinterpret_cast<uintptr_t>(gamma) | (static_cast<uintptr_t>(hidden_size) * (dtype_code == UB_DTYPE_F32 ? 4 : 2));
+  if (!(bits & 15)) {
+    UB_DISPATCH_FLOAT(dtype_code, T, return ub::launch_pdl(rms_norm_row_kernel<T>, dim3(num_tokens), dim3(256), s,
+                                                           static_cast<T*>(output), static_cast<const T*>(input),
+                                                           static_cast<const T*>(gamma), hidden_size, epsilon));
+  }
+  const int grid = (num_tokens + 7) / 8;
   UB_DISPATCH_FLOAT(dtype_code, T, (rms_norm_kernel<T><<<grid, 256, 0, s>>>(static_cast<T*>(output),
                                                                           static_cast<const T*>(input),
                                                                           static_cast<const T*>(gamma), num_tokens,

@@ -20,7 +20,7 @@ from typing import Callable, Optional, Tuple
 import numpy as np
 
 from . import ops
-from ._lib import DTYPE_BF16
+from ._lib import DTYPE_BF16, check, lib
 
 QK = {True: 256, False: 32}
 BLOCK_BYTES = {True: 144, False: 34}
@@ -177,12 +177,8 @@ class TPLinearStack:
 
 
 def ops_copy_cols(dev, dst, src, M: int, src_cols: int, cols: int) -> None:
-    """dst[M, cols] = src[M, :cols] for bf16 rows (one strided device copy)."""
-    import ctypes
-
-    from ._lib import check, lib
-    check(lib().ub_memcpy_dtod_2d(dev._handle, ctypes.c_void_p(dst.ptr), cols * 2, ctypes.c_void_p(src.ptr),
-                                  src_cols * 2, cols * 2, M), "dtod_2d")
+    """dst[M, cols] = src[M, :cols] for bf16 rows."""
+    check(lib().ub_copy_rows(dst.ptr, cols * 2, src.ptr, src_cols * 2, cols * 2, M, dev.stream), "copy_rows")
 
 
 class EPMoELayer:
