@@ -13,15 +13,24 @@
 // The token tile is the "B" operand (N = TOK <= 256, trimmed to the valid tokens of a ragged last tile),
 // K-major bf16 in the 128-byte-swizzled canonical layout, written to shared memory by 2-D tensor-map
 // copies.  The accumulator D[128 lanes x TOK columns] lives in tensor memory next to the weight stages
-// (columns 0..255 accumulators, 256.. weight stages of 32 columns each).  K is consumed 64 values per
-// stage (one 64-value Q4_K group), four UMMA K=16 steps each.
+// (columns 0..255 accumulators, 256.. weight stages of 64 columns each).  A weight stage holds 128 K values (two
+// 64-value groups), a token stage 64; each token stage is four UMMA K=16 steps.
+//
+// What bounds it.  An MMA of 128 x 256 x 16 takes 128 cycles of the tensor pipe, a weight stage 1024.  A producer warp
+// needs about 830 for it: 500 for the arithmetic of 64 values per thread and 75 to 150 for each barrier it looks at and for
+// the stores to land, whatever they carry.  With stages of 64 values that chain was 700 cycles against 512 of MMAs: the
+// producers held the tensor pipe back.  Three changes took 2048 tokens at 14336x4096 from 190 to 181 us and 512 tokens at
+// 57344x8192 from 376 to 346 us: weight stages of 128 values; one thread per 64-value group (both nibble halves from the
+// same words) in code that is not unrolled over the groups of a super-block (instruction fetch); and the issuing thread
+// chosen by elect.sync.  Up to 128 tokens (Q8_0: 64) run in qgemm_tc2.cu.
 //
 //   warp 0        allocates TMEM, then one elected lane issues tcgen05.mma and tcgen05.commit
 //   warps 1-4     epilogue: tcgen05.ld -> bf16 -> staging tile in shared memory (accumulator released
 //                 here) -> 16-byte coalesced stores to y, overlapping the next tile's main loop
 //   warps 5-12    weight producers: read their row's packed super-block from a shared-memory ring, turn
 //                 nibbles into bf16 (128 + q) with one byte permute per pair, minus 128 (exact), times d*sc
-//                 minus dmin*m with packed bf16 FMAs; tcgen05.st, tcgen05.wait::st, mbarrier arrive
+//                 minus dmin*m with packed bf16 FMAs; tcgen05.st; the stage is handed over (tcgen05.wait::st, mbarrier
+//                 arrive) after the next one's arithmetic
 //   warp 13       one lane issues all bulk copies: packed weight tiles ([128 rows][144 bytes], one 2-D
 //                 tensor-map copy per super-block column, two super-blocks ahead) and token tiles (one
 //                 copy per K step, as far ahead as the ring allows)
@@ -31,7 +40,6 @@
 #include <string.h>
 
 #include <mutex>
-#include <type_traits>
 
 #include "rowblock.cuh"
 
@@ -39,16 +47,11 @@ namespace {
 
 using namespace ub;
 
-constexpr int kTcProducerWarps = 8;   // warps that dequantise one K step (128 rows x 2 nibble halves)
-// Sets of such warps (template parameter SETS); set i takes the K steps with step % SETS == i.  Measured on B200:
-// a second set does not help, neither with 256-token tiles (C3 204 us against 191 us with one) nor with 16 to 128
-// tokens (14336x4096: 27.9 us against 26.1 us at 16 tokens, where a K step takes 0.42 us whatever the token
-// count: 0.20 us of producer arithmetic, 0.10 us until tcgen05.st has landed, 0.20 us for the issuing thread to
-// get four MMAs and a commit out).  Every launch uses one set.
-constexpr int tc_threads(int sets) { return (5 + kTcProducerWarps * sets + 1) * 32; }
+constexpr int kTcProducerWarps = 8;   // warps that dequantise a weight stage (128 rows x two 64-value groups)
+constexpr int kTcThreads = (5 + kTcProducerWarps + 1) * 32;
 constexpr int kTcBK = 64;
 
-constexpr int kTcMaxStages = 8;
+constexpr int kTcMaxStages = 8, kTcMaxAStages = 4;
 constexpr int kTcWStages = 8;                        // most slots a ring of packed weight tiles has
 // Shared-memory plan per token-tile size: the 256-token tile spends its memory on token stages (the
 // copies' latency, not their bandwidth, bounds a K step) and keeps the other two areas small.
@@ -59,8 +62,8 @@ constexpr int tc_stage_tok(int tok, int ctas) {  // staging rows
   return (tok > 128 || ctas > 1) ? 64 : (tok < 128 ? tok : 128);
 }
 // Shared memory of a launch: token stages, output staging tile, packed-weight ring, 1 KB for alignment.
-constexpr size_t tc_smem_bytes(int tok, int stages, int ctas, int wst, int fmt, int kg) {
-  return static_cast<size_t>(stages) * (tok * 128 * kg) + static_cast<size_t>(tc_stage_tok(tok, ctas)) * 256 +
+constexpr size_t tc_smem_bytes(int tok, int stages, int ctas, int wst, int fmt) {
+  return static_cast<size_t>(stages) * (tok * 128) + static_cast<size_t>(tc_stage_tok(tok, ctas)) * 256 +
          static_cast<size_t>(tc_wstages(tok, ctas, wst)) * (128 * (fmt ? 8 * 34 : 144)) + 1024;
 }
 // One slot of the packed-weight ring holds 256 K values of 128 rows: a Q4_K super-block (144 bytes) or eight
@@ -87,7 +90,9 @@ struct TcRun {
 };
 
 struct TcShared {
-  unsigned long long full[kTcMaxStages], empty[kTcMaxStages], tmem_full[2], tmem_empty[2];
+  unsigned long long full[kTcMaxStages], empty[kTcMaxStages];    // token stages
+  unsigned long long afull[kTcMaxAStages], aempty[kTcMaxAStages];  // weight stages in tensor memory
+  unsigned long long tmem_full[2], tmem_empty[2];
   unsigned long long wfull[kTcWStages], wempty[kTcWStages];
   uint32_t tmem_base;
   int abort_flag;
@@ -104,9 +109,10 @@ struct TcShared {
 // help (MoE layer of 256 tokens, one CTA per SM: 3 -> 5 slots 589 -> 567 us; dense M = 2048: 2 -> 4 slots no
 // change), the packed tiles are not what a K step waits for.
 // FMT: 0 = Q4_K super-blocks, 1 = Q8_0 blocks (dense mode only).
-// KG: 64-value groups of K per pipeline step.  A step costs the same barrier round trips whatever it computes.
-template <int TOK, int STAGES, int MODE, int CTAS, int WST, int FMT, int SETS, int KG>
-__global__ void __launch_bounds__(tc_threads(SETS), CTAS)
+// AST: weight stages in tensor memory.  One holds 128 K values (64 columns) and is written by the eight producer warps, a
+// thread one 64-value group of its row; token stages hold 64 K values.
+template <int TOK, int STAGES, int MODE, int CTAS, int WST, int FMT, int AST>
+__global__ void __launch_bounds__(kTcThreads, CTAS)
 qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err_word,
                     const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
                     const TcGroup grp) {
@@ -116,10 +122,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
   __shared__ float run_w[MODE == 2 ? TOK : 1];
   __shared__ int run_dst[MODE == 2 ? TOK : 1];
   static_assert(STAGES <= kTcMaxStages, "barrier arrays");
-  constexpr uint32_t kBGroup = TOK * 128;              // TOK token rows x 64 bf16
-  constexpr uint32_t kBBytes = kBGroup * KG;
-  constexpr int kOwn = 4 / KG / SETS;                  // steps of a super-block that a set takes: kOwn * set, ...
-  static_assert(kOwn >= 1, "every set has a step of each super-block");
+  constexpr uint32_t kBBytes = TOK * 128;              // TOK token rows x 64 bf16
   constexpr int kStageTok = tc_stage_tok(TOK, CTAS);   // tokens the output staging tile holds
   constexpr int kWStages = tc_wstages(TOK, CTAS, WST);
   static_assert(kWStages <= kTcWStages, "barrier arrays");
@@ -131,8 +134,8 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
   constexpr int kAccBufs = (TOK > 128 || CTAS > 1) ? 1 : 2;  // accumulator buffers at the start of the allocation
   constexpr uint32_t kAccStride = 128;
   constexpr uint32_t kTmemCols = CTAS > 1 ? 256 : 512;        // columns this CTA allocates
-  constexpr uint32_t kATmemCol = CTAS > 1 ? 128 : 256;        // first column of the weight stages (32 KG each)
-  static_assert(TOK * kAccBufs <= static_cast<int>(kATmemCol) && kATmemCol + 32 * KG * STAGES <= kTmemCols, "TMEM plan");
+  constexpr uint32_t kATmemCol = CTAS > 1 ? 128 : 256;        // first column of the weight stages (64 each)
+  static_assert(TOK * kAccBufs <= static_cast<int>(kATmemCol) && kATmemCol + 64 * AST <= kTmemCols && AST <= kTcMaxAStages, "TMEM plan");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the swizzled tiles need 1024-byte alignment; the launch reserves 1 KB of slack for rounding the base up
   const uint32_t smem_raw = static_cast<uint32_t>(__cvta_generic_to_shared(tc_smem));
@@ -141,16 +144,18 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
   const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(&sh));
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * kTcMaxStages + 8u * s; };
-  auto tfull_bar = [&](int b) { return bars + 16u * kTcMaxStages + 8u * b; };
-  auto tempty_bar = [&](int b) { return bars + 16u * kTcMaxStages + 16u + 8u * b; };
-  auto wfull_bar = [&](int b) { return bars + 16u * kTcMaxStages + 32u + 8u * b; };
-  auto wempty_bar = [&](int b) { return bars + 16u * kTcMaxStages + 32u + 8u * kTcWStages + 8u * b; };
+  auto afull_bar = [&](int b) { return bars + 16u * kTcMaxStages + 8u * b; };
+  auto aempty_bar = [&](int b) { return afull_bar(kTcMaxAStages + b); };
+  auto tfull_bar = [&](int b) { return afull_bar(2 * kTcMaxAStages + b); };
+  auto tempty_bar = [&](int b) { return tfull_bar(2 + b); };
+  auto wfull_bar = [&](int b) { return tfull_bar(4 + b); };
+  auto wempty_bar = [&](int b) { return wfull_bar(kTcWStages + b); };
   const int vblock = static_cast<int>(blockIdx.x), vgrid = static_cast<int>(gridDim.x);
   volatile int* abort_flag = &sh.abort_flag;
 
   constexpr int kTileCols = MODE == 1 ? 64 : 128;  // output columns per tile
   const int w_tiles = (N + kTileCols - 1) / kTileCols, t_tiles = (M + TOK - 1) / TOK;
-  const int ksteps = K / (kTcBK * KG);
+  const int ksteps = K / (2 * kTcBK);
 
   if (MODE != 0) {
     // Token runs: consecutive alignment blocks of one expert, merged up to TOK tokens.  Every CTA builds
@@ -159,7 +164,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
     const int padded = *grp.num_post_pad;
     int nblocks = padded > 0 ? (padded + grp.block - 1) / grp.block : 0;
     if (nblocks > kTcMaxRuns) nblocks = kTcMaxRuns;  // the launcher guarantees this never cuts
-    for (int i = threadIdx.x; i < nblocks; i += tc_threads(SETS)) ids[i] = grp.experts_ids[i];
+    for (int i = threadIdx.x; i < nblocks; i += kTcThreads) ids[i] = grp.experts_ids[i];
     __syncthreads();
     if (threadIdx.x == 0) {
       int n = 0;
@@ -193,8 +198,12 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
-      tc_mbar_init(full_bar(s), kTcProducerWarps + 1);  // eight weight warps + the token copy's expect_tx
+      tc_mbar_init(full_bar(s), 1);
       tc_mbar_init(empty_bar(s), 1);
+    }
+    for (int s = 0; s < AST; s++) {
+      tc_mbar_init(afull_bar(s), kTcProducerWarps);
+      tc_mbar_init(aempty_bar(s), 1);
     }
     for (int b = 0; b < 2; b++) {
       tc_mbar_init(tfull_bar(b), 1);
@@ -202,7 +211,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
     }
     for (int b = 0; b < kWStages; b++) {
       tc_mbar_init(wfull_bar(b), 1);
-      tc_mbar_init(wempty_bar(b), kTcProducerWarps * SETS);
+      tc_mbar_init(wempty_bar(b), kTcProducerWarps);
     }
     sh.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -219,9 +228,9 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
   const uint32_t tmem_base = sh.tmem_base;
   if (warp == 0) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int s = 0;
-      uint32_t phase = 0, acc_phase = 0;
+    if (elect_one()) {
+      int s = 0, as = 0;
+      uint32_t phase = 0, aphase = 0, acc_phase = 0;
       int buf = 0;
       bool ok = true;
       for (int tile = vblock; tile < ntiles && ok; tile += vgrid) {
@@ -236,21 +245,28 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf) * kAccStride;
         for (int ks = 0; ks < ksteps; ks++) {
-          ok = tc_wait(full_bar(s), phase, abort_flag);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_tmem = tmem_base + kATmemCol + 32u * KG * s;
+          ok = tc_wait(afull_bar(as), aphase, abort_flag);
+          const uint32_t a_tmem = tmem_base + kATmemCol + 64u * as;
 #pragma unroll
-          for (int g = 0; g < KG; g++) {
-            const uint64_t b_desc = make_sw128_desc(smem_base + s * kBBytes + g * kBGroup);
+          for (int g = 0; g < 2; g++) {
+            if (ok) ok = tc_wait(full_bar(s), phase, abort_flag);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t b_desc = make_sw128_desc(smem_base + s * kBBytes);
 #pragma unroll
             for (int j = 0; j < 4; j++)  // K = 16 per instruction: 8 TMEM columns of A, 32 bytes of a B row
               umma_bf16_ts(d_tmem, a_tmem + 32u * g + 8u * j, b_desc + 2 * j, idesc, (ks > 0 || g > 0 || j > 0) ? 1u : 0u);
+            umma_commit(empty_bar(s));  // stage is free once these MMAs have read it
+            if (++s == STAGES) {
+              s = 0;
+              phase ^= 1;
+            }
           }
-          umma_commit(empty_bar(s));  // stage is free once these MMAs have read it
-          if (++s == STAGES) {
-            s = 0;
-            phase ^= 1;
+          if (!ok) break;
+          umma_commit(aempty_bar(as));
+          if (++as == AST) {
+            as = 0;
+            aphase ^= 1;
           }
         }
         if (!ok) break;
@@ -364,112 +380,63 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
         acc_phase ^= 1;
       }
     }
-  } else if (warp <= 4 + kTcProducerWarps * SETS) {
+  } else if (warp <= 4 + kTcProducerWarps) {
     // ------------------------------------------------------------ weight producers (256 threads per set)
-    // One flat loop over (tile, super-block); the super-block's four K steps (its four 64-value groups) are
-    // dealt round robin to the producer sets.  Packed weights arrive in shared memory as
-    // [128 rows][144 bytes] per super-block; a thread owns one weight row (= its TMEM lane) and one nibble
-    // half and reads its row's header and 32-byte pieces from there (rows are 144 bytes apart, so a
+    // One flat loop over (tile, super-block), two weight stages of 128 values each.  Packed weights arrive in shared memory
+    // as [128 rows][144 bytes] per super-block; a thread owns one weight row (= its TMEM lane) and one of a stage's two
+    // 64-value groups and reads its row's header and 32-byte pieces from there (rows are 144 bytes apart, so a
     // quarter-warp's 16-byte reads hit all 32 banks once).
     // weight row inside the tile = the TMEM lane this warp may access (32 * (warp % 4) + lane);
-    // half: 0 = low nibbles (even sub-blocks), 1 = high nibbles
-    const int wrow = 32 * (warp & 3) + lane, half = ((warp - 5) >> 2) & 1, set = (warp - 5) >> 3;
+    // gsel: which group of a stage
+    const int wrow = 32 * (warp & 3) + lane, gsel = (warp - 5) >> 2;
     const int nsb = K >> 8;
     const int my_tiles = vblock < ntiles ? (ntiles - vblock + vgrid - 1) / vgrid : 0;
     const int total_sb = my_tiles * nsb;  // super-block iterations
-    const unsigned char* const w_ring = tiles + kWOff + wrow * kWRow;
-    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kATmemCol;
+    const uint32_t w_ring = smem_base + kWOff + wrow * kWRow;
+    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kATmemCol + 32u * gsel;
 
-    int s = kOwn * set;  // stage of the step being dequantised
+    int s = 0;  // weight stage being filled
     uint32_t phase = 0;
     int ws = 0;  // packed-weight ring slot
     uint32_t wphase = 0;
     bool ok = true;
-
-    // one super-block (four K steps); HALF is a compile-time copy of `half` so that nibble selection and
-    // the scale bytes' positions are immediate operands.  (Measured on B200: one rolled code path for both
-    // halves, with the half as a run-time shift, is no faster, although instruction fetch is the second largest
-    // stall of the grouped launches.)
-    auto super_block = [&](auto half_c, auto set_c) {
-      constexpr int HALF = decltype(half_c)::value, SET = decltype(set_c)::value;
-      ok = __all_sync(0xFFFFFFFFu, tc_wait(wfull_bar(ws), wphase, abort_flag));
-      if (!ok) return;
-      const unsigned char* blk = w_ring + ws * kTcWBytes;
-      uint32_t scw[2] = {0, 0}, mnw[2] = {0, 0};
-      float d = 0.f, dmin = 0.f;
-      if (FMT == 0) {
-        const uint4 hdr = *reinterpret_cast<const uint4*>(blk);  // rows past N arrive as zeros: d = dmin = 0
-        d = half_bits_to_f32(hdr.x), dmin = half_bits_to_f32(hdr.x >> 16);
-        q4k_unpack_scales(hdr.y, hdr.z, hdr.w, scw[0], scw[1], mnw[0], mnw[1]);
+    // A stage's stores land while the next one is computed; it is handed to the MMAs after that.
+    int due = -1;
+    auto hand_over = [&]() {
+      if (due < 0) return;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc_mbar_arrive(afull_bar(due));
+      due = -1;
+    };
+    for (int q = 0; q < total_sb && ok; q++) {
+      if (!__all_sync(0xFFFFFFFFu, tc_mbar_test(wfull_bar(ws), wphase))) {
+        hand_over();
+        ok = __all_sync(0xFFFFFFFFu, tc_wait(wfull_bar(ws), wphase, abort_flag));
+        if (!ok) break;
       }
+      RowBlock<FMT> blk;  // rows past N arrive as zeros: d = dmin = 0
+      blk.open(w_ring + ws * kTcWBytes);
 #pragma unroll
-      for (int Gi = 0; Gi < kOwn; Gi++) {
-        uint32_t ots[KG][16];  // this thread's 32 values of each group = 16 TMEM columns of packed pairs
-#pragma unroll
-        for (int g = 0; g < KG; g++) {
-        const int G = KG * (kOwn * SET + Gi) + g;
-        uint32_t (&ot)[16] = ots[g];
-        if (FMT == 0) {
-          const int j = 2 * G + HALF;
-          const uint32_t sc = (scw[j >> 2] >> (8 * (j & 3))) & 0xFF, mn = (mnw[j >> 2] >> (8 * (j & 3))) & 0xFF;
-          const __nv_bfloat162 dsc = __float2bfloat162_rn(d * static_cast<float>(sc));
-          const __nv_bfloat162 ndm = __float2bfloat162_rn(-dmin * static_cast<float>(mn));
-          const uint4 qa = *reinterpret_cast<const uint4*>(blk + 16 + 32 * G);
-          const uint4 qb = *reinterpret_cast<const uint4*>(blk + 32 + 32 * G);
-          const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#pragma unroll
-          for (int cc = 0; cc < 4; cc++) {  // 8 values = bytes 8cc .. 8cc+7
-            const uint32_t w0 = HALF ? (w[2 * cc] >> 4) & 0x0F0F0F0Fu : w[2 * cc] & 0x0F0F0F0Fu;
-            const uint32_t w1 = HALF ? (w[2 * cc + 1] >> 4) & 0x0F0F0F0Fu : w[2 * cc + 1] & 0x0F0F0F0Fu;
-            ot[4 * cc] = deq_pair<0x4140>(w0, dsc, ndm);
-            ot[4 * cc + 1] = deq_pair<0x4342>(w0, dsc, ndm);
-            ot[4 * cc + 2] = deq_pair<0x4140>(w1, dsc, ndm);
-            ot[4 * cc + 3] = deq_pair<0x4342>(w1, dsc, ndm);
-          }
-        } else {
-          // Q8_0 block 2G + HALF of the row's eight: 34 bytes at byte 34 (2G + HALF) of a 272-byte row, i.e. three
-          // aligned 16-byte pieces from piece (34 (2G + HALF)) / 16; inside them the f16 scale sits at byte
-          // 4G + 2 HALF and the 32 signed bytes follow it, so the even blocks' words straddle two loaded words.
-          const uint4* pc = reinterpret_cast<const uint4*>(blk) + ((34 * (2 * G + HALF)) >> 4);
-          const uint4 p0 = pc[0], p1 = pc[1], p2 = pc[2];
-          const uint32_t c[12] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y, p2.z, p2.w};
-          const float df = half_bits_to_f32(HALF ? c[G] >> 16 : c[G]);
-          const __nv_bfloat16 dh1 = __float2bfloat16_rn(df);
-          // d = dh + dl in two bf16 pieces: fma(q, dh, q * dl) is the f32 product d * q rounded once
-          const __nv_bfloat162 dh = __bfloat162bfloat162(dh1);
-          const __nv_bfloat162 dl = __float2bfloat162_rn(df - __bfloat162float(dh1));
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const uint32_t w = HALF ? c[G + 1 + i] : __funnelshift_r(c[G + i], c[G + i + 1], 16);
-            const uint32_t lo7 = w & 0x7F7F7F7Fu, sg = w & 0x80808080u;
-            ot[2 * i] = deq8_pair<0x4140>(lo7, sg, dh, dl);
-            ot[2 * i + 1] = deq8_pair<0x4342>(lo7, sg, dh, dl);
-          }
-        }
-        }
-        if (Gi == kOwn - 1) {  // this warp has read all it needs from the slot
+      for (int i = 0; i < 2; i++) {
+        // the MMAs that read this weight stage one ring turn ago must have completed: a look ahead of the arithmetic, whose
+        // answer takes 120 cycles
+        const bool ready = tc_mbar_test(aempty_bar(s), phase ^ 1);
+        uint32_t ot[32];  // this thread's 64 values = 32 TMEM columns of packed pairs
+        blk.one_piece(2 * i + gsel, ot);
+        if (i == 1) {  // this warp has read all it needs from the slot
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(wempty_bar(ws));
         }
-        // the MMAs that read this weight stage one ring turn ago must have completed
-        ok = __all_sync(0xFFFFFFFFu, tc_wait(empty_bar(s), phase ^ 1, abort_flag));
-        if (!ok) return;
+        hand_over();
+        if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, tc_wait(aempty_bar(s), phase ^ 1, abort_flag));
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int g = 0; g < KG; g++) tmem_st16(a_lane + 32u * KG * s + 32u * g + 16u * HALF, ots[g]);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) tc_mbar_arrive(full_bar(s));
-        if (++s == STAGES) {
+        tmem_st32(a_lane + 64u * s, ot);
+        due = s;
+        if (++s == AST) {
           s = 0;
-          phase ^= 1;
-        }
-      }
-      if (SETS > 1) {  // the other sets' steps
-        s += 4 / KG - kOwn;
-        if (s >= STAGES) {
-          s -= STAGES;
           phase ^= 1;
         }
       }
@@ -477,28 +444,14 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
         ws = 0;
         wphase ^= 1;
       }
-    };
-    using I0 = std::integral_constant<int, 0>;
-    using I1 = std::integral_constant<int, 1>;
-    if (SETS == 1 || set == 0) {
-      if (half) {
-        for (int q = 0; q < total_sb && ok; q++) super_block(I1{}, I0{});
-      } else {
-        for (int q = 0; q < total_sb && ok; q++) super_block(I0{}, I0{});
-      }
-    } else if constexpr (SETS > 1) {
-      if (half) {
-        for (int q = 0; q < total_sb && ok; q++) super_block(I1{}, I1{});
-      } else {
-        for (int q = 0; q < total_sb && ok; q++) super_block(I0{}, I1{});
-      }
     }
+    hand_over();
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   } else {
     // ------------------------------------------------------------ bulk copies (one lane)
     // Packed weight tiles run kWStages - 1 super-blocks ahead of the token tiles; token tiles run as far
     // ahead of the MMA as the ring allows.
-    if (lane == 0) {
+    if (elect_one()) {
       const int nsb = K >> 8;
       const int my_tiles = vblock < ntiles ? (ntiles - vblock + vgrid - 1) / vgrid : 0;
       const int total_sb = my_tiles * nsb;
@@ -539,21 +492,19 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
         int m0, valid, wrow0_, n0_;
         tile_info(vblock + ti * vgrid, m0, valid, wrow0_, n0_);
         const int boxes = MODE == 0 ? 1 : (valid + 63) >> 6;  // grouped modes: boxes of 64 tokens, no more than the run has
-        for (int G = 0; G < 4 / KG; G++) {
+        for (int G = 0; G < 4; G++) {
           ok = tc_wait(empty_bar(s), phase ^ 1, abort_flag);
           if (!ok) break;
           const uint32_t bar = full_bar(s);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                       "r"(MODE == 0 ? kBBytes : static_cast<uint32_t>(boxes * 64 * 128 * KG))
+                       "r"(MODE == 0 ? kBBytes : static_cast<uint32_t>(boxes * 64 * 128))
                        : "memory");
-#pragma unroll
-          for (int g = 0; g < KG; g++)
-            for (int b = 0; b < boxes; b++)
-              asm volatile(
-                  "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
-                      "r"(smem_base + s * kBBytes + g * kBGroup + b * (64 * 128)),
-                  "l"(reinterpret_cast<uint64_t>(&x_map)), "r"(bar), "r"((sb * 4 + G * KG + g) * kTcBK), "r"(m0 + 64 * b)
-                  : "memory");
+          for (int b = 0; b < boxes; b++)
+            asm volatile(
+                "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
+                    "r"(smem_base + s * kBBytes + b * (64 * 128)),
+                "l"(reinterpret_cast<uint64_t>(&x_map)), "r"(bar), "r"((sb * 4 + G) * kTcBK), "r"(m0 + 64 * b)
+                : "memory");
           if (++s == STAGES) {
             s = 0;
             phase ^= 1;
@@ -590,10 +541,11 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-template <int TOK, int STAGES, int MODE, int CTAS = 1, int WST = 0, int FMT = 0, int SETS = 1, int KG = 1>
+template <int TOK, int STAGES, int MODE, int CTAS = 1, int WST = 0, int FMT = 0>
 int launch_tc(void* y, const void* x, const void* wq, int M, int N, int K, const TcGroup& grp, int w_rows_total,
               cudaStream_t s) {
-  constexpr size_t smem = tc_smem_bytes(TOK, STAGES, CTAS, WST, FMT, KG);
+  constexpr size_t smem = tc_smem_bytes(TOK, STAGES, CTAS, WST, FMT);
+  constexpr int kAst = CTAS > 1 ? 2 : 4;
   static_assert(smem <= 227 * 1024 / CTAS, "shared memory plan");
   const int sms = ub::num_sms();
   int grid = sms * CTAS;  // grouped launches learn their tile count on the device; idle CTAs leave at once
@@ -628,13 +580,13 @@ int launch_tc(void* y, const void* x, const void* wq, int M, int N, int K, const
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return ub::fail(UB_ERR_UNSUPPORTED);
-  auto kernel = qgemm_q4k_tc_kernel<TOK, STAGES, MODE, CTAS, WST, FMT, SETS, KG>;
+  auto kernel = qgemm_q4k_tc_kernel<TOK, STAGES, MODE, CTAS, WST, FMT, kAst>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) {
     ub::set_cuda_error(e);
     return ub::fail(UB_ERR_CUDA);
   }
-  kernel<<<grid, tc_threads(SETS), smem, s>>>(static_cast<__nv_bfloat16*>(y), M, N, K, ub::device_error_word(), map,
+  kernel<<<grid, kTcThreads, smem, s>>>(static_cast<__nv_bfloat16*>(y), M, N, K, ub::device_error_word(), map,
                                         wmap, grp);
   return ub::check_launch();
 }
