@@ -22,7 +22,8 @@
 // producers held the tensor pipe back.  Three changes took 2048 tokens at 14336x4096 from 190 to 181 us and 512 tokens at
 // 57344x8192 from 376 to 346 us: weight stages of 128 values; one thread per 64-value group (both nibble halves from the
 // same words) in code that is not unrolled over the groups of a super-block (instruction fetch); and the issuing thread
-// chosen by elect.sync.  Up to 128 tokens (Q8_0: 64) run in qgemm_tc2.cu.
+// chosen by elect.sync.  Dense launches of few tiles run in
+// qgemm_tc2.cu (q4k_gemm_tc, q8_0_gemm_tc).
 //
 //   warp 0        allocates TMEM, then one elected lane issues tcgen05.mma and tcgen05.commit
 //   warps 1-4     epilogue: tcgen05.ld -> bf16 -> staging tile in shared memory (accumulator released
@@ -618,7 +619,11 @@ void* tensor_map_encoder() { return reinterpret_cast<void*>(encode_tiled_fn()); 
 // Returns UB_ERR_UNSUPPORTED when the driver offers no tensor-map encoder (the caller falls back).
 int q4k_gemm_tc1(int fmt, void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
 int q4k_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s) {
-  if (M <= 128) return q4k_gemm_tc1(12, y, x, wq, M, N, K, fresh, s);
+  // 128-token tiles (with a K split where they leave half of the SMs idle) while one round of CTAs holds all of them: 256-token
+  // tiles would leave SMs without one.  Measured on B200, us, 128- / 256-token tiles: 4096 rows of 4096 values with 130
+  // tokens 15.9 / 22.4, 256 18.8 / 27.1, 512 22.8 / 28.8; 4096x14336 with 200 tokens 37 / 63; 6144x4096 with 384 23.2 / 28.8.
+  const int tiles128 = (N + 127) / 128 * ((M + 127) / 128);
+  if (M <= 128 || tiles128 <= ub::num_sms()) return q4k_gemm_tc1(12, y, x, wq, M, N, K, fresh, s);
   const TcGroup none = {nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
   return launch_tc<256, 5, 0>(y, x, wq, M, N, K, none, N, s);
 }
