@@ -227,8 +227,6 @@ __global__ void bf16_to_f32_kernel(float* __restrict__ out, const __nv_bfloat16*
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-constexpr int kMoeFewTokens = 4;  // most tokens that ub_moe_layer_q4k takes one at a time
-
 }  // namespace
 
 namespace ub {
@@ -346,12 +344,13 @@ int ub_moe_layer_q4k(void* out, const void* hidden, const void* router_logits, c
 
   int st = ub::topk_softmax_bf16_impl(router_logits, w_t, idx, T, E, top_k, norm_topk_prob != 0, s);
   if (st != UB_OK) return st;
-  // Few tokens: a token at a time through the one-token kernels, each token's experts read at streaming speed.  Beyond, the
-  // grouped kernel's cost grows with the experts touched and not with the tokens.  Measured on B200, 8 experts top-2,
-  // 4096 / 14336, us per layer: one token 54 against 206; the layer of four tokens takes four times that, 190, as the grouped
-  // kernel for the seven experts that four to eight tokens touch takes more than 300.
-  if (T <= kMoeFewTokens && !((reinterpret_cast<uintptr_t>(w13q) | reinterpret_cast<uintptr_t>(w2q) |
-                                   reinterpret_cast<uintptr_t>(hidden)) & 15)) {
+  // Few tokens: a token at a time through the one-token kernels, each slot's expert read at streaming speed, against a
+  // fixed cost of about five slots and a little more than one per expert touched of the grouped kernels.  Measured on B200,
+  // 8 experts top-2, 4096 / 14336, us per layer, this way / grouped: one token 54 / 204, two 103 / 236, four 199 / 288,
+  // eight 400 / 362; 1024 / 1024: two tokens 21 / 51, four 36 / 53.
+  const size_t touched = slots < static_cast<size_t>(E) ? slots : static_cast<size_t>(E);
+  if (slots <= 5 + 9 * touched / 10 && !((reinterpret_cast<uintptr_t>(w13q) | reinterpret_cast<uintptr_t>(w2q) |
+                                          reinterpret_cast<uintptr_t>(hidden)) & 15)) {
     for (int t = 0; t < T; t++) {
       st = ub::q4k_moe_one_token(static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(t) * H, act,
                                  static_cast<const __nv_bfloat16*>(hidden) + static_cast<size_t>(t) * H, w13q, w2q,
