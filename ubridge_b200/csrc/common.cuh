@@ -46,9 +46,9 @@ __device__ __forceinline__ void report_device_error(int* err_word, int code) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
-inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+inline int launch_pdl_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid, cfg.blockDim = block, cfg.stream = s;
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = s;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -59,6 +59,11 @@ inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t 
     return fail(UB_ERR_CUDA);
   }
   return check_launch();
+}
+
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+  return launch_pdl_smem(kernel, grid, block, 0, s, args...);
 }
 
 // ---- 16 bytes of a storage type ----

@@ -97,6 +97,8 @@ __global__ void __launch_bounds__(128) topk_softmax_kernel(const T* __restrict__
   }
 }
 
+// An ordinary launch: as a dependent one it let the expert kernels behind it take their place on the SMs early, which cost
+// the one-token expert layer 2 of 54 us.
 template <typename T>
 int topk_softmax_launch(const void* in, void* out_w, int* out_idx, int T_tokens, int E, int k, int norm,
                         cudaStream_t s, int* out_src = nullptr) {
@@ -144,6 +146,8 @@ __global__ void __launch_bounds__(kAlignThreads) moe_align_kernel(
   const int pad_value = T * k;
   const int max_padded = T * k + E * (block - 1);
   const int max_blocks = max_padded / block;
+  pdl_wait();
+  pdl_open();
   int tn = T;
   if (real_token_num) {
     tn = *real_token_num;
@@ -244,10 +248,8 @@ int moe_align_launch(int32_t* sorted_ids, int32_t* experts_ids, int32_t* num_pos
     }
   }
   const int blocks = E < 64 ? E : 64;
-  moe_align_kernel<<<blocks, kAlignThreads, smem, s>>>(sorted_ids, experts_ids, num_post_pad, topk_ids,
-                                                       real_token_num, expert_map, E, block, T, k,
-                                                       ub::device_error_word());
-  return ub::check_launch();
+  return ub::launch_pdl_smem(moe_align_kernel, dim3(blocks), dim3(kAlignThreads), smem, s, sorted_ids, experts_ids,
+                             num_post_pad, topk_ids, real_token_num, expert_map, E, block, T, k, ub::device_error_word());
 }
 
 // ------------------------------------------------------------------ dense grouped GEMM (reference signature)
@@ -579,6 +581,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) topk_sum_kernel(T* __restrict__ out, const T* __restrict__ in, size_t T_tokens,
                                                         int topk, int H) {
   const size_t total = T_tokens * H;
+  pdl_wait();
+  pdl_open();
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const size_t tk = i / H;
@@ -763,9 +767,9 @@ int ub_topk_sum(void* out, const void* in, int T_tokens, int topk, int H, int dt
   if (T_tokens == 0 || H == 0) return ub::fail(UB_OK);
   if (!out || !in || T_tokens < 0 || topk <= 0 || H < 0) return ub::fail(UB_ERR_INVALID_ARG);
   const size_t total = static_cast<size_t>(T_tokens) * H;
-  UB_DISPATCH_FLOAT(dtype, T, (topk_sum_kernel<T><<<ew_grid(total), 256, 0, ub::as_stream(stream)>>>(
-                                  static_cast<T*>(out), static_cast<const T*>(in), static_cast<size_t>(T_tokens), topk,
-                                  H)));
+  UB_DISPATCH_FLOAT(dtype, T, return ub::launch_pdl(topk_sum_kernel<T>, dim3(ew_grid(total)), dim3(256),
+                                                    ub::as_stream(stream), static_cast<T*>(out), static_cast<const T*>(in),
+                                                    static_cast<size_t>(T_tokens), topk, H));
   return ub::check_launch();
 }
 

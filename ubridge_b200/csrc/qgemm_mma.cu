@@ -222,6 +222,8 @@ __global__ void __launch_bounds__(128) q4k_grouped_mma_kernel(
 
 __global__ void bf16_to_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ in, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_open();
   if (i < n) out[i] = __bfloat162float(in[i]);
 }
 
@@ -359,7 +361,9 @@ int ub_moe_layer_q4k(void* out, const void* hidden, const void* router_logits, c
     }
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
-  bf16_to_f32_kernel<<<static_cast<int>((slots + 255) / 256), 256, 0, s>>>(w_f32, w_t, static_cast<int>(slots));
+  st = ub::launch_pdl(bf16_to_f32_kernel, dim3(static_cast<unsigned>((slots + 255) / 256)), dim3(256), s, w_f32, w_t,
+                      static_cast<int>(slots));
+  if (st != UB_OK) return st;
   st = ub::moe_align(sorted_ids, experts_ids, npp, idx, nullptr, expert_map, E, block_size, T, top_k, s);
   if (st != UB_OK) return st;
   const int positions = static_cast<int>(max_padded);

@@ -154,6 +154,8 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
   const int vblock = static_cast<int>(blockIdx.x), vgrid = static_cast<int>(gridDim.x);
   volatile int* abort_flag = &sh.abort_flag;
 
+  pdl_wait();
+  pdl_open();
   constexpr int kTileCols = MODE == 1 ? 64 : 128;  // output columns per tile
   const int w_tiles = (N + kTileCols - 1) / kTileCols, t_tiles = (M + TOK - 1) / TOK;
   const int ksteps = K / (2 * kTcBK);
@@ -587,9 +589,8 @@ int launch_tc(void* y, const void* x, const void* wq, int M, int N, int K, const
     ub::set_cuda_error(e);
     return ub::fail(UB_ERR_CUDA);
   }
-  kernel<<<grid, kTcThreads, smem, s>>>(static_cast<__nv_bfloat16*>(y), M, N, K, ub::device_error_word(), map,
-                                        wmap, grp);
-  return ub::check_launch();
+  return ub::launch_pdl_smem(kernel, dim3(grid), dim3(kTcThreads), smem, s, static_cast<__nv_bfloat16*>(y), M, N, K,
+                             ub::device_error_word(), map, wmap, grp);
 }
 
 // xg[i, :] = hidden[sorted_ids[i] / top_k, :] for the positions the alignment produced (zeros for padding)
@@ -599,6 +600,8 @@ __global__ void __launch_bounds__(256) moe_gather_rows_kernel(__nv_bfloat16* __r
                                                               const int32_t* __restrict__ num_post_pad, int num_valid,
                                                               int top_k, int H) {
   const int i = blockIdx.x;
+  pdl_wait();
+  pdl_open();
   if (i >= *num_post_pad) return;
   const int sid = sorted_ids[i];
   const bool live = sid >= 0 && sid < num_valid;
@@ -651,10 +654,8 @@ bool q4k_moe_tc_supported(int positions, int K, int N, int block) {
 int moe_gather_rows(void* xg, const void* hidden, const int32_t* sorted_ids, const int32_t* num_post_pad, int positions,
                     int num_valid, int top_k, int H, cudaStream_t s) {
   if (positions <= 0) return UB_OK;
-  moe_gather_rows_kernel<<<positions, 256, 0, s>>>(static_cast<__nv_bfloat16*>(xg),
-                                                   static_cast<const __nv_bfloat16*>(hidden), sorted_ids, num_post_pad,
-                                                   num_valid, top_k, H);
-  return ub::check_launch();
+  return ub::launch_pdl(moe_gather_rows_kernel, dim3(positions), dim3(256), s, static_cast<__nv_bfloat16*>(xg),
+                        static_cast<const __nv_bfloat16*>(hidden), sorted_ids, num_post_pad, num_valid, top_k, H);
 }
 
 // Grouped expert GEMM over rows in aligned order (A[positions, K] bf16).
