@@ -5,6 +5,7 @@ import pytest
 
 from oracle import oracle as o
 from ubridge_b200 import DTYPE_BF16, DTYPE_F32, ops
+from ubridge_b200._lib import UbridgeError
 
 from _util import fetch, to_storage
 
@@ -68,3 +69,19 @@ def test_rms_norm_in_front(dev, N, K):
     want = o.c_qmatmul(o.rms_norm(x, g, 1e-5, o.UB_BF16), w, N, K, True)
     # bf16 activations after the norm (a boundary case may round the other way) and bf16 output
     assert o.rel_l2(fetch(dev, d_y, DTYPE_BF16, (1, N)), want) < 8e-3
+
+
+def test_what_needs_a_workspace_still_does(dev):
+    """Gate/up and RMSNorm forms of one token: without a workspace, and gate/up in f32, for K % 2048 == 0 only."""
+    I, K = 64, 1280
+    d_w = dev.htod_sync_copy(np.zeros(2 * I * K // 256 * 144, dtype=np.uint8))
+    d_x, d_y = dev.htod_sync_copy(np.zeros(K, dtype=np.uint16)), dev.alloc(I * 4)
+    with pytest.raises(UbridgeError):
+        ops.qmatmul_q4k_gate_up(d_y, d_x, d_w, 1, I, K, out_dtype=DTYPE_BF16, stream=dev.stream)
+    with pytest.raises(UbridgeError):
+        ops.qmatmul_q4k_rmsnorm(d_y, d_x, d_x, 1e-5, d_w, 1, I, K, gate_up=False, out_dtype=DTYPE_BF16, workspace=None,
+                                ws_bytes=0, stream=dev.stream)
+    ws_bytes = ops.qmatmul_q4k_gate_up_workspace_bytes(1, I, K)
+    with pytest.raises(UbridgeError):
+        ops.qmatmul_q4k_gate_up(d_y, d_x, d_w, 1, I, K, out_dtype=DTYPE_F32, workspace=dev.alloc(ws_bytes),
+                                ws_bytes=ws_bytes, stream=dev.stream)

@@ -2,14 +2,16 @@
 //
 // The reference picks a matmul variant per shape with AtenGemmTuner (src/gemm_tuner.rs:326-359,
 // small-M special cases :502-514) and kernels/matmul.cpp:1197-1208 (LHS-resident decode kernel when it
-// fits, batched kernel otherwise).  The same idea here is a three-way split on M:
-//   M <= 16           bandwidth-bound decode GEMV (qgemv.cu), f32 or bf16 activations, no workspace;
-//                     from M = 9 on, Q4_K with bf16 activations AND bf16 output takes the tensor-core kernel
-//                     instead (one pass of it is faster than two passes of eight tokens; no workspace either);
-//   M  > 16, Q4_K     tcgen05 tensor-core GEMM with in-kernel dequantisation (bf16 activations and output;
-//                     other types are converted through the caller's workspace);
-//   M  > 16, Q8_0     the same tensor-core kernel with a Q8_0 producer (K % 256 == 0, 16-byte aligned weights,
-//                     workspace as for Q4_K when the types are not bf16); otherwise the decode kernel in passes.
+// fits, batched kernel otherwise).  The same idea here is a split on M:
+//   M = 1             one-token decode kernels (qgemv_m1.cu, qgemv_q8_m1.cu), any whole super-blocks per row;
+//   M <= 16           integer decode kernels in passes of up to eight tokens (qgemv.cu), or the tensor-core kernel with
+//                     two-piece weights in one pass (qgemm_tc2.cu; the line: two_piece_is_faster); from M = 9 on Q4_K with
+//                     bf16 activations AND bf16 output takes the one-piece tensor-core kernels.  No workspace;
+//   M  > 16, Q4_K     tcgen05 tensor-core GEMM with in-kernel dequantisation, one piece (qgemm_tc2.cu while one round of CTAs
+//                     holds all 128-token tiles, qgemm_tc.cu beyond; bf16 activations and output, other types are
+//                     converted through the caller's workspace);
+//   M  > 16, Q8_0     the same kernels with a Q8_0 producer (K % 256 == 0, 16-byte aligned weights, workspace as for Q4_K
+//                     when the types are not bf16); otherwise the decode kernel in passes.
 #include <string.h>
 
 #include <mutex>
@@ -325,12 +327,14 @@ int ub_qmatmul_q4k_gate_up_bf16(void* y, const void* x, const void* wq, int M, i
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(wq) & 15)) return ub::fail(UB_ERR_INVALID_ARG);
   cudaStream_t s = ub::as_stream(stream);
   if (ub::take_weights_written(s)) fresh = true;
-  if (M == 1) {
+  const size_t need = ub_qmatmul_q4k_gate_up_workspace_bytes(M, I, K);
+  const bool ws_ok = workspace && ws_bytes >= need && !(reinterpret_cast<uintptr_t>(workspace) & 255);
+  // without a workspace, and in f32, the one-launch form is promised for K % 2048 == 0 only
+  if (M == 1 && (K % 2048 == 0 || (ws_ok && out_dtype != UB_DTYPE_F32))) {
     const int st = ub::q4k_gemv_m1_gate_up<__nv_bfloat16>(wq, static_cast<const __nv_bfloat16*>(x), y, I, K, out_dtype,
                                                          fresh, nullptr, 0.f, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
-  const size_t need = ub_qmatmul_q4k_gate_up_workspace_bytes(M, I, K);
   if (!workspace || ws_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)) return ub::fail(UB_ERR_WORKSPACE);
   char* ws = static_cast<char*>(workspace);
   const size_t gu_bytes = align_up(static_cast<size_t>(M) * 2 * I * 2, 256);
@@ -383,7 +387,9 @@ int ub_qmatmul_q4k_rmsnorm_bf16(void* y, const void* x, const void* gamma, float
       (reinterpret_cast<uintptr_t>(wq) & 15))
     return ub::fail(UB_ERR_INVALID_ARG);
   cudaStream_t s = ub::as_stream(stream);
-  if (M == 1) {
+  const size_t need = ub_qmatmul_q4k_rmsnorm_workspace_bytes(M, N, K, gate_up);
+  const bool ws_ok = workspace && ws_bytes >= need && !(reinterpret_cast<uintptr_t>(workspace) & 255);
+  if (M == 1 && (K % 2048 == 0 || (ws_ok && !(gate_up && out_dtype == UB_DTYPE_F32)))) {
     const bool fresh = ub::take_weights_written(s);
     int st;
     if (gate_up) {
@@ -395,7 +401,6 @@ int ub_qmatmul_q4k_rmsnorm_bf16(void* y, const void* x, const void* gamma, float
     }
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
-  const size_t need = ub_qmatmul_q4k_rmsnorm_workspace_bytes(M, N, K, gate_up);
   if (!workspace || ws_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)) return ub::fail(UB_ERR_WORKSPACE);
   char* ws = static_cast<char*>(workspace);
   const size_t xn_bytes = align_up(static_cast<size_t>(M) * K * 2, 256);
