@@ -11,8 +11,10 @@
 //         Q4_K, qh[32] fifth bits, qs[128] low nibbles; for 64-value group g: values 0..31 take the low nibbles
 //         of qs[32g..], bit 2g of qh[l] and pair 2g, values 32..63 the high nibbles, bit 2g+1 and pair 2g+1;
 //         y = d * sc * q - dmin * m)
-// with the published GGML arithmetic.  Their matmul is a plain bandwidth kernel (a warp per weight row,
-// activations staged in shared memory as f32, f32 FMA, fixed reduction order), for up to eight tokens per pass.
+// with the published GGML arithmetic.  Their matmul: up to four tokens with rows of whole 2048 values on the staged kernels
+// (qgemv_q5k.cu, qgemv_q4_0.cu), more tokens and other rows on the tensor-core kernel with two-piece weights
+// (qgemm_tc2.cu); what neither takes on a plain bandwidth kernel (a warp per weight row, activations staged in shared
+// memory as f32, f32 FMA, fixed reduction order) here.
 #include <type_traits>
 
 #include "common.cuh"

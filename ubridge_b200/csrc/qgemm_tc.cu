@@ -19,11 +19,10 @@
 // What bounds it.  An MMA of 128 x 256 x 16 takes 128 cycles of the tensor pipe, a weight stage 1024.  A producer warp
 // needs about 830 for it: 500 for the arithmetic of 64 values per thread and 75 to 150 for each barrier it looks at and for
 // the stores to land, whatever they carry.  With stages of 64 values that chain was 700 cycles against 512 of MMAs: the
-// producers held the tensor pipe back.  Three changes took 2048 tokens at 14336x4096 from 190 to 181 us and 512 tokens at
-// 57344x8192 from 376 to 346 us: weight stages of 128 values; one thread per 64-value group (both nibble halves from the
-// same words) in code that is not unrolled over the groups of a super-block (instruction fetch); and the issuing thread
-// chosen by elect.sync.  Dense launches of few tiles run in
-// qgemm_tc2.cu (q4k_gemm_tc, q8_0_gemm_tc).
+// producers held the tensor pipe back.  Weight stages of 128 values, one thread per 64-value group (both nibble halves from
+// the same words), the issuing thread chosen by elect.sync and stores that land during the next stage's arithmetic took
+// 2048 tokens at 14336x4096 from 190 to 177 us and 512 tokens at 57344x8192 from 376 to 335 us (bursts).  Dense launches
+// of few tiles run in qgemm_tc2.cu (q4k_gemm_tc, q8_0_gemm_tc).
 //
 //   warp 0        allocates TMEM, then one elected lane issues tcgen05.mma and tcgen05.commit
 //   warps 1-4     epilogue: tcgen05.ld -> bf16 -> staging tile in shared memory (accumulator released
