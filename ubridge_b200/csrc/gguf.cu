@@ -193,8 +193,9 @@ int gguf_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int y
   // take.  Measured on B200, us, four tokens at a time / two-piece for any number up to 16: Q5_K 14336x4096 34.3 / 33, Q4_0
   // 29.4 / 33.4; one token 4096x5120 Q5_K 32.6 / 19, Q4_0 25 / 18.6.  f32 results: as for Q6_K.
   if (K % 2048 ? y_dtype != UB_DTYPE_F32 : M > 4 && (y_dtype != UB_DTYPE_F32 || K <= 4096)) {
+    // rows that the staged kernels do not take were never requested ahead of the dependency wait
     const int st = ub::gguf_gemm_tc2(FMT == 1 ? GGML_Q5_K : GGML_Q4_0, y, y_dtype, x, std::is_same<XT, float>::value, wq, M,
-                                     N, K, fresh, s);
+                                     N, K, fresh || K % 2048 != 0, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   for (int m0 = 0; m0 < M;) {

@@ -458,7 +458,9 @@ int q6k_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int ou
   // 45 / 37, 4096x5120 14.2 / 19.8 / 17.2.  Its error is below that of the staged kernel (15-bit activations) but above
   // that of the f32 one, so f32 results leave the latter only where the former had them.
   if (K % 2048 ? M > 2 && out_dtype != UB_DTYPE_F32 : M > 4 && (out_dtype != UB_DTYPE_F32 || K <= 4096)) {
-    const int st = ub::gguf_gemm_tc2(14, y, out_dtype, x, std::is_same<XT, float>::value, wq, M, N, K, fresh, s);
+    // rows that the staged kernel does not take were never requested ahead of the dependency wait
+    const int st = ub::gguf_gemm_tc2(14, y, out_dtype, x, std::is_same<XT, float>::value, wq, M, N, K,
+                                     fresh || K % 2048 != 0, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   for (int m0 = 0; m0 < M;) {  // passes of up to four tokens: the weights are read once per pass

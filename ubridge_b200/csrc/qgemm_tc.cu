@@ -625,7 +625,8 @@ int q4k_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, boo
   // tiles would leave SMs without one.  Measured on B200, us, 128- / 256-token tiles: 4096 rows of 4096 values with 130
   // tokens 15.9 / 22.4, 256 18.8 / 27.1, 512 22.8 / 28.8; 4096x14336 with 200 tokens 37 / 63; 6144x4096 with 384 23.2 / 28.8.
   const int tiles128 = (N + 127) / 128 * ((M + 127) / 128);
-  if (M <= 128 || tiles128 <= ub::num_sms()) return q4k_gemm_tc1(12, y, x, wq, M, N, K, fresh, s);
+  // (weights ahead of the dependency wait up to 64 tokens only: beyond, callers may have them written by the kernel in front)
+  if (M <= 128 || tiles128 <= ub::num_sms()) return q4k_gemm_tc1(12, y, x, wq, M, N, K, fresh || M > 64, s);
   const TcGroup none = {nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
   return launch_tc<256, 5, 0>(y, x, wq, M, N, K, none, N, s);
 }

@@ -78,12 +78,6 @@ __device__ __forceinline__ uint32_t tc_peer_addr(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void tc_peer_arrive(uint32_t peer_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer_bar) : "memory");
 }
-// four bytes into another CTA's shared memory, counted on a barrier of that CTA (no fence on this side)
-__device__ __forceinline__ void tc_peer_store_tx(uint32_t peer_addr, uint32_t v, uint32_t peer_bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(peer_addr), "r"(v),
-               "r"(peer_bar)
-               : "memory");
-}
 __device__ __forceinline__ void tc_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -112,15 +106,7 @@ __device__ __forceinline__ uint64_t make_sw128_desc(uint32_t smem_addr) {
   return d;
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// same, with the A operand read from tensor memory (128 lanes x 8 columns of packed bf16 pairs per K = 16)
+// tcgen05.mma with the A operand read from tensor memory (128 lanes x 8 columns of packed bf16 pairs per K = 16)
 __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
