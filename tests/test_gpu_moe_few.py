@@ -48,3 +48,27 @@ def test_few_tokens(dev, T, H, I, E, k, norm, mapped):
     assert dev.device_status() == 0
 
 
+@pytest.mark.parametrize("T,H,I,k,own", [(1, 512, 1024, 2, 0), (3, 768, 1280, 2, 0), (2, 512, 1024, 3, 2), (2, 2048, 2304, 2, 1)])
+def test_weights_of_other_ranks_are_not_read(dev, T, H, I, k, own):
+    """Every matrix but those of this rank (none, some) holds NaN scales: the others' slots add exact zeros."""
+    E = 4
+    rng = np.random.default_rng(T + H + I + own)
+    emap = np.full(E, -1, dtype=np.int32)
+    emap[1:1 + own] = np.arange(1, 1 + own)  # matrix 0 is nobody's
+    w13, w2 = o.gen_q4k_weight(rng, E * 2 * I, H), o.gen_q4k_weight(rng, E * H, I)
+    hidden, logits = o.gen_activation(rng, T, H, True), o.gen_activation(rng, T, E, True)
+    want = np.zeros((T, H), dtype=np.float32)
+    if own:
+        want, _ = o.moe_layer_exact(hidden, logits, o.c_dequant(w13, True).reshape(E, 2 * I, H),
+                                    o.c_dequant(w2, True).reshape(E, H, I), k, 64, True, expert_map=emap)
+    for w in (w13, w2):
+        b = w.reshape(E, -1, 144)
+        for e in range(E):
+            if e not in emap:
+                b[e, :, 0:4] = 0xFF  # d = dmin = NaN
+    got = _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, emap)
+    if own:
+        assert o.rel_l2(got, want) < 1e-2
+    else:
+        assert np.array_equal(got, want)
+    assert dev.device_status() == 0

@@ -546,8 +546,9 @@ __device__ __forceinline__ uint32_t stage_at(int r, int w) {
   return ODD ? static_cast<uint32_t>((w >> 1) * kOddBox + r * kOddRow + (w & 1) * UB_Q4K_BYTES)
              : static_cast<uint32_t>(r * (8 * UB_Q4K_BYTES) + w * UB_Q4K_BYTES);
 }
-// One token through the experts it is routed to (SEL).  The tensor holds E matrices of `rows` rows; slot j takes matrix
-// idx[j] (through `map`, when given: -1 = held by another rank, the slot contributes nothing).
+// One token through the experts it is routed to (SEL).  The tensor holds matrices of `rows` rows; slot j takes matrix
+// idx[j] (through `map`, when given: -1 = held by another rank).  Only the slots whose matrix is here are worked on: a rank's
+// tensor may end behind its own matrices, or hold none at all.
 struct ExpertSel {
   const int32_t* idx;           // [slots] expert of each slot
   const __nv_bfloat16* weight;  // [slots] routed weights
@@ -555,21 +556,33 @@ struct ExpertSel {
   int slots, rows, experts;
 };
 constexpr int kSelMax = 16;
-// Reads the slots' experts into shared memory (all threads of the CTA).
-__device__ __forceinline__ void sel_load(const ExpertSel& sel, int* mat, float* weight, int* err_word) {
-  if (static_cast<int>(threadIdx.x) < sel.slots) {
-    int e = sel.idx[threadIdx.x];
-    if (e < 0 || e >= sel.experts) {  // the router chose nothing (logits that are not numbers)
-      report_device_error(err_word, UB_ERR_BAD_INDEX);
-      e = -1;
-    } else if (sel.map) {
-      e = sel.map[e];
-      if (e >= sel.experts) e = -1;
+// Reads the slots into shared memory, those of this rank only, in order (all threads of the CTA); returns how many there are.
+__device__ __forceinline__ int sel_load(const ExpertSel& sel, int* mat, float* weight, int* count, int* err_word) {
+  const int lane = threadIdx.x;
+  if (lane < 32) {
+    int e = -1;
+    float wt = 0.f;
+    if (lane < sel.slots) {
+      e = sel.idx[lane];
+      if (weight) wt = __bfloat162float(sel.weight[lane]);  // (both loads in flight at once)
+      if (e < 0 || e >= sel.experts) {  // the router chose nothing (logits that are not numbers)
+        report_device_error(err_word, UB_ERR_BAD_INDEX);
+        e = -1;
+      } else if (sel.map) {
+        e = sel.map[e];
+        if (e >= sel.experts) e = -1;
+      }
     }
-    mat[threadIdx.x] = e < 0 ? 0 : e;
-    if (weight) weight[threadIdx.x] = e < 0 ? 0.f : __bfloat162float(sel.weight[threadIdx.x]);
+    const uint32_t own = __ballot_sync(0xFFFFFFFFu, e >= 0);
+    if (e >= 0) {
+      const int at = __popc(own & ((1u << lane) - 1u));
+      mat[at] = e;
+      if (weight) weight[at] = wt;
+    }
+    if (lane == 0) *count = __popc(own);
   }
   __syncthreads();
+  return __reduce_max_sync(0xFFFFFFFFu, *count);  // the same everywhere, and known to the compiler as such
 }
 // the copies of one stage: rows row0 .. row0 + 15 (GU: eight gate rows from row0, eight up rows from row1), stage c of
 // the rows; a stage behind the row's end only arrives
@@ -608,7 +621,8 @@ __device__ __forceinline__ void stage_copy(const CUtensorMap& w_map, uint32_t ds
 // halves of every MMA row pair meet in one thread of the epilogue.  Gate and up are rounded to the output type
 // before the activation, which gives the bits of the two-kernel sequence (matmul, then ub_silu_and_mul).
 // MULTI: K is consumed in `npass` passes (rows too long for all activation fragments to be resident at once).
-// SEL (with GU): N rows are the slots' gate rows one slot behind the other, act[slot][row].
+// SEL (with GU): the rows are the gate rows of the slots, of those of this rank (N: of all), one slot behind the other,
+// act[slot][row].
 template <typename XT, bool GU, bool MULTI, bool ODD, bool SEL>
 __global__ void __launch_bounds__(kThreadsM1, 2)
 qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int nsb, int npass, int y_dtype, int S,
@@ -616,7 +630,7 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
                          const ExpertSel sel, const __grid_constant__ CUtensorMap w_map) {
   constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;  // a row's piece: 1152 bytes = 9 lines
   const int nch = (nsb + 7) >> 3;
-  __shared__ int sel_mat[SEL ? kSelMax : 1];
+  __shared__ int sel_mat[SEL ? kSelMax : 1], sel_count;
   extern __shared__ __align__(128) unsigned char m1_smem_raw[];
   unsigned char* const sm =
       m1_smem_raw + ((1024u - (static_cast<uint32_t>(__cvta_generic_to_shared(m1_smem_raw)) & 1023u)) & 1023u);
@@ -629,12 +643,6 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   const uint32_t bars_s = static_cast<uint32_t>(__cvta_generic_to_shared(bars));
   unsigned char* const frag = sm + static_cast<size_t>(S) * kStageBytes;  // [nch * 8][kFragBytesPerSb]
   constexpr int kTileRows = GU ? 8 : 16;  // output rows per tile
-  const int total_tiles = (N + kTileRows - 1) / kTileRows;
-  const int my_tiles =
-      static_cast<int>(blockIdx.x) < total_tiles ? (total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  const int my_items = my_tiles * nch;
-  const int nbatches = (my_tiles + kBatchTiles - 1) / kBatchTiles;
-
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
@@ -643,7 +651,28 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
+  auto tiles_of = [&](int rows) {
+    const int total = (rows + kTileRows - 1) / kTileRows;
+    return static_cast<int>(blockIdx.x) < total ? static_cast<int>((total - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
+  };
+  int my_tiles = tiles_of(N);
+  auto here = [&](int c) { return !ODD || 8 * c + warp < nsb; };  // this warp has a super-block in stage c
+  Raw8<XT> raw[kMaxChunks];
+  auto load_x = [&](int c0, int cn) {
+#pragma unroll
+    for (int c = 0; c < kMaxChunks; c++)
+      if (c < cn && here(c0 + c)) raw[c].load(x + static_cast<size_t>(8 * (c0 + c) + warp) * 256 + 8 * lane);
+  };
+  if (SEL) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    load_x(0, nch);  // in flight while the slots are read: behind them it was 0.5 us of a launch
+    const int own = sel_load(sel, sel_mat, nullptr, &sel_count, err_word);
+    if (own != sel.slots) N = own * (sel.rows >> 1), my_tiles = tiles_of(N);
+  } else {
+    __syncthreads();
+  }
+  const int my_items = my_tiles * nch;
+  const int nbatches = (my_tiles + kBatchTiles - 1) / kBatchTiles;
 
   // K in passes of cpp stages (npass > 1: rows too long for all activation fragments to be resident at once; the
   // launcher then guarantees a single batch of tiles): items run pass by pass, inside a pass tile by tile.
@@ -671,8 +700,7 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   if (threadIdx.x == 0)
     for (int n = 0; n < n_early; n++) issue_item(n);
 
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (SEL) sel_load(sel, sel_mat, nullptr, err_word);
+  if (!SEL) asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t epoch = ar.world > 1 ? ar_epoch(ar) : 0;  // of the fused all-reduce, read after the wait
 
   // ---- activations of this warp's super-blocks of one pass (stages c0 .. c0 + cn - 1, super-block 8c + warp) ->
@@ -680,12 +708,8 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   // behind a warp-level barrier.
   // (Fetching the next pass's activations into shared memory with asynchronous copies while the current pass
   // computes was measured and is no faster: 37.0 against 35.7 us at 8192 x 28672; it costs a ring stage.)
-  auto here = [&](int c) { return !ODD || 8 * c + warp < nsb; };  // this warp has a super-block in stage c
   auto quantise = [&](int c0, int cn, bool first) {
-    Raw8<XT> raw[kMaxChunks];
-#pragma unroll
-    for (int c = 0; c < kMaxChunks; c++)
-      if (c < cn && here(c0 + c)) raw[c].load(x + static_cast<size_t>(8 * (c0 + c) + warp) * 256 + 8 * lane);
+    if (!SEL) load_x(c0, cn);
     Raw8<XT> graw[kMaxChunks];
     if (gamma)
 #pragma unroll
@@ -894,7 +918,8 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
 constexpr int kWideWarps = 16;
 constexpr int kWideMaxUnits = 7;  // stages per half: rows up to 28672 values
 
-// SEL: a row is the slots' rows one behind the other, each ncs stages long, x the slots' activations likewise; the routed
+// SEL: a row is the rows of this rank's slots one behind the other, each ncs stages long (behind them stages of no bytes, one
+// for each of the other slots'; with no slot here the result is zero), x their activations likewise; the routed
 // weight goes into the activations' block scales, so the sum over the slots is the row's sum.
 // PAD: some warps have no super-block in some stages (ODD, SEL, or an odd number of stages).
 template <typename XT, bool ODD, bool SEL, bool PAD>
@@ -903,14 +928,8 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
                          int* err_word, const ExpertSel sel, const __grid_constant__ CUtensorMap w_map) {
   constexpr int kStageBytes = 16 * 8 * UB_Q4K_BYTES;  // a row's piece: 1152 bytes = 9 lines
   const int ncs = (nsb + 7) >> 3;
-  const int nch = ((SEL ? sel.slots * ncs : ncs) + 1) & ~1;  // stages of a row, even: an odd row ends with one of no bytes
-  __shared__ int sel_mat[SEL ? kSelMax : 1];
+  __shared__ int sel_mat[SEL ? kSelMax : 1], sel_count;
   __shared__ float sel_w[SEL ? kSelMax : 1];
-  // stage c -> slot and the stage inside it
-  auto split = [&](int c, int& slot_j, int& cc) {
-    slot_j = SEL ? c / ncs : 0, cc = c - slot_j * ncs;
-    if (SEL && slot_j >= sel.slots) cc = ncs;  // the stage of no bytes
-  };
   extern __shared__ __align__(128) unsigned char m1_smem_raw[];
   unsigned char* const sm =
       m1_smem_raw + ((1024u - (static_cast<uint32_t>(__cvta_generic_to_shared(m1_smem_raw)) & 1023u)) & 1023u);
@@ -922,12 +941,6 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
   const uint32_t ring_s = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
   const uint32_t bars_s = static_cast<uint32_t>(__cvta_generic_to_shared(bars));
   unsigned char* const frag = sm + static_cast<size_t>(S) * kStageBytes;  // [nch * 8][kFragBytesPerSb]
-  const int total_tiles = (N + 15) / 16;
-  const int my_tiles =
-      static_cast<int>(blockIdx.x) < total_tiles ? (total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  const int my_items = my_tiles * nch;
-  const int nbatches = (my_tiles + kBatchTiles - 1) / kBatchTiles;
-
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
@@ -936,13 +949,26 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  const int nch = ((SEL ? sel.slots * ncs : ncs) + 1) & ~1;  // stages of a row, even: an odd row ends with one of no bytes
+  // stage c -> slot and the stage inside it
+  auto split = [&](int c, int& slot_j, int& cc) {
+    slot_j = SEL ? c / ncs : 0, cc = c - slot_j * ncs;
+    if (SEL && slot_j >= sel.slots) cc = ncs;  // the stage of no bytes
+  };
+  int own = 1;  // slots of this rank; the stages of the others behind them carry no bytes either
   __syncthreads();
+  const int total_tiles = (N + 15) / 16;
+  const int my_tiles =
+      static_cast<int>(blockIdx.x) < total_tiles ? (total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const int my_items = my_tiles * nch;
+  const int nbatches = (my_tiles + kBatchTiles - 1) / kBatchTiles;
 
   // item n of this CTA = (tile n / nch, stage n % nch) -> ring slot n % S
   auto issue_item = [&](int n) {
     const int tile = n / nch, c = n - tile * nch;
     int row0 = 16 * (static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x)), j, cc;
     split(c, j, cc);
+    if (SEL && j >= own) cc = ncs;
     if (SEL && cc < ncs) row0 += sel_mat[j] * sel.rows;
     stage_copy<ODD, false, PAD>(w_map, ring_s + (n % S) * kStageBytes, bars_s + 8 * (n % S), cc, nsb, row0, 0);
   };
@@ -951,9 +977,11 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
     for (int n = 0; n < n_early; n++) issue_item(n);
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (SEL) sel_load(sel, sel_mat, sel_w, err_word);
+  if (SEL) own = sel_load(sel, sel_mat, sel_w, &sel_count, err_word);
 
   // ---- activations of this warp's super-blocks (stages c = half, half + 2, ...; super-block 8c + w8) ----
+  // (SEL: of all slots, whatever lies behind this rank's: those fragments are not used, and leaving them out by what was
+  // read from memory costs a launch 1 us.)
   {
     Raw8<XT> raw[kWideMaxUnits];
 #pragma unroll
@@ -973,9 +1001,6 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       float v[8];
       raw[u].unpack(v);
       const float slot_w = SEL ? sel_w[j] : 1.f;
-      if (SEL && slot_w == 0.f)
-#pragma unroll
-        for (int e = 0; e < 8; e++) v[e] = 0.f;  // an expert of another rank: whatever its activations hold
       float amax = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
@@ -1060,7 +1085,7 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
         if (PAD) {
           int j, cc;
           split(c, j, cc);
-          if (8 * cc + w8 >= nsb) continue;
+          if (8 * cc + w8 >= nsb || (SEL && j >= own)) continue;
         }
         const unsigned char* f = frag + static_cast<size_t>(8 * c + w8) * kFragBytesPerSb;
         const uint4 f0 = reinterpret_cast<const uint4*>(f)[lane], f1 = reinterpret_cast<const uint4*>(f + 512)[lane];
