@@ -184,8 +184,8 @@ int ub_qmatmul_q6k_bf16(void* y, const void* x, const void* wq, int M, int N, in
  * by a kernel that is followed by an event / synchronisation / any non-kernel operation, or simply written
  * long ago (model weights).  If the kernel launched immediately before the matmul on the same stream is the
  * one that WRITES wq (a dequantise / upload / repack kernel of the caller), OR UB_QMATMUL_WEIGHTS_FRESH into
- * out_dtype: the launch then requests nothing ahead of its dependency wait.  ub_quantize_q8_0 and
- * ub_repack_to_interleaved set this for the next matmul on their stream by themselves.  x and y carry no
+ * out_dtype: the launch then requests nothing ahead of its dependency wait.  ub_quantize_q8_0,
+ * ub_repack_to_interleaved and ub_copy_rows set this for the next matmul on their stream by themselves.  x and y carry no
  * such condition. */
 #define UB_QMATMUL_WEIGHTS_FRESH 0x100
 size_t ub_qmatmul_workspace_bytes(int M, int N, int K, int is_q4k);
@@ -285,7 +285,8 @@ void topsaten_release_graph_workspace_pool(void* stream);
 /* ------------------------------------------------------------------ MoE: new fused entry points */
 /* out[t, :D] = silu(in[t, :D]) * in[t, D:2D]  (kernels/topsaten_ops_wrapper.cpp:375-391) */
 int ub_silu_and_mul(void* out, const void* in, int rows, int D, int dtype, void* stream);
-/* dst[height][width] = src[height][width] (bytes) at the given row pitches, device memory */
+/* dst[height][width] = src[height][width] (bytes) at the given row pitches, device memory of the stream's device.  It may
+ * write weights: a matmul behind it on the stream waits for them. */
 int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t height,
                  void* stream);
 /* out[t,:] = sum_j in[t,j,:]  (the reference's caller uses topsaten_sum, src/ffi.rs:841-849) */

@@ -4,7 +4,7 @@ import pytest
 
 from oracle import oracle as o
 from ubridge_b200 import DTYPE_BF16, DTYPE_F16, DTYPE_F32, ops
-from ubridge_b200._lib import check, lib
+from ubridge_b200._lib import UB_QMATMUL_WEIGHTS_FRESH, check, lib
 
 from _util import ESIZE, fetch, to_storage
 
@@ -50,3 +50,36 @@ def test_copy_rows(dev, rows, width, src_pitch, dst_pitch):
     check(lib().ub_copy_rows(d_d.ptr, dst_pitch, d_s.ptr, src_pitch, width, rows, dev.stream), "copy_rows")
     dst[:, :width] = src[:, :width]
     assert np.array_equal(dev.dtoh_sync_copy(d_d, np.uint8, (rows, dst_pitch)), dst)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (1, 4096, 5120), (3, 2048, 14336), (16, 4096, 2048)])
+@pytest.mark.parametrize("flag", [0, UB_QMATMUL_WEIGHTS_FRESH])
+@pytest.mark.parametrize("between", [False, True])
+def test_copied_weights_are_complete(dev, M, N, K, flag, between):
+    """Weight rows cut out of a wider matrix by ub_copy_rows, and the matmul that reads them behind it on the stream, directly
+    or behind another matmul, with nothing else in between: it must not request them ahead of the copy."""
+    rng = np.random.default_rng(M + N + K)
+    w = o.gen_q4k_weight(rng, N, K)
+    x = o.gen_activation(rng, M, K, True)
+    width = K // 256 * 144
+    wide = np.zeros((N, 3 * width), dtype=np.uint8)
+    wide[:, width:2 * width] = w.reshape(N, width)
+    d_wide, d_x, d_y = dev.htod_sync_copy(wide), dev.htod_sync_copy(to_storage(x, DTYPE_BF16)), dev.alloc(M * N * 4)
+    d_w = [dev.htod_sync_copy(w), dev.alloc(w.size)]
+    d_other = dev.htod_sync_copy(o.gen_q4k_weight(rng, 64, K))
+    d_other_y = dev.alloc(M * 64 * 4)
+
+    def matmul(y, w_, n, f=0):
+        ops.qmatmul(y, d_x, w_, M, n, K, is_q4k=True, x_dtype=DTYPE_BF16, out_dtype=DTYPE_F32 | f, stream=dev.stream)
+
+    matmul(d_y, d_w[0], N)
+    want = fetch(dev, d_y, DTYPE_F32, (M, N))
+    assert o.rel_l2(want, o.c_qmatmul(x, w, N, K, True)) < 1e-4
+    for rep in range(5):
+        d_w[1] = dev.alloc_zeros(w.size)  # stale bytes cannot pass
+        dev.synchronize()
+        check(lib().ub_copy_rows(d_w[1].ptr, width, d_wide.ptr + width, 3 * width, width, N, dev.stream), "copy_rows")
+        if between:
+            matmul(d_other_y, d_other, 64)
+        matmul(d_y, d_w[1], N, flag)
+        assert np.array_equal(fetch(dev, d_y, DTYPE_F32, (M, N)), want)

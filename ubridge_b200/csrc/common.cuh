@@ -24,11 +24,12 @@ void set_cuda_error(cudaError_t e);
 int fail(int st);                 // records and returns st
 int check_launch();               // cudaGetLastError -> UB_OK / UB_ERR_CUDA (recorded)
 
-// ---- weight bytes produced on a stream by this library's own kernels (quantise, repack) ----
-// mark: called by those entry points; take: true once for the next quantized matmul on that stream, which then
-// requests no weight tile ahead of its dependency wait.
-void mark_weights_written(cudaStream_t s);
-bool take_weights_written(cudaStream_t s);
+// ---- weight bytes produced on a stream by this library's own kernels (quantise, repack, copy) ----
+// mark: called by those entry points, with the bytes that they write where other uses are common (a copy of activations);
+// take: called by the next quantized matmul on that stream, clears the mark and tells whether the matmul's weights may be
+// among those bytes: it then requests no weight tile ahead of its dependency wait.
+void mark_weights_written(cudaStream_t s, const void* dst = nullptr, size_t bytes = SIZE_MAX);
+bool take_weights_written(cudaStream_t s, const void* weights, size_t bytes);
 
 // ---- per-device error word written by kernels instead of trapping ----
 // Address of the device's error word (resolved once per device with cudaGetSymbolAddress).

@@ -333,7 +333,7 @@ int ub_qmatmul_gguf(void* y, const void* x, const void* blob, int ggml_type, int
     return ub::fail(UB_ERR_INVALID_ARG);
   if (reinterpret_cast<uintptr_t>(blob) & (ggml_type == GGML_Q5_K ? 15 : 1)) return ub::fail(UB_ERR_INVALID_ARG);
   cudaStream_t s = ub::as_stream(stream);
-  if (ub::take_weights_written(s)) fresh = true;
+  if (ub::take_weights_written(s, blob, ub_gguf_tensor_bytes(ggml_type, static_cast<size_t>(N) * K))) fresh = true;
   if (ggml_type == GGML_Q4_0)
     return f32 ? gguf_matmul<float, 0>(y, static_cast<const float*>(x), blob, M, N, K, out_dtype, fresh, s)
                : gguf_matmul<__nv_bfloat16, 0>(y, static_cast<const __nv_bfloat16*>(x), blob, M, N, K, out_dtype, fresh, s);

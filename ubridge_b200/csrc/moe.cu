@@ -593,13 +593,13 @@ __global__ void __launch_bounds__(256) topk_sum_kernel(T* __restrict__ out, cons
   }
 }
 
-// dst[r][c] = src[r][c] in 16-byte pieces, pitches in pieces; overlapped with its neighbours on the stream
+// dst[r][c] = src[r][c] in 16-byte pieces, pitches in pieces.  It starts under the kernel in front of it, but lets no kernel
+// start under itself: what it writes may be weights, which a matmul two launches on requests while the one in between runs.
 __global__ void __launch_bounds__(256) copy_rows_kernel(uint4* __restrict__ dst, size_t dst_pitch,
                                                         const uint4* __restrict__ src, size_t src_pitch, unsigned nv,
                                                         unsigned rows) {
   const unsigned c = blockIdx.x * 256 + threadIdx.x;
   pdl_wait();
-  pdl_open();
   if (c >= nv) return;
   for (unsigned r = blockIdx.y; r < rows; r += gridDim.y) dst[r * dst_pitch + c] = src[r * src_pitch + c];
 }
@@ -741,8 +741,8 @@ int ub_silu_and_mul(void* out, const void* in, int rows, int D, int dtype, void*
   return ub::check_launch();
 }
 
-// dst[height][width] = src[height][width] bytes at the given row pitches, both in memory of the current device.  Rows of
-// whole 16-byte pieces go through a kernel that overlaps with its neighbours on the stream, others through the runtime.
+// dst[height][width] = src[height][width] bytes at the given row pitches, on the device of `stream`.  Rows of whole 16-byte
+// pieces go through a kernel that starts under the one in front of it, others through the runtime.
 int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t height,
                  void* stream) {
   if (width == 0 || height == 0) return ub::fail(UB_OK);
@@ -750,9 +750,21 @@ int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch,
   const size_t bits = reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | dst_pitch | src_pitch | width;
   if (!(bits & 15) && width < (1u << 30) && height < (1u << 30)) {
     const unsigned nv = static_cast<unsigned>(width >> 4), rows = static_cast<unsigned>(height);
-    return ub::launch_pdl(copy_rows_kernel, dim3((nv + 255) / 256, rows < 32768 ? rows : 32768), dim3(256),
-                          ub::as_stream(stream), static_cast<uint4*>(dst), dst_pitch >> 4, static_cast<const uint4*>(src),
-                          src_pitch >> 4, nv, rows);
+    // a kernel is launched on the current device, a copy of the runtime on its stream's
+    int current = 0, own = 0;
+    cudaError_t e = cudaGetDevice(&current);
+    if (e == cudaSuccess) e = stream ? cudaStreamGetDevice(ub::as_stream(stream), &own) : (own = current, cudaSuccess);
+    if (e == cudaSuccess && own != current) e = cudaSetDevice(own);
+    if (e != cudaSuccess) {
+      ub::set_cuda_error(e);
+      return ub::fail(UB_ERR_CUDA);
+    }
+    const int st = ub::launch_pdl(copy_rows_kernel, dim3((nv + 255) / 256, rows < 32768 ? rows : 32768), dim3(256),
+                                  ub::as_stream(stream), static_cast<uint4*>(dst), dst_pitch >> 4,
+                                  static_cast<const uint4*>(src), src_pitch >> 4, nv, rows);
+    if (own != current) cudaSetDevice(current);
+    if (st == UB_OK) ub::mark_weights_written(ub::as_stream(stream), dst, (height - 1) * dst_pitch + width);
+    return st;
   }
   const cudaError_t e = cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, height, cudaMemcpyDeviceToDevice,
                                           ub::as_stream(stream));

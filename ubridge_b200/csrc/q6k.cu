@@ -452,7 +452,7 @@ int q6k_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int ou
   const int esz = out_dtype == UB_DTYPE_F32 ? 4 : 2;
   const int grid = (N + 8 * kQ6kRowsPerWarp - 1) / (8 * kQ6kRowsPerWarp);  // the CTA scheduler evens out the load
   const uint8_t* w = static_cast<const uint8_t*>(wq);
-  if (ub::take_weights_written(s)) fresh = true;
+  if (ub::take_weights_written(s, wq, static_cast<size_t>(N) * (K / UB_QK_K) * UB_Q6K_BYTES)) fresh = true;
   // The tensor-core kernel with two-piece weights from the second pass on; rows that the staged kernel does not take from
   // three tokens on.  Measured on B200, us, one token at a time / four / two-piece for any number up to 16: 4096x14336 17.5 /
   // 45 / 37, 4096x5120 14.2 / 19.8 / 17.2.  Its error is below that of the staged kernel (15-bit activations) but above

@@ -167,6 +167,11 @@ bool two_piece_is_faster(bool is_q4k, int M, int K, int out_dtype) {
   return !made_for && !(M <= 4 && pairs_fit);
 }
 
+inline size_t weight_bytes(bool is_q4k, int N, int K) {
+  return is_q4k ? static_cast<size_t>(N) * (K / UB_QK_K) * UB_Q4K_BYTES
+                : static_cast<size_t>(N) * (K / UB_QK8_0) * UB_Q8_0_BYTES;
+}
+
 inline int conv_grid(size_t n) {
   size_t b = (n + 255) / 256;
   const size_t cap = static_cast<size_t>(ub::num_sms()) * 8;
@@ -190,7 +195,7 @@ int qmatmul(bool is_q4k, int x_dtype, void* y, const void* x, const void* wq, in
       (x_dtype == UB_DTYPE_F32 && (K % 4)))
     return ub::fail(UB_ERR_INVALID_ARG);
   cudaStream_t s = ub::as_stream(stream);
-  if (ub::take_weights_written(s)) fresh = true;
+  if (ub::take_weights_written(s, wq, weight_bytes(is_q4k, N, K))) fresh = true;
 
   if (is_q4k && M > kDecodeOnePassM && M <= kDecodeMaxM && x_dtype == UB_DTYPE_BF16 && out_dtype == UB_DTYPE_BF16) {
     const int st = ub::q4k_gemm_tc(y, x, wq, M, N, K, fresh, s);
@@ -326,7 +331,7 @@ int ub_qmatmul_q4k_gate_up_bf16(void* y, const void* x, const void* wq, int M, i
     return ub::fail(UB_ERR_INVALID_ARG);
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(wq) & 15)) return ub::fail(UB_ERR_INVALID_ARG);
   cudaStream_t s = ub::as_stream(stream);
-  if (ub::take_weights_written(s)) fresh = true;
+  if (ub::take_weights_written(s, wq, weight_bytes(true, 2 * I, K))) fresh = true;
   const size_t need = ub_qmatmul_q4k_gate_up_workspace_bytes(M, I, K);
   const bool ws_ok = workspace && ws_bytes >= need && !(reinterpret_cast<uintptr_t>(workspace) & 255);
   // without a workspace, and in f32, the one-launch form is promised for K % 2048 == 0 only
@@ -390,7 +395,7 @@ int ub_qmatmul_q4k_rmsnorm_bf16(void* y, const void* x, const void* gamma, float
   const size_t need = ub_qmatmul_q4k_rmsnorm_workspace_bytes(M, N, K, gate_up);
   const bool ws_ok = workspace && ws_bytes >= need && !(reinterpret_cast<uintptr_t>(workspace) & 255);
   if (M == 1 && (K % 2048 == 0 || (ws_ok && !(gate_up && out_dtype == UB_DTYPE_F32)))) {
-    const bool fresh = ub::take_weights_written(s);
+    const bool fresh = ub::take_weights_written(s, wq, weight_bytes(true, gate_up ? 2 * N : N, K));
     int st;
     if (gate_up) {
       st = ub::q4k_gemv_m1_gate_up<__nv_bfloat16>(wq, static_cast<const __nv_bfloat16*>(x), y, N, K, out_dtype, fresh,
@@ -444,8 +449,9 @@ int ub_qmatmul_q4k_allreduce_residual_bf16(void* y, const void* x, const void* w
       ar.residual = static_cast<const __nv_bfloat16*>(residual);
       const ub::M1Extras ex = {nullptr, 0.f, &ar};
       const int st = ub::q4k_gemv_m1x<__nv_bfloat16>(wq, static_cast<const __nv_bfloat16*>(x), y, N, K, UB_DTYPE_BF16,
-                                                     ub::take_weights_written(ub::as_stream(stream)), ex,
-                                                     ub::as_stream(stream));
+                                                     ub::take_weights_written(ub::as_stream(stream), wq,
+                                                                              weight_bytes(true, N, K)),
+                                                     ex, ub::as_stream(stream));
       if (st != UB_ERR_UNSUPPORTED) return st;
     }
     const int st = qmatmul(true, UB_DTYPE_BF16, y, x, wq, M, N, K, UB_DTYPE_BF16, nullptr, 0, stream);
@@ -469,7 +475,7 @@ int ub_qmatmul_q4k_allreduce_residual_bf16(void* y, const void* x, const void* w
     ar.rank = rank, ar.world = world, ar.max_bytes = max_bytes;
     ar.residual = static_cast<const __nv_bfloat16*>(residual);
     ar.spin_limit = ub::oneshot_spin_limit();
-    const bool fresh = ub::take_weights_written(s);
+    const bool fresh = ub::take_weights_written(s, wq, weight_bytes(true, N, K));
     const int st = ub::qgemv_ar<__nv_bfloat16>(true, y, static_cast<const __nv_bfloat16*>(x), wq, 1, N, K, UB_DTYPE_BF16,
                                                fresh, &ar, s);
     if (st != UB_ERR_UNSUPPORTED) return st;

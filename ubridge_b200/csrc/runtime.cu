@@ -21,12 +21,17 @@ struct ErrWordCache {
 };
 ErrWordCache g_err_cache;
 
-// Streams on which this library has just launched a kernel that writes GGUF weight bytes (quantise, repack).
+// Streams on which this library has just launched a kernel that writes GGUF weight bytes (quantise, repack, copy), and
+// between which addresses.
 // The decode kernels request weight tiles before their dependency wait, which is only safe while no kernel
 // in front of them on the stream produces those bytes; the next quantized matmul on a marked stream is
 // launched without that early request and clears the mark.
 std::mutex g_fresh_mu;
-std::vector<cudaStream_t> g_fresh_streams;
+struct FreshMark {
+  cudaStream_t stream;
+  uintptr_t lo, hi;
+};
+std::vector<FreshMark> g_fresh_streams;
 std::atomic<int> g_fresh_count{0};
 }  // namespace
 
@@ -47,21 +52,27 @@ int check_launch() {
   return UB_OK;
 }
 
-void mark_weights_written(cudaStream_t s) {
+void mark_weights_written(cudaStream_t s, const void* dst, size_t bytes) {
+  const uintptr_t lo = reinterpret_cast<uintptr_t>(dst), hi = bytes > UINTPTR_MAX - lo ? UINTPTR_MAX : lo + bytes;
   std::lock_guard<std::mutex> lk(g_fresh_mu);
-  for (cudaStream_t t : g_fresh_streams)
-    if (t == s) return;
-  g_fresh_streams.push_back(s);
+  for (FreshMark& m : g_fresh_streams)
+    if (m.stream == s) {
+      m.lo = lo < m.lo ? lo : m.lo, m.hi = hi > m.hi ? hi : m.hi;
+      return;
+    }
+  g_fresh_streams.push_back({s, lo, hi});
   g_fresh_count.store(static_cast<int>(g_fresh_streams.size()), std::memory_order_release);
 }
-bool take_weights_written(cudaStream_t s) {
+bool take_weights_written(cudaStream_t s, const void* weights, size_t bytes) {
   if (g_fresh_count.load(std::memory_order_acquire) == 0) return false;
+  const uintptr_t w = reinterpret_cast<uintptr_t>(weights);
   std::lock_guard<std::mutex> lk(g_fresh_mu);
   for (size_t i = 0; i < g_fresh_streams.size(); i++)
-    if (g_fresh_streams[i] == s) {
+    if (g_fresh_streams[i].stream == s) {
+      const FreshMark m = g_fresh_streams[i];
       g_fresh_streams.erase(g_fresh_streams.begin() + i);
       g_fresh_count.store(static_cast<int>(g_fresh_streams.size()), std::memory_order_release);
-      return true;
+      return w < m.hi && (m.lo <= w || m.lo - w < bytes);
     }
   return false;
 }
