@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as o
-from ubridge_b200 import DTYPE_BF16, ops
+from ubridge_b200 import DTYPE_BF16, DTYPE_F32, ops
 
 from _util import fetch, to_storage
 
@@ -72,3 +72,38 @@ def test_weights_of_other_ranks_are_not_read(dev, T, H, I, k, own):
     else:
         assert np.array_equal(got, want)
     assert dev.device_status() == 0
+
+
+@pytest.mark.parametrize("H,I", [(512, 1024), (2048, 4096), (768, 1280)])
+@pytest.mark.parametrize("what", ["nan", "inf", "gate overflows"])
+def test_what_is_not_finite_stays_so(dev, H, I, what):
+    """A NaN or an infinity in one token, or a gate whose SiLU is NaN (-inf): that token becomes NaN, as in the grouped
+    kernels, the others keep their bits."""
+    T, E, k = 3, 4, 2
+    rng = np.random.default_rng(H + I)
+    w13, w2 = o.gen_q4k_weight(rng, E * 2 * I, H), o.gen_q4k_weight(rng, E * H, I)
+    hidden, logits = o.gen_activation(rng, T, H, True), o.gen_activation(rng, T, E, True)
+    clean = _layer(dev, T, H, I, E, k, hidden, logits, w13, w2)
+    bad = hidden.copy()
+    if what == "gate overflows":
+        bad[1] = 3e38  # sums beyond the largest float, of either sign
+    else:
+        bad[1, H // 2 + 3] = np.nan if what == "nan" else np.inf
+    got = _layer(dev, T, H, I, E, k, bad, logits, w13, w2)
+    assert np.isfinite(clean).all()
+    assert np.isnan(got[1]).all()
+    assert np.array_equal(got[[0, 2]], clean[[0, 2]])
+
+
+@pytest.mark.parametrize("K", [2048, 4096, 768, 8192, 14336])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_one_token_that_is_not_finite(dev, K, bad):
+    """The one-token matmul itself: short rows, rows in several stages, the sixteen-warp kernel."""
+    N = 40
+    rng = np.random.default_rng(K)
+    x = o.gen_activation(rng, 1, K, True)
+    x[0, K - 5] = bad
+    d_y = dev.alloc(N * 4)
+    ops.qmatmul(d_y, dev.htod_sync_copy(to_storage(x, DTYPE_BF16)), dev.htod_sync_copy(o.gen_q4k_weight(rng, N, K)), 1, N, K,
+                is_q4k=True, x_dtype=DTYPE_BF16, out_dtype=DTYPE_F32, stream=dev.stream)
+    assert np.isnan(fetch(dev, d_y, DTYPE_F32, (1, N))).all()

@@ -76,6 +76,13 @@ struct Vec16 {
   __device__ __forceinline__ void set(int i, T v) { reinterpret_cast<T*>(&r)[i] = v; }
 };
 
+// the larger value, NaN when either is (fmaxf drops it)
+__device__ __forceinline__ float fmax_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int num_sms() {

@@ -55,6 +55,9 @@ constexpr int kMaxStagesM1 = 8;
 constexpr int kBatchTiles = 4;        // tiles whose row sums are added across warps at once
 constexpr uint32_t kSpinM1 = 400000;
 constexpr float kXQMaxM1 = 32258.f;   // 127 * 254
+// Scale of a block whose largest magnitude is amax (a NaN among its values comes through fmax_nan): NaN where a value is not
+// finite.  Such a value has no fixed-point form, its block's integers mean nothing, and the token becomes NaN.
+__device__ __forceinline__ float scale_of(float amax) { return amax * (1.f / kXQMaxM1) + (amax - amax); }
 constexpr size_t kRingBudget = 110 * 1024 + 512;  // two CTAs per SM: 2 x (ring + 1 KB slack + static + 1 KB reserved) <= 228 KB
 
 __device__ __forceinline__ void mb_init(uint32_t bar, uint32_t count) {
@@ -263,11 +266,11 @@ qgemv_q4k_m1_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, int y
     for (int k = 0; k < SBW; k++) {
       float amax = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[k][e]));
+      for (int e = 0; e < 8; e++) amax = fmax_nan(amax, fabsf(v[k][e]));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+      for (int o = 16; o > 0; o >>= 1) amax = fmax_nan(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
       const float inv = amax > 0.f ? kXQMaxM1 / amax : 0.f;
-      xs[k] = amax * (1.f / kXQMaxM1);
+      xs[k] = scale_of(amax);
       // Round through the mantissa of 1.5 * 2^23.  q = rint(v inv); hi = rint(v inv / 254) differs from
       // rint(q / 254) only where q / 254 is within 0.002 of a half, and there both choices leave |lo| <= 127.
       const float inv254 = inv * (1.f / 254.f);
@@ -743,9 +746,9 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       }
       float amax = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
+      for (int e = 0; e < 8; e++) amax = fmax_nan(amax, fabsf(v[e]));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+      for (int o = 16; o > 0; o >>= 1) amax = fmax_nan(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
       const float inv = amax > 0.f ? kXQMaxM1 / amax : 0.f;
       const float inv254 = inv * (1.f / 254.f);
       int hi[8], lo[8], sum = 0;
@@ -776,7 +779,7 @@ qgemv_q4k_m1_long_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       }
       const int s_lo = __shfl_sync(0xFFFFFFFFu, sum, 4 * t), s_hi = __shfl_sync(0xFFFFFFFFu, sum, 16 + 4 * t);
       if (g == 0) reinterpret_cast<int2*>(f + 1024)[t] = make_int2(s_lo, s_hi);
-      if (lane == 0) *reinterpret_cast<float*>(f + 1024 + 32) = amax * (1.f / kXQMaxM1);
+      if (lane == 0) *reinterpret_cast<float*>(f + 1024 + 32) = scale_of(amax);
     }
     __syncwarp();
   };
@@ -1003,9 +1006,9 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       const float slot_w = SEL ? sel_w[j] : 1.f;
       float amax = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
+      for (int e = 0; e < 8; e++) amax = fmax_nan(amax, fabsf(v[e]));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+      for (int o = 16; o > 0; o >>= 1) amax = fmax_nan(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
       const float inv = amax > 0.f ? kXQMaxM1 / amax : 0.f;
       const float inv254 = inv * (1.f / 254.f);
       int hi[8], lo[8], sum = 0;
@@ -1036,7 +1039,7 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
       }
       const int s_lo = __shfl_sync(0xFFFFFFFFu, sum, 4 * t), s_hi = __shfl_sync(0xFFFFFFFFu, sum, 16 + 4 * t);
       if (g == 0) reinterpret_cast<int2*>(f + 1024)[t] = make_int2(s_lo, s_hi);
-      if (lane == 0) *reinterpret_cast<float*>(f + 1024 + 32) = amax * (1.f / kXQMaxM1) * slot_w;
+      if (lane == 0) *reinterpret_cast<float*>(f + 1024 + 32) = scale_of(amax) * slot_w;
     }
     __syncwarp();
   }
