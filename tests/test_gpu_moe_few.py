@@ -4,6 +4,7 @@ import pytest
 
 from oracle import oracle as o
 from ubridge_b200 import DTYPE_BF16, DTYPE_F32, ops
+from ubridge_b200._lib import UB_ERR_BAD_INDEX
 
 from _util import fetch, to_storage
 
@@ -107,3 +108,19 @@ def test_one_token_that_is_not_finite(dev, K, bad):
     ops.qmatmul(d_y, dev.htod_sync_copy(to_storage(x, DTYPE_BF16)), dev.htod_sync_copy(o.gen_q4k_weight(rng, N, K)), 1, N, K,
                 is_q4k=True, x_dtype=DTYPE_BF16, out_dtype=DTYPE_F32, stream=dev.stream)
     assert np.isnan(fetch(dev, d_y, DTYPE_F32, (1, N))).all()
+
+
+@pytest.mark.parametrize("T", [1, 2, 40])
+@pytest.mark.parametrize("entry", [-2, 4])
+def test_a_map_out_of_range_is_reported(dev, T, entry):
+    """Few tokens and the grouped path alike, whether or not a token goes to that expert."""
+    H, I, E, k = 256, 256, 4, 1
+    rng = np.random.default_rng(T)
+    w13, w2 = o.gen_q4k_weight(rng, E * 2 * I, H), o.gen_q4k_weight(rng, E * H, I)
+    hidden, logits = o.gen_activation(rng, T, H, True), o.gen_activation(rng, T, E, True)
+    logits[:, 0] = 9  # every token to expert 0, the bad entry is expert 3's
+    emap = np.array([0, 1, 2, entry], dtype=np.int32)
+    _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, emap)
+    assert dev.device_status() == UB_ERR_BAD_INDEX
+    _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, np.array([0, 1, 2, -1], dtype=np.int32))
+    assert dev.device_status() == 0

@@ -573,9 +573,12 @@ __device__ __forceinline__ int sel_load(const ExpertSel& sel, int* mat, float* w
         e = -1;
       } else if (sel.map) {
         e = sel.map[e];
-        if (e >= sel.experts) e = -1;
+        if (e >= sel.experts) e = -1;  // reported below
       }
     }
+    if (sel.map && blockIdx.x == 0)  // the whole map, as the alignment of the grouped path checks it
+      for (int i = lane; i < sel.experts; i += 32)
+        if (sel.map[i] < -1 || sel.map[i] >= sel.experts) report_device_error(err_word, UB_ERR_BAD_INDEX);
     const uint32_t own = __ballot_sync(0xFFFFFFFFu, e >= 0);
     if (e >= 0) {
       const int at = __popc(own & ((1u << lane) - 1u));
