@@ -610,3 +610,32 @@ def test_matmul_with_residual_on_one_rank(dev, N, K):
                                                        None, 0, 1, 0, dev.stream), "residual matmul")
     got = fetch(dev, d_y, DTYPE_BF16, (1, N))
     assert o.rel_l2(got, want) < 5e-3
+
+
+@pytest.mark.parametrize("N,K", [(2048, 4096), (2048, 18944), (80000, 14336)])
+def test_repack_then_matmul_with_residual_back_to_back(dev, N, K):
+    """The same on the one-rank residual form: a shape that the one-token kernel with that epilogue does not take falls back
+    to the matmul, which must still know that its weights have just been written."""
+    import ctypes
+
+    from ubridge_b200._lib import check, lib
+
+    rng = np.random.default_rng(N + K)
+    rows = min(N, 2048)  # packed rows, repeated: the last rows are what is checked
+    w = np.tile(o.gen_q4k_weight(rng, rows, K).reshape(rows, -1), ((N + rows - 1) // rows, 1))[:N].reshape(-1)
+    x, res = o.gen_activation(rng, 1, K, True), o.gen_activation(rng, 1, N, True)
+    want = o.c_qmatmul(x, np.ascontiguousarray(w.reshape(N, -1)[:rows]), rows, K, True)
+    want = np.tile(want, (1, (N + rows - 1) // rows))[:, :N] + res
+    nblocks = N * K // 256
+    d_w = dev.htod_sync_copy(w)
+    d_split = dev.alloc(w.size)
+    ops.repack_to_split(d_split, d_w, nblocks, True, stream=dev.stream)
+    d_x, d_r, d_y = (dev.htod_sync_copy(to_storage(v, DTYPE_BF16)) for v in (x, res, res))
+    for rep in range(3):
+        d_w2 = dev.alloc_zeros(w.size)
+        dev.synchronize()
+        ops.repack_to_interleaved(d_w2, d_split, nblocks, True, stream=dev.stream)
+        check(lib().ub_qmatmul_q4k_allreduce_residual_bf16(
+            ctypes.c_void_p(d_y.ptr), ctypes.c_void_p(d_x.ptr), ctypes.c_void_p(d_w2.ptr), ctypes.c_void_p(d_r.ptr), 1, N, K,
+            None, 0, 1, 0, dev.stream), "residual")
+        assert o.rel_l2(fetch(dev, d_y, DTYPE_BF16, (1, N)), want) < 8e-3  # bf16, rounded twice behind the fallback

@@ -405,6 +405,7 @@ int ub_qmatmul_q4k_rmsnorm_bf16(void* y, const void* x, const void* gamma, float
       st = ub::q4k_gemv_m1x<__nv_bfloat16>(wq, static_cast<const __nv_bfloat16*>(x), y, N, K, out_dtype, fresh, ex, s);
     }
     if (st != UB_ERR_UNSUPPORTED) return st;
+    if (fresh) ub::mark_weights_written(s);  // still true of the matmul below
   }
   if (!workspace || ws_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)) return ub::fail(UB_ERR_WORKSPACE);
   char* ws = static_cast<char*>(workspace);
@@ -448,11 +449,12 @@ int ub_qmatmul_q4k_allreduce_residual_bf16(void* y, const void* x, const void* w
       memset(&ar, 0, sizeof(ar));
       ar.residual = static_cast<const __nv_bfloat16*>(residual);
       const ub::M1Extras ex = {nullptr, 0.f, &ar};
-      const int st = ub::q4k_gemv_m1x<__nv_bfloat16>(wq, static_cast<const __nv_bfloat16*>(x), y, N, K, UB_DTYPE_BF16,
-                                                     ub::take_weights_written(ub::as_stream(stream), wq,
-                                                                              weight_bytes(true, N, K)),
-                                                     ex, ub::as_stream(stream));
+      cudaStream_t s = ub::as_stream(stream);
+      const bool fresh = ub::take_weights_written(s, wq, weight_bytes(true, N, K));
+      const int st =
+          ub::q4k_gemv_m1x<__nv_bfloat16>(wq, static_cast<const __nv_bfloat16*>(x), y, N, K, UB_DTYPE_BF16, fresh, ex, s);
       if (st != UB_ERR_UNSUPPORTED) return st;
+      if (fresh) ub::mark_weights_written(s);  // still true of the matmul below
     }
     const int st = qmatmul(true, UB_DTYPE_BF16, y, x, wq, M, N, K, UB_DTYPE_BF16, nullptr, 0, stream);
     return st != UB_OK ? st : add_residual();
@@ -479,6 +481,7 @@ int ub_qmatmul_q4k_allreduce_residual_bf16(void* y, const void* x, const void* w
     const int st = ub::qgemv_ar<__nv_bfloat16>(true, y, static_cast<const __nv_bfloat16*>(x), wq, 1, N, K, UB_DTYPE_BF16,
                                                fresh, &ar, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
+    if (fresh) ub::mark_weights_written(s);  // still true of the matmul below
   }
   int st = qmatmul(true, UB_DTYPE_BF16, y, x, wq, M, N, K, UB_DTYPE_BF16, nullptr, 0, stream);
   if (st != UB_OK) return st;
