@@ -85,3 +85,19 @@ def test_what_needs_a_workspace_still_does(dev):
     with pytest.raises(UbridgeError):
         ops.qmatmul_q4k_gate_up(d_y, d_x, d_w, 1, I, K, out_dtype=DTYPE_F32, workspace=dev.alloc(ws_bytes),
                                 ws_bytes=ws_bytes, stream=dev.stream)
+
+
+@pytest.mark.parametrize("K,bound", [(18944, 1.4e-5), (27648, 1.4e-5), (33024, 5e-6)])
+def test_long_rows_keep_their_precision(dev, K, bound):
+    """One activation of 256 a hundred times the others.  Rounding these activations in f64 to 16 bits with a scale per 32 values
+    leaves 8.3e-6 and 7.4e-6 of the result, to 15 bits with a scale per 256 2.7e-5 and 2.1e-5; f32 throughout far less."""
+    N = 600
+    rng = np.random.default_rng(K)
+    w = o.gen_q4k_weight(rng, N, K)
+    x = rng.standard_normal((1, K)).astype(np.float32)
+    x[0, 7::256] = 100
+    d_y = dev.alloc(N * 4)
+    ops.qmatmul(d_y, dev.htod_sync_copy(x), dev.htod_sync_copy(w), 1, N, K, is_q4k=True, x_dtype=DTYPE_F32,
+                out_dtype=DTYPE_F32, stream=dev.stream)
+    assert o.rel_l2(fetch(dev, d_y, DTYPE_F32, (1, N)), x.astype(np.float64) @ o.c_dequant(w, True).reshape(N, K).T) < bound
+    assert dev.device_status() == 0

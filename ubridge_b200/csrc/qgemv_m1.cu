@@ -1295,7 +1295,8 @@ namespace ub {
 
 // y[N] = dequant(Wq) . x for one token; UB_ERR_UNSUPPORTED (without touching the thread's status) for shapes
 // these kernels do not take (beyond 12288 values: more rows than one batch of tiles per CTA, or
-// with the RMSNorm prologue; unaligned weights; no tensor-map encoder).
+// with the RMSNorm prologue; beyond 17920 values: rows that are not whole 2048 values; unaligned weights; no tensor-map
+// encoder).
 // fresh: the weight bytes may have been written by the kernel launched just before on the same stream.
 template <typename XT>
 int q4k_gemv_m1x(const void* wq, const XT* x, void* y, int N, int K, int y_dtype, bool fresh, const M1Extras& ex,
@@ -1306,6 +1307,10 @@ int q4k_gemv_m1x(const void* wq, const XT* x, void* y, int N, int K, int y_dtype
   memset(&none, 0, sizeof(none));
   const ArParams& a = ex.ar ? *ex.ar : none;
   const XT* gamma = static_cast<const XT*>(ex.gamma);
+  // Rows that are not whole 2048 values and too long for the one-CTA-per-SM kernel of this precision (qgemv_imma.cu) have
+  // kernels with more bits (16 with a scale per 32 values, f32 beyond 32768; here 15 with a scale per 256): f32 results
+  // 2.0e-5 against 2.6e-5 of the exact ones, with one outlier in 256 activations a third of the error.
+  if (K % 2048 && K > 17920) return UB_ERR_UNSUPPORTED;
   if (K == 4096) return launch_m1<XT, 2>(w, x, y, N, K, y_dtype, fresh, gamma, ex.eps, a, s);
   if (K == 2048) return launch_m1<XT, 1>(w, x, y, N, K, y_dtype, fresh, gamma, ex.eps, a, s);
   if (K >= 12288 && !gamma && a.world <= 1 && !a.residual) {
