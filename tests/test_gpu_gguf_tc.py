@@ -48,3 +48,29 @@ def test_two_piece_weights(dev, tag, x_dtype, M, N, K):
         for m in range(M):
             assert o.rel_l2(got[m], want[m]) < (tol if N >= 100 else max(tol, 4e-3)), (dt, m)
         assert np.array_equal(got, run(dt))  # the parts of a K split are added in a fixed order
+
+
+def test_half_the_rows_take_no_longer(dev):
+    """Every cluster of a K split is on the GPU at once: 2048 rows (sixteen tiles) in one round, as 4096 rows are."""
+    import torch
+
+    stream = torch.cuda.ExternalStream(int(getattr(dev.stream, "value", dev.stream)))
+    M, K = 8, 4096
+    us = {}
+    for N in (2048, 4096):
+        blob = dev.htod_sync_copy(o.gen_q6k_weight(np.random.default_rng(N), N, K).reshape(-1))
+        d_x, d_y = dev.htod_sync_copy(np.zeros((M, K), dtype=np.uint16)), dev.alloc(M * N * 2)
+        best = 1e9
+        for rep in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(500000)  # the calls below are queued before the first one runs
+                a.record(stream)
+            for _ in range(20):
+                ops.qmatmul_gguf(d_y, d_x, blob, o.GGML_Q6_K, M, N, K, x_dtype=DTYPE_BF16, out_dtype=DTYPE_BF16,
+                                 stream=dev.stream)
+            b.record(stream)
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 50)
+        us[N] = best
+    assert us[2048] < 1.1 * us[4096], us

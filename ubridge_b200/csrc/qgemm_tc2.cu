@@ -496,6 +496,18 @@ qgemm_tc2_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ xf
   }
 }
 
+// The widest K split whose clusters are all resident at once.  A cluster stays inside one group of SMs.  Reported by
+// cudaOccupancyMaxActiveClusters: with one CTA per SM 74 pairs, 33 clusters of four and 15 of eight, with two CTAs per SM
+// 148, 71 and 33.  Sixteen of eight took a second round: Q6_K, five tokens, 2048 rows of 4096 values 19.8 us, with clusters
+// of four 12.8.
+inline int k_split(int tiles, int nsb, int ctas) {
+  const int slots = ub::num_sms() * ctas, eights = ctas == 1 ? 15 : 16;
+  int ks = 1;
+  while (ks < 8 && nsb >= 4 * ks && tiles <= (ks == 1 ? slots / 2 : ks == 2 ? slots * 33 / 148 : slots * eights / 148))
+    ks *= 2;
+  return ks;
+}
+
 template <int FMT, int TOK, int STAGES, int WST, bool XF, int PIECES = 2, int CTAS = 1, int SETS = 2, int UNR = 1>
 int launch2(void* y, int y_dtype, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s) {
   constexpr size_t smem = smem_of(FMT, TOK, STAGES, WST, XF, PIECES);
@@ -505,10 +517,7 @@ int launch2(void* y, int y_dtype, const void* x, const void* wq, int M, int N, i
   // token tiles of equal size: 333 tokens are two tiles of 176, not 256 and 77
   const int t_tiles = (M + TOK - 1) / TOK, tile_tok = ((M + t_tiles - 1) / t_tiles + 15) / 16 * 16;
   const int tiles = ((N + 127) / 128) * t_tiles, slots = ub::num_sms() * CTAS, nsb = K / UB_QK_K;
-  // The widest K split whose clusters are all resident at once.  A cluster stays inside one group of SMs: of 148, 74 pairs,
-  // 33 clusters of four and 16 of eight fit.
-  int ks = 1;
-  while (ks < 8 && nsb >= 4 * ks && tiles <= (ks == 1 ? slots / 2 : ks == 2 ? slots * 33 / 148 : slots * 16 / 148)) ks *= 2;
+  const int ks = k_split(tiles, nsb, CTAS);
   const int grid = ks > 1 ? tiles * ks : (tiles < slots ? tiles : slots);
   CUtensorMap xmap, wmap;
   memset(&xmap, 0, sizeof(xmap));
