@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as o
-from ubridge_b200 import DTYPE_BF16, DTYPE_F32, ops
+from ubridge_b200 import DTYPE_BF16, DTYPE_F16, DTYPE_F32, ops
 
 from _util import ESIZE, fetch, to_storage
 
@@ -53,3 +53,35 @@ def test_one_piece_launches(dev, is_q4k, M, N, K):
     # weights and results rounded to bf16 (2^-9 each at most); a single row may be a small difference of large terms
     assert o.rel_l2(got, o.c_qmatmul(x, w, N, K, is_q4k)) < (1e-2 if N > 1 else 3e-2)
     assert np.array_equal(got, _run(dev, w, x, M, N, K, is_q4k, DTYPE_BF16, DTYPE_BF16))
+
+
+@pytest.mark.parametrize("x_dtype", [DTYPE_BF16, DTYPE_F32])
+@pytest.mark.parametrize("tag,M,N,K", [
+    (o.GGML_Q6_K, 4, 2048, 512), (o.GGML_Q6_K, 4, 1024, 2304), (o.GGML_Q5_K, 1, 2048, 1024), (o.GGML_Q5_K, 2, 1024, 1280),
+    (o.GGML_Q4_0, 1, 2048, 1280), (o.GGML_Q4_0, 4, 1024, 512), (8, 2, 2048, 512), (8, 4, 2048, 512),
+])
+def test_small_matrices_stay_with_the_decode_kernels(dev, x_dtype, tag, M, N, K):
+    """A pass of these takes half the time of a tensor-core launch.  Their f32 results are always the decode kernels', so the
+    f16 results of the same kernel are those rounded, bit for bit; two-piece weights differ in some of 4000."""
+    gen = {o.GGML_Q4_0: o.gen_q4_0_weight, o.GGML_Q5_K: o.gen_q5k_weight, o.GGML_Q6_K: o.gen_q6k_weight, 8: o.gen_q8_0_weight}
+    rng = np.random.default_rng(tag + M + N + K)
+    d_w = dev.htod_sync_copy(np.ascontiguousarray(gen[tag](rng, N, K)).reshape(-1))
+    d_x = dev.htod_sync_copy(to_storage(o.gen_activation(rng, M, K, x_dtype == DTYPE_BF16) * 0.01, x_dtype))
+    y = {}
+    for dt in (DTYPE_F32, DTYPE_F16):
+        d_y = dev.alloc(M * N * 4)
+        ops.qmatmul_gguf(d_y, d_x, d_w, tag, M, N, K, x_dtype=x_dtype, out_dtype=dt, stream=dev.stream)
+        y[dt] = fetch(dev, d_y, dt, (M, N))
+    assert np.array_equal(y[DTYPE_F16], y[DTYPE_F32].astype(np.float16).astype(np.float32))
+
+
+@pytest.mark.parametrize("is_q4k,M,N,K,x_dtype", [(True, 9, 6144, 4096, DTYPE_F32), (True, 10, 6144, 4096, DTYPE_BF16),
+                                                  (False, 9, 12288, 4096, DTYPE_BF16), (True, 9, 1024, 1792, DTYPE_F32)])
+def test_a_second_pass_where_it_is_the_faster_way(dev, is_q4k, M, N, K, x_dtype):
+    """Eight tokens and the rest through the decode kernels: the bits of two calls."""
+    rng = np.random.default_rng(M + N + K)
+    w = (o.gen_q4k_weight if is_q4k else o.gen_q8_0_weight)(rng, N, K)
+    x = o.gen_activation(rng, M, K, x_dtype == DTYPE_BF16)
+    got = _run(dev, w, x, M, N, K, is_q4k, x_dtype, DTYPE_F32)
+    assert np.array_equal(got[:8], _run(dev, w, x[:8], 8, N, K, is_q4k, x_dtype, DTYPE_F32))
+    assert np.array_equal(got[8:], _run(dev, w, x[8:], M - 8, N, K, is_q4k, x_dtype, DTYPE_F32))

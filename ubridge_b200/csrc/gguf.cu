@@ -32,6 +32,7 @@ template <typename XT>
 int q4_0_gemv_staged(const void* wq, const XT* x, void* y, int M, int N, int K, int y_dtype, bool fresh, cudaStream_t s);
 int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
                   bool fresh, cudaStream_t s);
+bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32);
 }
 
 namespace {
@@ -189,13 +190,15 @@ template <typename XT, int FMT>
 int gguf_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int y_dtype, bool fresh, cudaStream_t s) {
   const uint8_t* w = static_cast<const uint8_t*>(wq);
   const size_t esz = y_dtype == UB_DTYPE_F32 ? 4 : 2;
-  // The tensor-core kernel with two-piece weights from the second pass on, and always for rows that the staged kernels do not
-  // take.  Measured on B200, us, four tokens at a time / two-piece for any number up to 16: Q5_K 14336x4096 34.3 / 33, Q4_0
-  // 29.4 / 33.4; one token 4096x5120 Q5_K 32.6 / 19, Q4_0 25 / 18.6.  f32 results: as for Q6_K.
-  if (K % 2048 ? y_dtype != UB_DTYPE_F32 : M > 4 && (y_dtype != UB_DTYPE_F32 || K <= 4096)) {
+  // The tensor-core kernel with two-piece weights from the second pass on, and where it pays for rows that the staged kernels
+  // do not take.  Measured on B200, us, four tokens at a time / two-piece for any number up to 16: Q5_K 14336x4096 34.3 / 33,
+  // Q4_0 29.4 / 33.4; one token 4096x5120 Q5_K 32.6 / 19, Q4_0 25 / 18.6.  f32 results: as for Q6_K.
+  constexpr bool x_f32 = std::is_same<XT, float>::value;
+  if (K % 2048 ? y_dtype != UB_DTYPE_F32 && (M > 4 || ub::two_piece_pays(FMT == 1 ? GGML_Q5_K : GGML_Q4_0, M, N, K, x_f32))
+               : M > 4 && (y_dtype != UB_DTYPE_F32 || K <= 4096)) {
     // rows that the staged kernels do not take were never requested ahead of the dependency wait
-    const int st = ub::gguf_gemm_tc2(FMT == 1 ? GGML_Q5_K : GGML_Q4_0, y, y_dtype, x, std::is_same<XT, float>::value, wq, M,
-                                     N, K, fresh || K % 2048 != 0, s);
+    const int st = ub::gguf_gemm_tc2(FMT == 1 ? GGML_Q5_K : GGML_Q4_0, y, y_dtype, x, x_f32, wq, M, N, K,
+                                     fresh || K % 2048 != 0, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   for (int m0 = 0; m0 < M;) {

@@ -27,6 +27,7 @@
 namespace ub {
 int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
                   bool fresh, cudaStream_t s);
+bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32);
 }
 
 namespace {
@@ -454,13 +455,14 @@ int q6k_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int ou
   const uint8_t* w = static_cast<const uint8_t*>(wq);
   if (ub::take_weights_written(s, wq, static_cast<size_t>(N) * (K / UB_QK_K) * UB_Q6K_BYTES)) fresh = true;
   // The tensor-core kernel with two-piece weights from the second pass on; rows that the staged kernel does not take from
-  // three tokens on.  Measured on B200, us, one token at a time / four / two-piece for any number up to 16: 4096x14336 17.5 /
-  // 45 / 37, 4096x5120 14.2 / 19.8 / 17.2.  Its error is below that of the staged kernel (15-bit activations) but above
-  // that of the f32 one, so f32 results leave the latter only where the former had them.
-  if (K % 2048 ? M > 2 && out_dtype != UB_DTYPE_F32 : M > 4 && (out_dtype != UB_DTYPE_F32 || K <= 4096)) {
+  // three tokens on where it pays.  Measured on B200, us, one token at a time / four / two-piece for any number up to 16:
+  // 4096x14336 17.5 / 45 / 37, 4096x5120 14.2 / 19.8 / 17.2.  Its error is below that of the staged kernel (15-bit
+  // activations) but above that of the f32 one, so f32 results leave the latter only where the former had them.
+  constexpr bool x_f32 = std::is_same<XT, float>::value;
+  if (K % 2048 ? M > 2 && out_dtype != UB_DTYPE_F32 && (M > 4 || ub::two_piece_pays(14, M, N, K, x_f32))
+               : M > 4 && (out_dtype != UB_DTYPE_F32 || K <= 4096)) {
     // rows that the staged kernel does not take were never requested ahead of the dependency wait
-    const int st = ub::gguf_gemm_tc2(14, y, out_dtype, x, std::is_same<XT, float>::value, wq, M, N, K,
-                                     fresh || K % 2048 != 0, s);
+    const int st = ub::gguf_gemm_tc2(14, y, out_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   for (int m0 = 0; m0 < M;) {  // passes of up to four tokens: the weights are read once per pass

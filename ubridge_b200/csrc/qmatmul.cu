@@ -38,6 +38,7 @@ void* tensor_map_encoder();
 int q4k_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
 int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
                   bool fresh, cudaStream_t s);
+bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32);
 int q8_0_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
 }  // namespace ub
 
@@ -147,24 +148,25 @@ __global__ void add_bf16_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Two to sixteen tokens: the tensor-core kernel with two-piece weights (one pass for all of them) or the decode kernels
-// (passes of up to eight).  Where the decode kernels run in one pass on rows they are made for they are the faster ones; the
-// line is where they need a second pass or fall back to the CUDA-core kernels.  Measured on B200, us, decode / two-piece:
-// Q4_K four tokens 4096x4096 7.4 / 12, 27648x5120 33.6 / 75, 57344x8192 72 / 230, but 4096x14336 135 / 30.6 and eight tokens
-// 15360x5120 75 / 42; Q8_0 four tokens 6144x4096 9.2 / 20.5, sixteen 25.6 / 21, four 6144x5120 76 / 25.
-// The integer decode kernels keep 15 bits of an activation (2.8e-5 of the result), the two pieces 16 bits and more (3e-6), the
-// CUDA-core ones compute in f32 (1e-7): where those run, f32 results stay with them.
-bool two_piece_is_faster(bool is_q4k, int M, int K, int out_dtype) {
+// (passes of up to eight).  Where the decode kernels run in one pass on rows they are made for they are the faster ones:
+// measured on B200, us, decode / two-piece, Q4_K four tokens 4096x4096 7.4 / 12, 27648x5120 33.6 / 75, 57344x8192 72 / 230, but
+// 4096x14336 135 / 30.6 and eight tokens 15360x5120 75 / 42; Q8_0 four tokens 6144x4096 9.2 / 20.5, four 6144x5120 76 / 25.
+// Where they need a second pass or fall back to the CUDA-core kernels, both are priced (two_piece_pays).
+// Error of f32 results (2-norm, f64): integer kernels, 15 bits of an activation, 2.8e-5; two pieces 2e-6 to 5e-6 with bf16
+// activations, 4e-6 to 1.2e-5 with f32 ones; CUDA-core kernels 1e-7 to 3e-6 (Q4_K while a row's activations fit its
+// shared memory 2e-5): where those run, f32 results stay with them.
+bool two_piece_is_faster(bool is_q4k, int M, int N, int K, bool x_f32, int out_dtype) {
   const int pass = M < kDecodeOnePassM ? M : kDecodeOnePassM, nsb = K / UB_QK_K;
   if (!is_q4k) {
     const bool quads_fit = K % 2048 == 0 && (pass + 3) / 4 * (K / UB_QK8_0) <= 568;  // in qgemv_imma.cu's shared memory
-    if (quads_fit) return M > kDecodeOnePassM;
-    return out_dtype != UB_DTYPE_F32 && K % UB_QK_K == 0;
+    if (quads_fit ? M <= kDecodeOnePassM : out_dtype == UB_DTYPE_F32 || K % UB_QK_K != 0) return false;
+  } else {
+    const bool made_for = K == 2048 || K == 4096 || (K == 8192 && M > 4);  // qgemv_mt.cu, qgemv_mc.cu
+    const bool pairs_fit = (pass + 1) / 2 * nsb <= 70;  // token pairs of a whole row in qgemv_imma.cu's shared memory
+    if (out_dtype == UB_DTYPE_F32 && !made_for && !pairs_fit) return false;
+    if (M <= kDecodeOnePassM && (made_for || (M <= 4 && pairs_fit))) return false;
   }
-  const bool made_for = K == 2048 || K == 4096 || (K == 8192 && M > 4);  // qgemv_mt.cu, qgemv_mc.cu
-  const bool pairs_fit = (pass + 1) / 2 * nsb <= 70;  // token pairs of a whole row in qgemv_imma.cu's shared memory
-  if (out_dtype == UB_DTYPE_F32 && !made_for && !pairs_fit) return false;
-  if (M > kDecodeOnePassM) return true;
-  return !made_for && !(M <= 4 && pairs_fit);
+  return ub::two_piece_pays(is_q4k ? 12 : 8, M, N, K, x_f32);
 }
 
 inline size_t weight_bytes(bool is_q4k, int N, int K) {
@@ -201,7 +203,7 @@ int qmatmul(bool is_q4k, int x_dtype, void* y, const void* x, const void* wq, in
     const int st = ub::q4k_gemm_tc(y, x, wq, M, N, K, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;  // unsupported shape or driver: the decode kernel below
   }
-  if (M >= 2 && M <= kDecodeMaxM && two_piece_is_faster(is_q4k, M, K, out_dtype)) {
+  if (M >= 2 && M <= kDecodeMaxM && two_piece_is_faster(is_q4k, M, N, K, x_dtype == UB_DTYPE_F32, out_dtype)) {
     const int st = ub::gguf_gemm_tc2(is_q4k ? 12 : 8, y, out_dtype, x, x_dtype == UB_DTYPE_F32, wq, M, N, K, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
