@@ -124,3 +124,23 @@ def test_a_map_out_of_range_is_reported(dev, T, entry):
     assert dev.device_status() == UB_ERR_BAD_INDEX
     _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, np.array([0, 1, 2, -1], dtype=np.int32))
     assert dev.device_status() == 0
+
+
+@pytest.mark.parametrize("T,H,I,mapped,grouped", [(6, 1024, 1024, True, True), (6, 1024, 1024, False, True),
+                                                 (2, 1024, 1024, True, False), (3, 1024, 1024, False, False)])
+def test_which_way_a_few_tokens_go(dev, T, H, I, mapped, grouped):
+    """The grouped kernels give a token the same bits whoever comes with it; one at a time the weights are not rounded.  With
+    eight experts on eight ranks (or a small layer) six tokens are faster grouped."""
+    E, k, many = 8, 2, 40
+    rng = np.random.default_rng(T + mapped)
+    emap = None
+    if mapped:
+        emap = np.full(E, -1, dtype=np.int32)
+        emap[3] = 0
+    w13, w2 = o.gen_q4k_weight(rng, E * 2 * I, H), o.gen_q4k_weight(rng, E * H, I)
+    hidden, logits = o.gen_activation(rng, many, H, True), o.gen_activation(rng, many, E, True)
+    logits[0, 3] = 9  # at least one token has work here
+    all_ = _layer(dev, many, H, I, E, k, hidden, logits, w13, w2, emap)
+    got = _layer(dev, T, H, I, E, k, hidden[:T], logits[:T], w13, w2, emap)
+    assert np.array_equal(got, all_[:T]) == grouped
+    assert o.rel_l2(got, all_[:T]) < 2e-2

@@ -14,6 +14,7 @@
 // of sub-block 2G+1, which feeds four mma steps.  Activations are read with the same k assignment, so
 // the reduction order inside a group is permuted but complete.  Weights are dequantised exactly in
 // f32 ((d*sc)*q - dmin*m) and rounded once to bf16 for the tensor core.
+#include <math.h>
 #include "common.cuh"
 
 namespace {
@@ -260,6 +261,30 @@ int q4k_moe_gemm_tc(void* C, const void* A, const void* Bq, const float* topk_w,
                     int num_valid, int block, int act_silu_mul, cudaStream_t s);
 }  // namespace ub
 
+namespace {
+
+// Expert layer, few tokens: a token at a time through the one-token kernels, each slot's expert read at streaming speed, or
+// the grouped kernels, which cost a chain of steps as long as the rows and then the experts touched.  In us, fitted to 250
+// timings on B200 (512 to 4096 / 1024 to 14336, 4 to 64 experts, one to ten tokens, within 15 %); a matrix here is an
+// expert's gate, up and down rows in MB.  One at a time / grouped, 8 experts top-2: 4096 / 14336 one token 55 / 181, six
+// 302 / 323, eight 400 / 326; 1024 / 1024 three tokens 28 / 36, four 36 / 36, six 51 / 37.
+// mapped: a rank that holds some of the experts, the host does not know how many.  Both ways cost less the fewer it holds;
+// one at a time is taken where it is the cheaper way with one of them as well as with all.  8 ranks of one expert each, us:
+// 4096 / 14336 four tokens 103 / 115, six 147 / 138; 1024 / 1024 four tokens 32 / 34, six 46 / 37.
+bool few_token_moe_pays(int T, int H, int I, int E, int top_k, bool mapped) {
+  if (top_k > E) return false;
+  const float mb = 3.f * H * I * (UB_Q4K_BYTES / 256.f) * 1e-6f;
+  const float touched = E * (1.f - powf(1.f - static_cast<float>(top_k) / E, static_cast<float>(T)));
+  auto cheaper = [&](float own) {  // own: share of the experts that this rank holds
+    const float one = 5.8f + T * (6.4f + own * top_k * (.45f + .243f * mb));
+    const float grouped = 22.4f + 1.25f * ((H + I) / 256) + own * touched * (.41f + .31f * mb);
+    return one <= grouped;
+  };
+  return cheaper(1.f) && (!mapped || cheaper(1.f / E));
+}
+
+}  // namespace
+
 extern "C" {
 
 int ub_fused_moe_q4k_gemm(void* C, const void* A, const void* Bq, const float* topk_weights, const int32_t* sorted_ids,
@@ -346,13 +371,9 @@ int ub_moe_layer_q4k(void* out, const void* hidden, const void* router_logits, c
 
   int st = ub::topk_softmax_bf16_impl(router_logits, w_t, idx, T, E, top_k, norm_topk_prob != 0, s);
   if (st != UB_OK) return st;
-  // Few tokens: a token at a time through the one-token kernels, each slot's expert read at streaming speed, against a
-  // fixed cost of about five slots and a little more than one per expert touched of the grouped kernels.  Measured on B200,
-  // 8 experts top-2, 4096 / 14336, us per layer, this way / grouped: one token 54 / 204, two 103 / 236, four 199 / 288,
-  // eight 400 / 362; 1024 / 1024: two tokens 21 / 51, four 36 / 53.
-  const size_t touched = slots < static_cast<size_t>(E) ? slots : static_cast<size_t>(E);
-  if (slots <= 5 + 9 * touched / 10 && !((reinterpret_cast<uintptr_t>(w13q) | reinterpret_cast<uintptr_t>(w2q) |
-                                          reinterpret_cast<uintptr_t>(hidden)) & 15)) {
+  if (few_token_moe_pays(T, H, I, E, top_k, expert_map != nullptr) &&
+      !((reinterpret_cast<uintptr_t>(w13q) | reinterpret_cast<uintptr_t>(w2q) |
+         reinterpret_cast<uintptr_t>(hidden)) & 15)) {
     for (int t = 0; t < T; t++) {
       st = ub::q4k_moe_one_token(static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(t) * H, act,
                                  static_cast<const __nv_bfloat16*>(hidden) + static_cast<size_t>(t) * H, w13q, w2q,
