@@ -83,3 +83,22 @@ def test_copied_weights_are_complete(dev, M, N, K, flag, between):
             matmul(d_other_y, d_other, 64)
         matmul(d_y, d_w[1], N, flag)
         assert np.array_equal(fetch(dev, d_y, DTYPE_F32, (M, N)), want)
+
+
+@pytest.mark.parametrize("dtype", sorted(ODT))
+@pytest.mark.parametrize("H", [8, 128, 256, 264, 512, 520, 1024, 2040, 2048, 2056, 3072, 3080])
+def test_a_row_is_normalised_alike_whatever_comes_with_it(dev, dtype, H):
+    """Rows that a warp takes where there are many, a CTA where there are few; in place as well."""
+    T, few = 3001, 5
+    rng = np.random.default_rng(H)
+    x = o.round_through(rng.standard_normal((T, H)).astype(np.float32) * 3, ODT[dtype])
+    d_g = dev.htod_sync_copy(to_storage(o.round_through(rng.uniform(0.5, 1.5, size=H).astype(np.float32), ODT[dtype]), dtype))
+    d_x, d_out, d_few = dev.htod_sync_copy(to_storage(x, dtype)), dev.alloc(T * H * 4), dev.alloc(few * H * 4)
+    ops.rms_norm(d_few, d_x, d_g, few, H, 1e-5, dtype, stream=dev.stream)
+    ops.rms_norm(d_out, d_x, d_g, T, H, 1e-5, dtype, stream=dev.stream)
+    got = fetch(dev, d_out, dtype, (T, H))
+    assert np.array_equal(got[:few], fetch(dev, d_few, dtype, (few, H)))
+    g = fetch(dev, d_g, dtype, (H,))
+    assert o.rel_l2(got, o.rms_norm(x, g, 1e-5, ODT[dtype])) < {DTYPE_F32: 1e-6, DTYPE_F16: 1e-3, DTYPE_BF16: 4e-3}[dtype]
+    ops.rms_norm(d_x, d_x, d_g, T, H, 1e-5, dtype, stream=dev.stream)
+    assert np.array_equal(fetch(dev, d_x, dtype, (T, H)), got)

@@ -138,6 +138,78 @@ __global__ void __launch_bounds__(256) rms_norm_row_kernel(T* out, const T* in, 
   for (int c = threadIdx.x + 256 * R; c < nv; c += 256) o[c] = norm(x[c], gm[c]);
 }
 
+// The same with a warp per row, for rows of up to 32 R pieces: a CTA and its barrier per row are more than such a row is
+// worth when there are many.  The sum of squares is taken in the order of the kernel above (eight groups of 32
+// pieces), so that a row's bits do not depend on how many rows come with it.
+template <typename T, int R>
+__global__ void __launch_bounds__(256) rms_norm_warp_kernel(T* out, const T* in, const T* __restrict__ gamma, int rows,
+                                                            int H, float eps) {
+  using namespace ub;
+  constexpr int V = Vec16<T>::N, G = R < 8 ? R : 8;
+  const int nv = H / V, lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_open();
+  if (row >= rows) return;
+  const Vec16<T>* x = reinterpret_cast<const Vec16<T>*>(in + static_cast<size_t>(row) * H);
+  Vec16<T>* o = reinterpret_cast<Vec16<T>*>(out + static_cast<size_t>(row) * H);
+  const Vec16<T>* gm = reinterpret_cast<const Vec16<T>*>(gamma);
+  Vec16<T> xv[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) xv[i].r = lane + 32 * i < nv ? x[lane + 32 * i].r : make_uint4(0, 0, 0, 0);
+  float acc[G];
+#pragma unroll
+  for (int g = 0; g < G; g++) acc[g] = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; i++)
+#pragma unroll
+    for (int e = 0; e < V; e++) acc[i % G] = fmaf(to_f32(xv[i].at(e)), to_f32(xv[i].at(e)), acc[i % G]);
+  // G sums over the lanes at once: at each of the first steps a lane keeps half of them
+#pragma unroll
+  for (int step = 16, n = G / 2; step > 0; step >>= 1, n >>= 1) {
+    if (n == 0) acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], step);
+#pragma unroll
+    for (int g = 0; g < n; g++) {
+      const bool upper = lane & step;
+      const float keep = upper ? acc[g + n] : acc[g], give = upper ? acc[g] : acc[g + n];
+      acc[g] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, step);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int g = 0; g < G; g++) ss += __shfl_sync(0xFFFFFFFFu, acc[0], g * (32 / G));
+  const float scale = rsqrtf(ss / static_cast<float>(H) + eps);
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int c = lane + 32 * i;
+    if (c < nv) {
+      const Vec16<T> g = gm[c];
+      Vec16<T> r;
+#pragma unroll
+      for (int e = 0; e < V; e++)
+        r.set(e, from_f32<T>(to_f32(from_f32<T>(to_f32(xv[i].at(e)) * scale)) * to_f32(g.at(e))));
+      o[c] = r;
+    }
+  }
+}
+// Measured on B200, bf16, us, a CTA / a warp per row (a warp per row with 2-byte accesses, the kernel of unaligned rows, before
+// either): 65536 rows of 128 values 173 / 11 (16), of 1024 189 / 41 (62), of 2048 216 / 80 (131); 4096 rows of 4096 17 / 21; 16
+// rows of 1024 1.6 / 2.5.
+template <typename T>
+int launch_rms_norm(void* out, const void* in, const void* gamma, int rows, int H, float eps, cudaStream_t s) {
+  T* o = static_cast<T*>(out);
+  const T *x = static_cast<const T*>(in), *g = static_cast<const T*>(gamma);
+  const int nv = H / ub::Vec16<T>::N;
+  auto kernel = rms_norm_row_kernel<T>;
+  auto warps = nv <= 32    ? rms_norm_warp_kernel<T, 1>
+               : nv <= 64  ? rms_norm_warp_kernel<T, 2>
+               : nv <= 128 ? rms_norm_warp_kernel<T, 4>
+               : nv <= 256 ? rms_norm_warp_kernel<T, 8>
+                           : rms_norm_warp_kernel<T, 12>;
+  if (nv <= 32 || (nv <= 384 && rows > 6 * ub::num_sms()))  // more rows than CTAs have room for at once
+    return ub::launch_pdl(warps, dim3((rows + 7) / 8), dim3(256), s, o, x, g, rows, H, eps);
+  return ub::launch_pdl(kernel, dim3(rows), dim3(256), s, o, x, g, H, eps);
+}
+
 // y += r (bf16), the residual add behind a matmul that could not carry it in its epilogue
 __global__ void add_bf16_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ r, size_t n) {
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -364,9 +436,7 @@ int topsaten_rms_norm(void* output, const void* input, const void* gamma, int nu
   const uintptr_t bits = reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(input) |
                          reinterpret_cast<uintptr_t>(gamma) | (static_cast<uintptr_t>(hidden_size) * (dtype_code == UB_DTYPE_F32 ? 4 : 2));
   if (!(bits & 15)) {
-    UB_DISPATCH_FLOAT(dtype_code, T, return ub::launch_pdl(rms_norm_row_kernel<T>, dim3(num_tokens), dim3(256), s,
-                                                           static_cast<T*>(output), static_cast<const T*>(input),
-                                                           static_cast<const T*>(gamma), hidden_size, epsilon));
+    UB_DISPATCH_FLOAT(dtype_code, T, return launch_rms_norm<T>(output, input, gamma, num_tokens, hidden_size, epsilon, s));
   }
   const int grid = (num_tokens + 7) / 8;
   UB_DISPATCH_FLOAT(dtype_code, T, (rms_norm_kernel<T><<<grid, 256, 0, s>>>(static_cast<T*>(output),
