@@ -102,3 +102,21 @@ def test_a_row_is_normalised_alike_whatever_comes_with_it(dev, dtype, H):
     assert o.rel_l2(got, o.rms_norm(x, g, 1e-5, ODT[dtype])) < {DTYPE_F32: 1e-6, DTYPE_F16: 1e-3, DTYPE_BF16: 4e-3}[dtype]
     ops.rms_norm(d_x, d_x, d_g, T, H, 1e-5, dtype, stream=dev.stream)
     assert np.array_equal(fetch(dev, d_x, dtype, (T, H)), got)
+
+
+@pytest.mark.parametrize("pieces", [1, 2, 3, 31, 32, 33, 128, 129, 256, 257])
+@pytest.mark.parametrize("rows", [1, 7, 300, 70001])
+def test_rows_of_any_number_of_pieces(dev, pieces, rows):
+    """Several rows in a CTA, the last of them missing; more rows than the grid is high.  Copy and SiLU.up."""
+    if rows * pieces > 300_000:
+        rows = 1500
+    rng = np.random.default_rng(pieces + rows)
+    src = rng.integers(0, 256, (rows, pieces + 1, 16), dtype=np.uint8)
+    d_s, d_d = dev.htod_sync_copy(src), dev.alloc(rows * pieces * 16)
+    check(lib().ub_copy_rows(d_d.ptr, pieces * 16, d_s.ptr, (pieces + 1) * 16, pieces * 16, rows, dev.stream), "copy_rows")
+    assert np.array_equal(dev.dtoh_sync_copy(d_d, np.uint8, (rows, pieces, 16)), src[:, :pieces])
+    D = pieces * 8
+    x = o.round_through(rng.standard_normal((rows, 2 * D)).astype(np.float32), o.UB_BF16)
+    d_o = dev.alloc(rows * D * 2)
+    ops.silu_and_mul(d_o, dev.htod_sync_copy(to_storage(x, DTYPE_BF16)), rows, D, DTYPE_BF16, stream=dev.stream)
+    assert np.allclose(fetch(dev, d_o, DTYPE_BF16, (rows, D)), o.silu_and_mul(x, o.UB_BF16), rtol=2 ** -7, atol=1e-7)

@@ -554,17 +554,30 @@ __global__ void __launch_bounds__(256) silu_and_mul_kernel(T* __restrict__ out, 
   }
 }
 
-// The same with 16-byte accesses (D whole 16-byte pieces, everything 16-byte aligned) and overlapped with its neighbours:
-// blockIdx.y walks the rows, so no element needs a division.
+// Row-wise kernels on 16-byte pieces: a CTA takes 2^lg pieces (at most 256) of each of 256 >> lg rows, blockIdx.y walks the
+// rows, so no element needs a division.  Measured on B200, SiLU.up, us, one row per CTA / this: 65536 rows of 64 values 36 / 6.2 (2-byte
+// accesses, the kernel of unaligned rows, 16), 4096 rows 5.1 / 1.8 (4.2).
+struct RowTiles {
+  int lg;
+  dim3 grid;
+  RowTiles(size_t nv, size_t rows) {
+    lg = 0;
+    while (lg < 8 && (static_cast<size_t>(1) << lg) < nv) lg++;
+    const size_t y = (rows + (256u >> lg) - 1) / (256u >> lg);
+    grid = dim3(static_cast<unsigned>((nv + (1u << lg) - 1) >> lg), static_cast<unsigned>(y < 32768 ? y : 32768));
+  }
+};
+
+// The same with 16-byte accesses (D whole 16-byte pieces, everything 16-byte aligned) and overlapped with its neighbours.
 template <typename T>
 __global__ void __launch_bounds__(256) silu_and_mul_vec_kernel(T* __restrict__ out, const T* __restrict__ in, int rows,
-                                                                int D) {
+                                                                int D, int lg) {
   constexpr int V = Vec16<T>::N;
-  const int c = blockIdx.x * 256 + threadIdx.x, nv = D / V;
+  const int c = (blockIdx.x << lg) + (threadIdx.x & ((1 << lg) - 1)), nv = D / V, per = 256 >> lg;
   pdl_wait();
   pdl_open();
   if (c >= nv) return;
-  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+  for (int r = blockIdx.y * per + (threadIdx.x >> lg); r < rows; r += gridDim.y * per) {
     const Vec16<T>* row = reinterpret_cast<const Vec16<T>*>(in + static_cast<size_t>(r) * 2 * D);
     const Vec16<T> g = row[c], u = row[nv + c];
     Vec16<T> o;
@@ -597,11 +610,12 @@ __global__ void __launch_bounds__(256) topk_sum_kernel(T* __restrict__ out, cons
 // start under itself: what it writes may be weights, which a matmul two launches on requests while the one in between runs.
 __global__ void __launch_bounds__(256) copy_rows_kernel(uint4* __restrict__ dst, size_t dst_pitch,
                                                         const uint4* __restrict__ src, size_t src_pitch, unsigned nv,
-                                                        unsigned rows) {
-  const unsigned c = blockIdx.x * 256 + threadIdx.x;
+                                                        unsigned rows, int lg) {
+  const unsigned c = (blockIdx.x << lg) + (threadIdx.x & ((1u << lg) - 1)), per = 256u >> lg;
   pdl_wait();
   if (c >= nv) return;
-  for (unsigned r = blockIdx.y; r < rows; r += gridDim.y) dst[r * dst_pitch + c] = src[r * src_pitch + c];
+  for (unsigned r = blockIdx.y * per + (threadIdx.x >> lg); r < rows; r += gridDim.y * per)
+    dst[r * dst_pitch + c] = src[r * src_pitch + c];
 }
 
 inline int ew_grid(size_t total) {
@@ -731,10 +745,9 @@ int ub_silu_and_mul(void* out, const void* in, int rows, int D, int dtype, void*
   const size_t total = static_cast<size_t>(rows) * D;
   const int esz = dtype == UB_DTYPE_F32 ? 4 : 2;
   if (!((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in) | (static_cast<uintptr_t>(D) * esz)) & 15)) {
-    const int nv = D / (16 / esz);
-    const dim3 grid((nv + 255) / 256, rows < 32768 ? rows : 32768);
-    UB_DISPATCH_FLOAT(dtype, T, return ub::launch_pdl(silu_and_mul_vec_kernel<T>, grid, dim3(256), ub::as_stream(stream),
-                                                      static_cast<T*>(out), static_cast<const T*>(in), rows, D));
+    const RowTiles t(D / (16 / esz), rows);
+    UB_DISPATCH_FLOAT(dtype, T, return ub::launch_pdl(silu_and_mul_vec_kernel<T>, t.grid, dim3(256), ub::as_stream(stream),
+                                                      static_cast<T*>(out), static_cast<const T*>(in), rows, D, t.lg));
   }
   UB_DISPATCH_FLOAT(dtype, T, (silu_and_mul_kernel<T><<<ew_grid(total), 256, 0, ub::as_stream(stream)>>>(
                                   static_cast<T*>(out), static_cast<const T*>(in), static_cast<size_t>(rows), D)));
@@ -759,9 +772,9 @@ int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch,
       ub::set_cuda_error(e);
       return ub::fail(UB_ERR_CUDA);
     }
-    const int st = ub::launch_pdl(copy_rows_kernel, dim3((nv + 255) / 256, rows < 32768 ? rows : 32768), dim3(256),
-                                  ub::as_stream(stream), static_cast<uint4*>(dst), dst_pitch >> 4,
-                                  static_cast<const uint4*>(src), src_pitch >> 4, nv, rows);
+    const RowTiles t(nv, rows);
+    const int st = ub::launch_pdl(copy_rows_kernel, t.grid, dim3(256), ub::as_stream(stream), static_cast<uint4*>(dst),
+                                  dst_pitch >> 4, static_cast<const uint4*>(src), src_pitch >> 4, nv, rows, t.lg);
     if (own != current) cudaSetDevice(current);
     if (st == UB_OK) ub::mark_weights_written(ub::as_stream(stream), dst, (height - 1) * dst_pitch + width);
     return st;
