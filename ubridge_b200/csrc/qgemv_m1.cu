@@ -1258,7 +1258,7 @@ int launch_m1_long(const uint8_t* wq, const XT* x, void* y, int N, int K, int y_
   ExpertSel esel;
   memset(&esel, 0, sizeof(esel));
   int w_rows = GU ? 2 * N : N;
-  if constexpr (GU) {
+  if constexpr (GU && std::is_same<XT, __nv_bfloat16>::value) {  // experts' activations are bf16
     if (sel) {
       esel = *sel, w_rows = sel_rows_total;
       kernel = nsb % 8 ? qgemv_q4k_m1_long_kernel<XT, true, false, true, true>
