@@ -312,6 +312,8 @@ int ub_indexed_moe_q4k(void* out, const void* in, const void* wq, const uint32_t
  * launches), on one stream with one caller-provided workspace.  expert_map may be NULL
  * (expert-parallel ranks pass local ids / -1, kernels/moe_align_host.cpp:298,535-543). */
 size_t ub_moe_layer_q4k_workspace_bytes(int T, int H, int I, int E, int top_k, int block_size);
+/* kernels that one call of these sizes launches (mapped: with an expert_map) */
+int ub_moe_layer_q4k_launches(int T, int H, int I, int E, int top_k, int block_size, int mapped);
 int ub_moe_layer_q4k(void* out, const void* hidden, const void* router_logits, const void* w13q, const void* w2q, const int32_t* expert_map, int T, int H, int I, int E, int top_k, int block_size, int norm_topk_prob, void* workspace, size_t ws_bytes, void* stream);
 
 /* ------------------------------------------------------------------ one-shot all-reduce over peer memory

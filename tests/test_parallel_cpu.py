@@ -143,3 +143,25 @@ def test_two_gloo_ranks_reproduce_the_unsharded_result(worker):
     kind, err, rng_ = q.get(timeout=10)
     # each rank rounds its own partial sums; the sum of two bf16-rounded halves differs from one rounding
     assert err < (1e-5 if kind == "tp" else 1e-2), (kind, err)
+
+
+@pytest.mark.parametrize("T,H,I,E,k,block,mapped,launches", [
+    (1, 4096, 14336, 8, 2, 64, 0, 3), (6, 4096, 14336, 8, 2, 64, 0, 13), (8, 4096, 14336, 8, 2, 64, 0, 7),
+    (10, 4096, 14336, 8, 2, 64, 1, 7), (6, 1024, 1024, 8, 2, 64, 0, 7), (1, 4096, 14336, 8, 3, 64, 0, 7),  # too long a row
+    (256, 4096, 14336, 8, 2, 64, 0, 7), (256, 4096, 14336, 8, 2, 24, 0, 6), (1, 100, 256, 8, 2, 64, 0, 0),
+    (1, 1024, 1024, 8, 16, 64, 0, 7),
+])
+def test_launches_of_an_expert_layer(T, H, I, E, k, block, mapped, launches):
+    """A token at a time (router and two per token) where the estimate and the kernels' limits allow, else grouped."""
+    from ubridge_b200._lib import lib
+
+    assert lib().ub_moe_layer_q4k_launches(T, H, I, E, k, block, mapped) == launches
+
+
+def test_launches_of_a_stack():
+    from ubridge_b200.parallel import TPLinearStack
+
+    for max_m, world, fused, want in ((1, 1, None, 4), (1, 2, None, 6), (1, 2, object(), 4), (4, 1, None, 6), (4, 2, None, 8)):
+        stack = TPLinearStack.__new__(TPLinearStack)
+        stack.max_m, stack.world, stack.fused = max_m, world, fused
+        assert stack.launches_per_forward == want

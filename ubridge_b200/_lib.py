@@ -145,6 +145,7 @@ _SIGS = {
     "ub_fused_moe_q4k_gemm": (c_int, [_P] * 7 + [c_int] * 9 + [_P, c_size_t, _P]),
     "ub_indexed_moe_q4k": (c_int, [_P, _P, _P, _P] + [c_int] * 7 + [_P]),
     "ub_moe_layer_q4k_workspace_bytes": (c_size_t, [c_int] * 6),
+    "ub_moe_layer_q4k_launches": (c_int, [c_int] * 7),
     "ub_moe_layer_q4k": (c_int, [_P] * 6 + [c_int] * 7 + [_P, c_size_t, _P]),
     "ecclGetVersion": (c_int, [POINTER(c_int)]),
     "ecclGetUniqueId": (c_int, [POINTER(EcclUniqueId)]),

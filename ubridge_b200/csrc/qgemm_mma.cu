@@ -253,6 +253,8 @@ int q4k_gemm_mma(void* y, const void* x, const void* wq, int M, int N, int K, cu
 namespace ub {
 int q4k_moe_one_token(void* out, void* act, const void* x, const void* w13, const void* w2, const int32_t* idx,
                       const void* weights, const int32_t* map, int H, int I, int E, int slots, cudaStream_t s);
+bool q4k_moe_one_token_takes(int H, int I, int slots);
+bool q4k_moe_tc_takes(int positions, int K, int N, int block);
 bool q4k_moe_tc_supported(int positions, int K, int N, int block);
 int moe_gather_rows(void* xg, const void* hidden, const int32_t* sorted_ids, const int32_t* num_post_pad, int positions,
                     int num_valid, int top_k, int H, cudaStream_t s);
@@ -273,14 +275,17 @@ namespace {
 // 4096 / 14336 four tokens 103 / 115, six 147 / 138; 1024 / 1024 four tokens 32 / 34, six 46 / 37.
 bool few_token_moe_pays(int T, int H, int I, int E, int top_k, bool mapped) {
   if (top_k > E) return false;
-  const float mb = 3.f * H * I * (UB_Q4K_BYTES / 256.f) * 1e-6f;
+  const float half = static_cast<float>(H) * I * (UB_Q4K_BYTES / 256.f) * 1e-6f, mb = 3.f * half;
+  // the one-token kernels take rows in stages of 2048 values, filled or not
+  auto filled = [](int k) { return static_cast<float>((k + 2047) / 2048 * 2048) / k; };
+  const float staged = half * (2.f * filled(H) + filled(I));
   const float touched = E * (1.f - powf(1.f - static_cast<float>(top_k) / E, static_cast<float>(T)));
-  auto cheaper = [&](float own) {  // own: share of the experts that this rank holds
-    const float one = 5.8f + T * (6.4f + own * top_k * (.45f + .243f * mb));
+  auto cheaper = [&](float own, float margin) {  // own: share of the experts that this rank holds
+    const float one = 5.f + T * (6.6f + own * top_k * (.45f + .215f * staged));
     const float grouped = 22.4f + 1.25f * ((H + I) / 256) + own * touched * (.41f + .31f * mb);
-    return one <= grouped;
+    return one * margin <= grouped;
   };
-  return cheaper(1.f) && (!mapped || cheaper(1.f / E));
+  return cheaper(1.f, 1.f) && (!mapped || cheaper(1.f / E, 1.15f));
 }
 
 }  // namespace
@@ -342,6 +347,15 @@ size_t ub_moe_layer_q4k_workspace_bytes(int T, int H, int I, int E, int top_k, i
   b += align_up(slots * H * 2, 256);
   b += align_up(max_padded * H * 2, 256);
   return b;
+}
+
+// Kernels of one ub_moe_layer_q4k of these sizes, pointers aligned.  A token at a time: router and two per token.  Grouped:
+// router, weight conversion, alignment, two GEMMs and the sum, with the tensor-core GEMMs the gathering of the tokens too.
+int ub_moe_layer_q4k_launches(int T, int H, int I, int E, int top_k, int block_size, int mapped) {
+  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || top_k <= 0 || block_size <= 0 || H % UB_QK_K || I % UB_QK_K) return 0;
+  if (few_token_moe_pays(T, H, I, E, top_k, mapped != 0) && ub::q4k_moe_one_token_takes(H, I, top_k)) return 1 + 2 * T;
+  const int positions = static_cast<int>(static_cast<size_t>(T) * top_k + static_cast<size_t>(E) * (block_size - 1));
+  return ub::q4k_moe_tc_takes(positions, H, I, block_size) && ub::q4k_moe_tc_takes(positions, I, H, block_size) ? 7 : 6;
 }
 
 int ub_moe_layer_q4k(void* out, const void* hidden, const void* router_logits, const void* w13q, const void* w2q,

@@ -645,9 +645,12 @@ int q8_0_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bo
 }
 
 // Limits of the grouped tcgen05 path; outside them the caller keeps the mma.sync kernels.
+bool q4k_moe_tc_takes(int positions, int K, int N, int block) {
+  return block > 0 && block % 16 == 0 && block <= 128 && K % UB_QK_K == 0 && N % 8 == 0 &&
+         (positions + block - 1) / block <= kTcMaxRuns;
+}
 bool q4k_moe_tc_supported(int positions, int K, int N, int block) {
-  return encode_tiled_fn() != nullptr && block > 0 && block % 16 == 0 && block <= 128 && K % UB_QK_K == 0 &&
-         N % 8 == 0 && (positions + block - 1) / block <= kTcMaxRuns;
+  return encode_tiled_fn() != nullptr && q4k_moe_tc_takes(positions, K, N, block);
 }
 
 // Gathers hidden rows into aligned order: xg[positions, H].

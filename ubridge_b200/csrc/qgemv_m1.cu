@@ -1346,12 +1346,14 @@ int q4k_gemv_m1_gate_up(const void* wq, const XT* x, void* y, int N, int K, int 
 // One token through its `slots` experts: act[slots][I] = silu(gate) * up from w13 ([E][2 I rows of H]), then
 // out[H] = sum over the slots of weight * (act . w2^T), w2 [E][H rows of I].  Two launches; act is scratch.
 // UB_ERR_UNSUPPORTED (nothing launched): rows too long for one pass, more slots or stages than the kernels keep.
+bool q4k_moe_one_token_takes(int H, int I, int slots) {
+  const int stages = slots * ((I / UB_QK_K + 7) / 8);
+  return slots <= kSelMax && H % UB_QK_K == 0 && I % UB_QK_K == 0 && (H / UB_QK_K + 7) / 8 <= kMaxChunks &&
+         stages <= 2 * kWideMaxUnits;
+}
 int q4k_moe_one_token(void* out, void* act, const void* x, const void* w13, const void* w2, const int32_t* idx,
                       const void* weights, const int32_t* map, int H, int I, int E, int slots, cudaStream_t s) {
-  const int stages = slots * ((I / UB_QK_K + 7) / 8);
-  if (slots > kSelMax || H % UB_QK_K || I % UB_QK_K || (H / UB_QK_K + 7) / 8 > kMaxChunks || stages > 2 * kWideMaxUnits ||
-      !ub::tensor_map_encoder())
-    return UB_ERR_UNSUPPORTED;
+  if (!q4k_moe_one_token_takes(H, I, slots) || !ub::tensor_map_encoder()) return UB_ERR_UNSUPPORTED;
   ArParams none;
   memset(&none, 0, sizeof(none));
   ExpertSel sel = {idx, static_cast<const __nv_bfloat16*>(weights), map, slots, 2 * I, E};

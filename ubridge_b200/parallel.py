@@ -140,11 +140,11 @@ class TPLinearStack:
     @property
     def launches_per_forward(self) -> int:
         """Kernels of this library per forward() at max_m: one token runs four launches (SiLU.up and the
-        exchanges ride in the matmuls' epilogues); otherwise four matmuls, SiLU.up and, beyond one rank, two
-        all-reduces (the stand-in copy for attention is a device copy, not a kernel of this library)."""
+        exchanges ride in the matmuls' epilogues); otherwise four matmuls (one launch each where the tokens take one pass),
+        the stand-in copy for attention, SiLU.up and, beyond one rank, two all-reduces."""
         if self.max_m == 1:
             return 4 if (self.world == 1 or self.fused is not None) else 6
-        return 5 + (2 if self.world > 1 else 0)
+        return 6 + (2 if self.world > 1 else 0)
 
     def _mm(self, y, x, w, M, N, K):
         ops.qmatmul(y, x, w, M, N, K, is_q4k=True, x_dtype=DTYPE_BF16, out_dtype=DTYPE_BF16, workspace=self.ws,
@@ -196,8 +196,10 @@ class EPMoELayer:
         self.ws = dev.alloc(self.ws_bytes)
         self.out = dev.alloc(T * H * 2)
 
-    # kernels per forward(): router, weight conversion, alignment, two grouped GEMMs, top-k sum
-    launches_per_forward = 6
+    @property
+    def launches_per_forward(self) -> int:
+        """Kernels of this library per forward(), the exchange not counted."""
+        return lib().ub_moe_layer_q4k_launches(self.T, self.H, self.I, self.E, self.top_k, self.block, self.map is not None)
 
     def forward(self, hidden, logits, norm_topk_prob: bool = True):
         ops.moe_layer_q4k(self.out, hidden, logits, self.w13, self.w2, self.T, self.H, self.I, self.E, self.top_k,
