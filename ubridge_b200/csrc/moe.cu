@@ -763,21 +763,14 @@ int ub_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch,
   const size_t bits = reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | dst_pitch | src_pitch | width;
   if (!(bits & 15) && width < (1u << 30) && height < (1u << 30)) {
     const unsigned nv = static_cast<unsigned>(width >> 4), rows = static_cast<unsigned>(height);
-    // a kernel is launched on the current device, a copy of the runtime on its stream's
-    int current = 0, own = 0;
-    cudaError_t e = cudaGetDevice(&current);
-    if (e == cudaSuccess) e = stream ? cudaStreamGetDevice(ub::as_stream(stream), &own) : (own = current, cudaSuccess);
-    if (e == cudaSuccess && own != current) e = cudaSetDevice(own);
-    if (e != cudaSuccess) {
-      ub::set_cuda_error(e);
-      return ub::fail(UB_ERR_CUDA);
-    }
     const RowTiles t(nv, rows);
     const int st = ub::launch_pdl(copy_rows_kernel, t.grid, dim3(256), ub::as_stream(stream), static_cast<uint4*>(dst),
                                   dst_pitch >> 4, static_cast<const uint4*>(src), src_pitch >> 4, nv, rows, t.lg);
-    if (own != current) cudaSetDevice(current);
-    if (st == UB_OK) ub::mark_weights_written(ub::as_stream(stream), dst, (height - 1) * dst_pitch + width);
-    return st;
+    if (st == UB_OK) {
+      ub::mark_weights_written(ub::as_stream(stream), dst, (height - 1) * dst_pitch + width);
+      return st;
+    }
+    cudaGetLastError();  // a stream of another device than the current one: a copy of the runtime goes by its stream
   }
   const cudaError_t e = cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, height, cudaMemcpyDeviceToDevice,
                                           ub::as_stream(stream));
