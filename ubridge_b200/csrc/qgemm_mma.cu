@@ -272,7 +272,7 @@ namespace {
 // 302 / 323, eight 400 / 326; 1024 / 1024 three tokens 28 / 36, four 36 / 36, six 51 / 37.
 // mapped: a rank that holds some of the experts, the host does not know how many.  Both ways cost less the fewer it holds;
 // one at a time is taken where it is the cheaper way with one of them as well as with all.  8 ranks of one expert each, us:
-// 4096 / 14336 four tokens 103 / 115, six 147 / 138; 1024 / 1024 four tokens 32 / 34, six 46 / 37.
+// 4096 / 14336 four tokens 87 / 121, six 107 / 129, eight 138 / 122; 1024 / 1024 four tokens 31 / 35, six 42 / 34.
 bool few_token_moe_pays(int T, int H, int I, int E, int top_k, bool mapped) {
   if (top_k > E) return false;
   const float half = static_cast<float>(H) * I * (UB_Q4K_BYTES / 256.f) * 1e-6f, mb = 3.f * half;
@@ -280,12 +280,12 @@ bool few_token_moe_pays(int T, int H, int I, int E, int top_k, bool mapped) {
   auto filled = [](int k) { return static_cast<float>((k + 2047) / 2048 * 2048) / k; };
   const float staged = half * (2.f * filled(H) + filled(I));
   const float touched = E * (1.f - powf(1.f - static_cast<float>(top_k) / E, static_cast<float>(T)));
-  auto cheaper = [&](float own, float margin) {  // own: share of the experts that this rank holds
+  auto cheaper = [&](float own) {  // own: share of the experts that this rank holds
     const float one = 5.f + T * (6.6f + own * top_k * (.45f + .215f * staged));
     const float grouped = 22.4f + 1.25f * ((H + I) / 256) + own * touched * (.41f + .31f * mb);
-    return one * margin <= grouped;
+    return one <= grouped;
   };
-  return cheaper(1.f, 1.f) && (!mapped || cheaper(1.f / E, 1.15f));
+  return cheaper(1.f) && (!mapped || cheaper(1.f / E));
 }
 
 }  // namespace

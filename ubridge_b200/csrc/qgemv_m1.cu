@@ -1047,6 +1047,14 @@ qgemv_q4k_m1_wide_kernel(const XT* __restrict__ x, void* __restrict__ y, int N, 
     __syncwarp();
   }
 
+  if (SEL && own == 0) {  // no expert of this token is here: the empty stages would still pass through the ring one by one
+    for (int i = threadIdx.x; i < my_tiles * 16; i += kWideWarps * 32) {
+      const int row = 16 * (static_cast<int>(blockIdx.x) + (i >> 4) * static_cast<int>(gridDim.x)) + (i & 15);
+      if (row < N) st_out(y, row, y_dtype, 0.f);
+    }
+    return;
+  }
+
   uint32_t off_h, off_q[4];
   {
     auto swz = [](uint32_t L) { return ODD ? L : L ^ (((L >> 7) & 7u) << 4); };
