@@ -27,7 +27,8 @@ def _layer(dev, T, H, I, E, k, hidden, logits, w13, w2, emap=None, norm=True):
     (2, 768, 1280, 5, 3, False),    # boxes of two super-blocks, an odd number of stages over the slots
     (3, 1024, 14336, 4, 2, True),   # two slots of seven stages: the longest the down launch takes
     (2, 512, 1024, 12, 8, True),    # eight slots
-    (6, 512, 768, 8, 2, True), (7, 512, 768, 8, 2, True),  # the most tokens of eight experts top-2, and one more
+    (3, 512, 768, 8, 2, True),      # the most tokens of this size that go one at a time
+    (6, 512, 768, 8, 2, True), (7, 512, 768, 8, 2, True),  # more: the grouped kernels
     (2, 512, 28672, 3, 2, True),    # more stages than the down launch takes: the grouped kernels
 ])
 @pytest.mark.parametrize("mapped", [False, True])

@@ -633,9 +633,9 @@ int q4k_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, boo
 
 // Same product for Q8_0 rows (K/32 blocks of 34 bytes); K % 256 == 0 (a row must be whole 16-byte pieces) and wq
 // 16-byte aligned, else UB_ERR_UNSUPPORTED and the caller keeps the decode kernel.  The 272-byte slots of the
-// packed ring leave room for four token stages at 256 tokens.  Measured on B200, 4096x4096 with 512 tokens
-// (64 tiles of 256 tokens on 148 SMs): 505 TFLOP/s; with 128-token tiles (128 tiles) 400: the producers'
-// work per flop doubles, which costs more than the idle SMs.
+// packed ring leave room for four token stages at 256 tokens.  No K split and 256-token tiles from 129 tokens on, however few
+// tiles there are: the comparison with 128-token tiles on record (4096x4096, 512 tokens: 505 TFLOP/s against 400) is of
+// producers that were slower by a fifth; the rule of q4k_gemm_tc has not been measured for this format.
 int q8_0_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s) {
   if (K % UB_QK_K || (reinterpret_cast<uintptr_t>(wq) & 15)) return UB_ERR_UNSUPPORTED;
   const TcGroup none = {nullptr, nullptr, nullptr, nullptr, 0, 0, 0};

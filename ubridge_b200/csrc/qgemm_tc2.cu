@@ -7,8 +7,10 @@
 // bf16 operand would keep 8 bits of a weight.  So every weight is the sum of TWO bf16 values: w = d * scale * q - min is
 // computed in f32, the first piece is w rounded to bf16 and the second the remainder rounded to bf16 (together within
 // 2^-18 of w), and each K step multiplies the token tile by both.  f32 activations are split too (upper 16 bits and the
-// remainder, which no magnitude overflows; within 2^-17); their product takes three MMAs (hi.hi, lo.hi, hi.lo), the
-// fourth is below 2^-17 of a term and of either sign.
+// remainder, which no magnitude overflows; within 2^-16); their product takes three MMAs (hi.hi, lo.hi, hi.lo), the
+// fourth is below 2^-16 of a term and of either sign.  Error against f64, 2-norm of f32 results: 2e-6 to 5e-6, with f32
+// activations 4e-6 to 1.2e-5 (rounding the first piece instead: 3.5e-6, but the second conversion per pair made 333
+// tokens through 4096x4096 159 us instead of 108).
 //
 // One CTA per SM, tiles of 128 weight rows x up to TOK tokens, K in steps of 64 values:
 //   warp 0        one lane issues tcgen05.mma (A from tensor memory, B from shared memory) and tcgen05.commit
