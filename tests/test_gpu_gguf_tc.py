@@ -74,3 +74,27 @@ def test_half_the_rows_take_no_longer(dev):
             best = min(best, a.elapsed_time(b) * 50)
         us[N] = best
     assert us[2048] < 1.1 * us[4096], us
+
+
+@pytest.mark.parametrize("x_dtype", [DTYPE_BF16, DTYPE_F32])
+@pytest.mark.parametrize("tag,M,K", [(o.GGML_Q6_K, 9, 2048), (o.GGML_Q5_K, 70, 768), (12, 6, 5120), (12, 40, 2048), (8, 33, 1280)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_token_that_is_not_finite(dev, x_dtype, tag, M, K, bad):
+    """Two pieces and one: that token's results are not finite (an infinity may become NaN: products with the second piece),
+    the others keep their bits."""
+    N = 200
+    gen = dict(GEN)
+    gen[12], gen[8] = o.gen_q4k_weight, o.gen_q8_0_weight
+    rng = np.random.default_rng(tag + M)
+    d_w = dev.htod_sync_copy(np.ascontiguousarray(gen[tag](rng, N, K)).reshape(-1))
+    x = o.gen_activation(rng, M, K, x_dtype == DTYPE_BF16)
+    y = []
+    for value in (x[2, 100], bad):
+        x[2, 100] = value
+        ws, d_y = dev.alloc(1 << 20), dev.alloc(M * N * 4)
+        ops.qmatmul_gguf(d_y, dev.htod_sync_copy(to_storage(x, x_dtype)), d_w, tag, M, N, K, x_dtype=x_dtype,
+                         out_dtype=DTYPE_BF16, workspace=ws, ws_bytes=1 << 20, stream=dev.stream)
+        y.append(fetch(dev, d_y, DTYPE_BF16, (M, N)))
+    others = [m for m in range(M) if m != 2]
+    assert np.isfinite(y[0]).all() and not np.isfinite(y[1][2]).any()
+    assert np.array_equal(y[0][others], y[1][others])

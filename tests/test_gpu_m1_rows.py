@@ -4,8 +4,8 @@ import numpy as np
 import pytest
 
 from oracle import oracle as o
-from ubridge_b200 import DTYPE_BF16, DTYPE_F32, ops
-from ubridge_b200._lib import UbridgeError
+from ubridge_b200 import DTYPE_BF16, DTYPE_F16, DTYPE_F32, ops
+from ubridge_b200._lib import UbridgeError, check, lib
 
 from _util import fetch, to_storage
 
@@ -101,3 +101,35 @@ def test_long_rows_keep_their_precision(dev, K, bound):
                 out_dtype=DTYPE_F32, stream=dev.stream)
     assert o.rel_l2(fetch(dev, d_y, DTYPE_F32, (1, N)), x.astype(np.float64) @ o.c_dequant(w, True).reshape(N, K).T) < bound
     assert dev.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K", [(300, 768), (520, 5120), (40, 11008), (300, 13824), (300, 17920)])
+def test_residual_behind_rows_of_any_length(dev, N, K):
+    """The epilogue that adds a residual row, on boxes of two super-blocks, odd ones among them, and in several passes."""
+    import ctypes
+
+    rng = np.random.default_rng(N + K)
+    w = o.gen_q4k_weight(rng, N, K)
+    x, r = o.gen_activation(rng, 1, K, True), o.round_through(rng.standard_normal((1, N)).astype(np.float32), o.UB_BF16)
+    d = [dev.htod_sync_copy(v) for v in (to_storage(x, DTYPE_BF16), w, to_storage(r, DTYPE_BF16))]
+    d_y = dev.alloc(N * 2)
+    check(lib().ub_qmatmul_q4k_allreduce_residual_bf16(ctypes.c_void_p(d_y.ptr), ctypes.c_void_p(d[0].ptr),
+                                                       ctypes.c_void_p(d[1].ptr), ctypes.c_void_p(d[2].ptr), 1, N, K, None,
+                                                       0, 1, 0, dev.stream), "residual")
+    assert o.rel_l2(fetch(dev, d_y, DTYPE_BF16, (1, N)), r + o.c_qmatmul(x, w, N, K, True)) < 5e-3  # one rounding to bf16
+    assert dev.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K", [(300, 768), (300, 5120), (300, 13824), (300, 14336)])
+def test_f16_results(dev, N, K):
+    """The f32 result rounded once (activations small enough that none overflows)."""
+    rng = np.random.default_rng(N + K)
+    d_w = dev.htod_sync_copy(o.gen_q4k_weight(rng, N, K))
+    x = o.round_through(o.gen_activation(rng, 1, K, True) * 0.0625, o.UB_BF16)
+    d_x = dev.htod_sync_copy(to_storage(x, DTYPE_BF16))
+    y = {}
+    for dt in (DTYPE_F32, DTYPE_F16):
+        d_y = dev.alloc(N * 4)
+        ops.qmatmul(d_y, d_x, d_w, 1, N, K, is_q4k=True, x_dtype=DTYPE_BF16, out_dtype=dt, stream=dev.stream)
+        y[dt] = fetch(dev, d_y, dt, (1, N))
+    assert np.array_equal(y[DTYPE_F16], y[DTYPE_F32].astype(np.float16).astype(np.float32))

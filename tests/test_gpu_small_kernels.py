@@ -120,3 +120,67 @@ def test_rows_of_any_number_of_pieces(dev, pieces, rows):
     d_o = dev.alloc(rows * D * 2)
     ops.silu_and_mul(d_o, dev.htod_sync_copy(to_storage(x, DTYPE_BF16)), rows, D, DTYPE_BF16, stream=dev.stream)
     assert np.allclose(fetch(dev, d_o, DTYPE_BF16, (rows, D)), o.silu_and_mul(x, o.UB_BF16), rtol=2 ** -7, atol=1e-7)
+
+
+@pytest.mark.parametrize("tag,M", [(o.GGML_Q6_K, 6), (o.GGML_Q5_K, 9), (o.GGML_Q4_0, 40), (8, 12)])
+def test_copied_weights_of_other_formats_are_complete(dev, tag, M):
+    """The same for the tensor-core launches of the other formats, which request weights early for rows of whole 2048 values."""
+    N, K = 2048, 4096
+    gen = {o.GGML_Q4_0: o.gen_q4_0_weight, o.GGML_Q5_K: o.gen_q5k_weight, o.GGML_Q6_K: o.gen_q6k_weight, 8: o.gen_q8_0_weight}
+    rng = np.random.default_rng(tag + M)
+    w = np.ascontiguousarray(gen[tag](rng, N, K)).reshape(8, -1)  # eight pieces of whole 16 bytes
+    wide = np.zeros((8, w.shape[1] + 64), dtype=np.uint8)
+    wide[:, 32:-32] = w
+    d_wide, d_w = dev.htod_sync_copy(wide), dev.htod_sync_copy(w)
+    d_x, d_y = dev.htod_sync_copy(to_storage(o.gen_activation(rng, M, K, True), DTYPE_BF16)), dev.alloc(M * N * 2)
+
+    def matmul():
+        ops.qmatmul_gguf(d_y, d_x, d_w, tag, M, N, K, x_dtype=DTYPE_BF16, out_dtype=DTYPE_BF16, stream=dev.stream)
+
+    matmul()
+    want = fetch(dev, d_y, DTYPE_BF16, (M, N))
+    for rep in range(3):
+        d_w = dev.alloc_zeros(w.size)
+        dev.synchronize()
+        check(lib().ub_copy_rows(d_w.ptr, w.shape[1], d_wide.ptr + 32, wide.shape[1], w.shape[1], 8, dev.stream), "copy_rows")
+        matmul()
+        assert np.array_equal(fetch(dev, d_y, DTYPE_BF16, (M, N)), want)
+
+
+@pytest.mark.parametrize("M", [1, 4, 20])
+def test_a_chain_gives_the_same_with_and_without_waiting(dev, M):
+    """Norm, matmul, copy, matmul, SiLU.up, matmul into the same buffers over and over: every launch overlaps its neighbours,
+    the result is that of the chain with a wait behind every call."""
+    rng = np.random.default_rng(M)
+    H, I = 1024, 1280
+    w1, w2, w3 = (dev.htod_sync_copy(o.gen_q4k_weight(rng, n, k)) for n, k in ((H + 512, H), (2 * I, H), (H, I)))
+    d_g = dev.htod_sync_copy(to_storage(np.full(H, 0.01, dtype=np.float32), DTYPE_BF16))
+    x = to_storage(o.gen_activation(rng, M, H, True), DTYPE_BF16)
+    bufs = [dev.alloc(M * n * 2) for n in (H, H + 512, H, 2 * I, I)]
+    ws = dev.alloc(1 << 20)
+
+    def chain(wait):
+        d_x = dev.htod_sync_copy(x)
+        a, b, c, d, e = bufs
+
+        def mm(y, src, w, n, k):
+            ops.qmatmul(y, src, w, M, n, k, is_q4k=True, x_dtype=DTYPE_BF16, out_dtype=DTYPE_BF16, workspace=ws,
+                        ws_bytes=1 << 20, stream=dev.stream)
+            wait()
+
+        for _ in range(6):
+            ops.rms_norm(a, d_x, d_g, M, H, 1e-5, DTYPE_BF16, stream=dev.stream)
+            wait()
+            mm(b, a, w1, H + 512, H)
+            check(lib().ub_copy_rows(c.ptr, H * 2, b.ptr, (H + 512) * 2, H * 2, M, dev.stream), "copy_rows")
+            wait()
+            mm(d, c, w2, 2 * I, H)
+            ops.silu_and_mul(e, d, M, I, DTYPE_BF16, stream=dev.stream)
+            wait()
+            mm(d_x, e, w3, H, I)
+        return fetch(dev, d_x, DTYPE_BF16, (M, H))
+
+    want = chain(dev.synchronize)
+    assert np.isfinite(want).all()
+    for _ in range(3):
+        assert np.array_equal(chain(lambda: None), want)
