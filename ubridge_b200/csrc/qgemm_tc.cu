@@ -28,8 +28,8 @@
 //   warps 1-4     epilogue: tcgen05.ld -> bf16 -> staging tile in shared memory (accumulator released
 //                 here) -> 16-byte coalesced stores to y, overlapping the next tile's main loop
 //   warps 5-12    weight producers: read their row's packed super-block from a shared-memory ring, turn
-//                 nibbles into bf16 (128 + q) with one byte permute per pair, minus 128 (exact), times d*sc
-//                 minus dmin*m with packed bf16 FMAs; tcgen05.st; the stage is handed over (tcgen05.wait::st, mbarrier
+//                 nibbles into the bf16 q * 2^-133 with one byte permute per pair, times d*sc minus dmin*m with
+//                 packed bf16 FMAs (rowblock.cuh); tcgen05.st; the stage is handed over (tcgen05.wait::st, mbarrier
 //                 arrive) after the next one's arithmetic
 //   warp 13       one lane issues all bulk copies: packed weight tiles ([128 rows][144 bytes], one 2-D
 //                 tensor-map copy per super-block column, two super-blocks ahead) and token tiles (one
@@ -328,7 +328,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int j = 0; j < 32; j++) {
-            float f = __uint_as_float(v[j]);
+            float f = __uint_as_float(v[j]) * one_piece_unscale(FMT ? kQ8 : kQ4K);
             if (MODE == 2) f *= run_w[c0 + c + j];
             st_col[(c + j) * 128] = __float2bfloat16_rn(f);
           }

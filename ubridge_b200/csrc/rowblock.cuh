@@ -19,23 +19,21 @@ constexpr uint32_t row_sb_bytes(int f) { return f == kQ8 ? 272 : f == kQ6K ? 210
 constexpr uint32_t slot_pitch(int f) { return f == kQ6K ? 240 : row_sb_bytes(f); }
 constexpr uint32_t slot_bytes(int f) { return (f == kQ6K ? 136 : 128) * slot_pitch(f); }
 
-// Two nibbles (bytes A and B of a word masked with 0x0F0F0F0F) -> packed bf16 (dsc*qA - dm, dsc*qB - dm)
+// Two bytes A and B of a word -> packed bf16 (s * byte + c).  A byte n with nothing above it is the bf16 n * 2^-133, below 128
+// a subnormal, from there on the first normal binade, which has the same spacing: no bias to subtract.  s carries 2^133.
 template <int SEL>
-__device__ __forceinline__ uint32_t deq_pair(uint32_t w4, __nv_bfloat162 dsc, __nv_bfloat162 ndm) {
-  const uint32_t biased = __byte_perm(w4, 0x43434343u, SEL);  // bf16 (128 + q) in each half
-  const uint32_t c128 = 0x43004300u;
-  const __nv_bfloat162 q = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&biased),
-                                   *reinterpret_cast<const __nv_bfloat162*>(&c128));
-  return bf162_bits(__hfma2(q, dsc, ndm));
+__device__ __forceinline__ uint32_t deq_pair(uint32_t w4, __nv_bfloat162 s, __nv_bfloat162 c) {
+  const uint32_t n = __byte_perm(w4, 0u, SEL);
+  return bf162_bits(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&n), s, c));
 }
 
-// Two signed bytes A and B of a word (given as its low seven bits and its sign bits) -> packed bf16 (d*qA, d*qB):
-// 0x43 over the low seven bits is bf16 (128 + m), 0x43 over the sign bit is 128 or 256, their difference is q.
+// Two signed bytes A and B of a word (given with their sign bits flipped: q + 128) -> packed bf16 (d * q): q 2^-6 from the bf16
+// n * 2^-133 in one exact step (2^127 n 2^-133 - 2), then d in two pieces, which carry 2^6: fma(q, dh, q dl) is d q rounded once.
 template <int SEL>
-__device__ __forceinline__ uint32_t deq8_pair(uint32_t lo7, uint32_t sg, __nv_bfloat162 dh, __nv_bfloat162 dl) {
-  const uint32_t biased = __byte_perm(lo7, 0x43434343u, SEL), off = __byte_perm(sg, 0x43434343u, SEL);
-  const __nv_bfloat162 q = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&biased),
-                                   *reinterpret_cast<const __nv_bfloat162*>(&off));
+__device__ __forceinline__ uint32_t deq8_pair(uint32_t u4, __nv_bfloat162 dh, __nv_bfloat162 dl) {
+  const uint32_t n = __byte_perm(u4, 0u, SEL), big = 0x7F007F00u, two = 0xC000C000u;
+  const __nv_bfloat162 q = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&n), *reinterpret_cast<const __nv_bfloat162*>(&big),
+                                   *reinterpret_cast<const __nv_bfloat162*>(&two));
   return bf162_bits(__hfma2(q, dh, __hmul2(q, dl)));
 }
 
@@ -85,6 +83,18 @@ __device__ __forceinline__ int lds_s8(uint32_t a) {
   return v;
 }
 
+// What the two forms cost, B200, 16 warps per SM, cycles for 256 values of 128 rows with the tcgen05.st: Q4_K one piece 636
+// (884 while the nibbles were biased by 128 and the bias subtracted: byte permutes, logic and 16-bit arithmetic all issue at half
+// rate, ten instructions per eight values now take 12 cycles of the one pipe and 8 of the other instead of 14 and 16), two
+// pieces 2100.  It is the largest part of a launch of few tokens: 16 tokens through 28672x4096 26.4 -> 23.9 us, Q8_0 45 tokens
+// 14336x4096 24.8 -> 21.8 us.
+//
+// one_piece: values times 2^-one_piece_exp, which the kernels' epilogues take back from the f32 sums.  Q4_K: with 2^28 the
+// scale times 2^133 stays finite for every f16 super-block scale (65504 * 63 * 2^105 < 2^127), and the smallest (6e-8)
+// is 2e-16, nowhere near bf16's smallest normal number: every bit of the values is the same without it.
+constexpr int one_piece_exp(int f) { return f == kQ4K ? 28 : 0; }
+constexpr float one_piece_unscale(int f) { return f == kQ4K ? 0x1p28f : 1.f; }
+
 template <int FMT>
 struct RowBlock {
   uint32_t base;  // shared-memory address of the row's block: 16-byte aligned, Q6_K: 2-byte aligned
@@ -129,13 +139,13 @@ struct RowBlock {
       uint32_t q[8];
       lds128(base + 16 + 32 * G, q), lds128(base + 32 + 32 * G, q + 4);
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
+      for (int h = 0; h < 2; h++) {  // upper nibbles stay where they are: 16 q
         float s, m;
         pair(2 * G + h, s, m);
-        const __nv_bfloat162 dsc = __float2bfloat162_rn(s), ndm = __float2bfloat162_rn(-m);
+        const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 0x1p101f : 0x1p105f)), ndm = __float2bfloat162_rn(m * -0x1p-28f);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          const uint32_t v = (h ? q[i] >> 4 : q[i]) & 0x0F0F0F0Fu;
+          const uint32_t v = q[i] & (h ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
           ot[16 * h + 2 * i] = deq_pair<0x4140>(v, dsc, ndm);
           ot[16 * h + 2 * i + 1] = deq_pair<0x4342>(v, dsc, ndm);
         }
@@ -146,16 +156,16 @@ struct RowBlock {
       uint32_t prev = lds32(at);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const float df = half_bits_to_f32(h ? prev >> 16 : prev);
-        const __nv_bfloat16 dh1 = __float2bfloat16_rn(df);  // d in two pieces: fma(q, dh, q dl) is d q rounded once
+        const float df = 64.f * half_bits_to_f32(h ? prev >> 16 : prev);
+        const __nv_bfloat16 dh1 = __float2bfloat16_rn(df);
         const __nv_bfloat162 dh = __bfloat162bfloat162(dh1), dl = __float2bfloat162_rn(df - __bfloat162float(dh1));
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const uint32_t next = lds32(at + 32 * h + 4 * i + 4);
-          const uint32_t w = h ? next : __funnelshift_r(prev, next, 16);
+          const uint32_t u = (h ? next : __funnelshift_r(prev, next, 16)) ^ 0x80808080u;
           prev = next;
-          ot[16 * h + 2 * i] = deq8_pair<0x4140>(w & 0x7F7F7F7Fu, w & 0x80808080u, dh, dl);
-          ot[16 * h + 2 * i + 1] = deq8_pair<0x4342>(w & 0x7F7F7F7Fu, w & 0x80808080u, dh, dl);
+          ot[16 * h + 2 * i] = deq8_pair<0x4140>(u, dh, dl);
+          ot[16 * h + 2 * i + 1] = deq8_pair<0x4342>(u, dh, dl);
         }
       }
     }
