@@ -11,9 +11,10 @@
 //         Q4_K, qh[32] fifth bits, qs[128] low nibbles; for 64-value group g: values 0..31 take the low nibbles
 //         of qs[32g..], bit 2g of qh[l] and pair 2g, values 32..63 the high nibbles, bit 2g+1 and pair 2g+1;
 //         y = d * sc * q - dmin * m)
-// with the published GGML arithmetic.  Their matmul: up to four tokens with rows of whole 2048 values on the staged kernels
-// (qgemv_q5k.cu, qgemv_q4_0.cu), more tokens and other rows on the tensor-core kernel with two-piece weights
-// (qgemm_tc2.cu); what neither takes on a plain bandwidth kernel (a warp per weight row, activations staged in shared
+// with the published GGML arithmetic.  Their matmul: one or two tokens with rows of whole 2048 values on the staged kernels
+// (qgemv_q5k.cu, qgemv_q4_0.cu), other rows, up to sixteen tokens and f32 results on the tensor-core kernel of the integers
+// (qgemm_unit.cu), more tokens on the one with two-piece weights (qgemm_tc2.cu); what none of them takes (rows that are
+// not whole 256 values, unaligned pointers) on a plain bandwidth kernel (a warp per weight row, activations staged in shared
 // memory as f32, f32 FMA, fixed reduction order) here.
 #include <type_traits>
 
@@ -32,7 +33,9 @@ template <typename XT>
 int q4_0_gemv_staged(const void* wq, const XT* x, void* y, int M, int N, int K, int y_dtype, bool fresh, cudaStream_t s);
 int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
                   bool fresh, cudaStream_t s);
-bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32);
+int gguf_gemm_unit(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
+                   bool fresh, cudaStream_t s);
+bool unit_takes(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32);
 }
 
 namespace {
@@ -190,15 +193,16 @@ template <typename XT, int FMT>
 int gguf_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int y_dtype, bool fresh, cudaStream_t s) {
   const uint8_t* w = static_cast<const uint8_t*>(wq);
   const size_t esz = y_dtype == UB_DTYPE_F32 ? 4 : 2;
-  // The tensor-core kernel with two-piece weights from the second pass on, and where it pays for rows that the staged kernels
-  // do not take.  Measured on B200, us, four tokens at a time / two-piece for any number up to 16: Q5_K 14336x4096 34.3 / 33,
-  // Q4_0 29.4 / 33.4; one token 4096x5120 Q5_K 32.6 / 19, Q4_0 25 / 18.6.  f32 results: as for Q6_K.
+  // Tensor cores: weights as integers for few tokens and for f32 results (qgemm_unit.cu), two bf16 pieces beyond (qgemm_tc2.cu).
+  // Rows that the staged kernels do not take were never requested ahead of the dependency wait.
   constexpr bool x_f32 = std::is_same<XT, float>::value;
-  if (K % 2048 ? y_dtype != UB_DTYPE_F32 && (M > 4 || ub::two_piece_pays(FMT == 1 ? GGML_Q5_K : GGML_Q4_0, M, N, K, x_f32))
-               : M > 4 && (y_dtype != UB_DTYPE_F32 || K <= 4096)) {
-    // rows that the staged kernels do not take were never requested ahead of the dependency wait
-    const int st = ub::gguf_gemm_tc2(FMT == 1 ? GGML_Q5_K : GGML_Q4_0, y, y_dtype, x, x_f32, wq, M, N, K,
-                                     fresh || K % 2048 != 0, s);
+  constexpr int tag = FMT == 1 ? GGML_Q5_K : GGML_Q4_0;
+  const bool y_f32 = y_dtype == UB_DTYPE_F32;
+  if (ub::unit_takes(tag, M, N, K, x_f32, y_f32)) {
+    const int st = ub::gguf_gemm_unit(tag, y, y_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
+    if (st != UB_ERR_UNSUPPORTED) return st;
+  } else if (M > 4 && (!y_f32 || (K % 2048 == 0 && K <= 4096))) {
+    const int st = ub::gguf_gemm_tc2(tag, y, y_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   for (int m0 = 0; m0 < M;) {

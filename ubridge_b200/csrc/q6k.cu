@@ -27,7 +27,9 @@
 namespace ub {
 int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
                   bool fresh, cudaStream_t s);
-bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32);
+int gguf_gemm_unit(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
+                   bool fresh, cudaStream_t s);
+bool unit_takes(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32);
 }
 
 namespace {
@@ -454,14 +456,16 @@ int q6k_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int ou
   const int grid = (N + 8 * kQ6kRowsPerWarp - 1) / (8 * kQ6kRowsPerWarp);  // the CTA scheduler evens out the load
   const uint8_t* w = static_cast<const uint8_t*>(wq);
   if (ub::take_weights_written(s, wq, static_cast<size_t>(N) * (K / UB_QK_K) * UB_Q6K_BYTES)) fresh = true;
-  // The tensor-core kernel with two-piece weights from the second pass on; rows that the staged kernel does not take from
-  // three tokens on where it pays.  Measured on B200, us, one token at a time / four / two-piece for any number up to 16:
-  // 4096x14336 17.5 / 45 / 37, 4096x5120 14.2 / 19.8 / 17.2.  Its error is below that of the staged kernel (15-bit
-  // activations) but above that of the f32 one, so f32 results leave the latter only where the former had them.
+  // Tensor cores: weights as integers for few tokens and for f32 results (qgemm_unit.cu, f32 rounding only), two bf16 pieces
+  // beyond (qgemm_tc2.cu; its error is below that of the staged kernel, 15-bit activations, but above that of the f32 one, so
+  // f32 results go there only where the former had them).  Rows that the staged kernel does not take were never requested
+  // ahead of the dependency wait.
   constexpr bool x_f32 = std::is_same<XT, float>::value;
-  if (K % 2048 ? M > 2 && out_dtype != UB_DTYPE_F32 && (M > 4 || ub::two_piece_pays(14, M, N, K, x_f32))
-               : M > 4 && (out_dtype != UB_DTYPE_F32 || K <= 4096)) {
-    // rows that the staged kernel does not take were never requested ahead of the dependency wait
+  const bool y_f32 = out_dtype == UB_DTYPE_F32;
+  if (ub::unit_takes(14, M, N, K, x_f32, y_f32)) {
+    const int st = ub::gguf_gemm_unit(14, y, out_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
+    if (st != UB_ERR_UNSUPPORTED) return st;
+  } else if (M > 4 && (!y_f32 || (K % 2048 == 0 && K <= 4096))) {
     const int st = ub::gguf_gemm_tc2(14, y, out_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }

@@ -592,91 +592,6 @@ int by_size(void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int
   return launch2<FMT, 256, 4, 2, false>(y, y_dtype, x, wq, M, N, K, fresh, s);
 }
 
-// ---- up to sixteen tokens: this kernel or the decode kernels (CUDA cores, integer MMA) ----
-// The two-piece launch costs much the same whatever the tokens, and its time falls with the matrix only down to the 6 to 9 us
-// that the barriers, tensor memory and the cluster exchange take; a decode kernel's pass takes one, two, four or eight
-// tokens and scales with the bytes.  Neither line nor constant of one size separates them, so both are priced, in us, by
-// straight lines fitted to 7000 timings on B200 (256 to 14336 values, 512 to 28672 rows, all but a few within 20 %):
-// rounds of CTAs times super-blocks per CTA here, super-blocks and rows there.  Where the decode kernels' time is within
-// 6 % they are taken.  Some crossings: Q6_K four tokens, 2048 rows: 4.2 / 8.0 us at 512 values, 8.3 / 10.8 at 2304, 16.3 /
-// 15.4 at 5120; Q5_K one token, 1024 rows: 6.2 / 8.3 at 1024 values, 27 / 10.9 at 5120; Q8_0 two tokens, 1024 rows: 4.2 /
-// 6.5 at 512, 13.8 / 9.2 at 3072; Q4_K nine tokens f32, 28672x4096: 42 / 76, 1024x4096: 13 / 11.
-struct Pass {  // us: fixed, per super-block of a row, per 1024 rows, per both
-  float fixed, sb, rows, sb_rows;
-  float us(int N, int nsb) const {
-    const float r = static_cast<float>(N) * (1.f / 1024.f);
-    return fixed + sb * nsb + rows * r + sb_rows * nsb * r;
-  }
-};
-constexpr float kNever = 1e9f;  // no decode kernel of this kind takes the pass
-
-// Token passes as the dispatchers cut them.
-float decode_us(int type, int M, int N, int K) {
-  const int nsb = K / UB_QK_K;
-  switch (type) {
-    case 2:   // Q4_0, Q5_K: rows that are not whole 2048 values
-    case 13: {
-      static const Pass q40[3] = {{2.9f, .535f, 0.f, .194f}, {3.06f, .83f, .06f, .22f}, {3.8f, 1.04f, .07f, .33f}};
-      static const Pass q5k[3] = {{2.9f, .62f, 0.f, .256f}, {3.1f, .716f, .1f, .238f}, {3.f, 1.5f, .04f, .326f}};
-      const Pass* p = type == 2 ? q40 : q5k;
-      return M == 1 ? p[0].us(N, nsb) : M == 2 ? p[1].us(N, nsb) : M == 4 ? p[2].us(N, nsb) : kNever;
-    }
-    case 14: {  // Q6_K, the same rows
-      static const Pass p3 = {7.5f, .86f, .22f, .1f}, p4 = {2.4f, .55f, .3f, .1f};
-      return M == 3 ? p3.us(N, nsb) : M == 4 ? p4.us(N, nsb) : kNever;
-    }
-    case 8: {
-      static const Pass rest[2] = {{2.1f, .88f, 0.f, .18f}, {2.45f, .98f, .03f, .34f}};
-      static const Pass lines[4] = {
-          {.98f, .151f, .125f, .031f}, {1.88f, .144f, .08f, .037f}, {1.9f, .186f, .116f, .037f}, {2.45f, .343f, .146f, .049f}};
-      if (K % 2048) return M == 2 ? rest[0].us(N, nsb) : M == 4 ? rest[1].us(N, nsb) : kNever;
-      float t = 0.f;
-      for (int left = M, n; left > 0; left -= n) {
-        n = left < 8 ? left : 8;
-        if ((n > 4 ? 2 : 1) * (K / UB_QK8_0) > 568) return kNever;  // token quads in qgemv_imma.cu's shared memory
-        t += lines[n == 1 ? 0 : n == 2 ? 1 : n <= 4 ? 2 : 3].us(N, nsb);
-      }
-      return t;
-    }
-    case 12: {
-      static const Pass lines[4] = {
-          {1.66f, .109f, .035f, .019f}, {1.25f, .186f, .038f, .02f}, {.74f, .353f, .041f, .03f}, {2.16f, .207f, .151f, .041f}};
-      static const Pass odd[3] = {{2.87f, .031f, .166f, .021f}, {2.46f, .152f, .37f, .001f}, {3.f, .315f, .335f, .014f}};
-      float t = 0.f;
-      for (int left = M, n; left > 0; left -= n) {
-        n = left < 8 ? left : 8;
-        const bool made_for = K == 2048 || K == 4096 || (K == 8192 && n > 4);  // qgemv_mt.cu, qgemv_mc.cu
-        if (!made_for && n > 1 && (n > 4 ? 4 : n > 2 ? 2 : 1) * nsb > 70) return kNever;  // token pairs, qgemv_imma.cu
-        const int c = n == 1 ? 0 : n == 2 ? 1 : n <= 4 ? 2 : 3;
-        if (c < 3) {
-          t += (K % 2048 ? odd[c] : lines[c]).us(N, nsb);
-        } else if (made_for) {
-          t += lines[3].us(N, nsb);
-        } else {  // tiles of 16 rows, four at a time between two reductions
-          const int tiles = ((N + 15) / 16 + ub::num_sms() - 1) / ub::num_sms();
-          t += 1.f + .36f * nsb + .88f * tiles + .065f * tiles * nsb + 2.5f * ((tiles + 3) / 4) + .046f * (n - 5) * nsb;
-        }
-      }
-      return t;
-    }
-    default: return kNever;
-  }
-}
-
-float two_piece_us(int type, int M, int N, int K, bool x_f32) {
-  struct Cost {
-    float fixed, step, step_f32;
-  };
-  const Cost c = type == 2    ? Cost{3.2f, 1.9f, 2.27f}
-                 : type == 13 ? Cost{3.3f, 2.02f, 2.18f}
-                 : type == 14 ? Cost{4.2f, 1.97f, 2.24f}
-                 : type == 8  ? Cost{2.6f, 1.95f, 2.55f}
-                              : Cost{2.4f, 1.77f, 2.2f};
-  const int tiles = (N + 127) / 128, nsb = K / UB_QK_K, ks = k_split(tiles, nsb, 1), sms = ub::num_sms();
-  const int steps = (tiles * ks + sms - 1) / sms * ((nsb + ks - 1) / ks);
-  return c.fixed + (ks > 1 ? 1.3f : 0.f) + (x_f32 ? c.step_f32 : c.step) * steps + .02f * M * (N * (1.f / 1024.f));
-}
-
 }  // namespace
 
 namespace ub {
@@ -692,15 +607,8 @@ int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32
     case 2: return by_size<kQ40>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
     case 13: return by_size<kQ5K>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
     case 14: return by_size<kQ6K>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
-    // Q4_K and Q8_0: few tokens only, beyond them the one-piece kernels are the ones in use
-    case 12: return M <= 64 ? few<kQ4K>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s) : UB_ERR_UNSUPPORTED;
-    case 8: return M <= 64 ? few<kQ8>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s) : UB_ERR_UNSUPPORTED;
     default: return UB_ERR_UNSUPPORTED;
   }
-}
-
-bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32) {
-  return 1.06f * two_piece_us(ggml_type, M, N, K, x_f32) < decode_us(ggml_type, M, N, K);
 }
 
 // y (bf16) = x (bf16) . W^T with weights rounded to bf16 once: the few-token launches of q4k_gemm_tc and q8_0_gemm_tc (fmt:

@@ -4,8 +4,8 @@
 // small-M special cases :502-514) and kernels/matmul.cpp:1197-1208 (LHS-resident decode kernel when it
 // fits, batched kernel otherwise).  The same idea here is a split on M:
 //   M = 1             one-token decode kernels (qgemv_m1.cu, qgemv_q8_m1.cu), any whole super-blocks per row;
-//   M <= 16           integer decode kernels in passes of up to eight tokens (qgemv.cu), or the tensor-core kernel with
-//                     two-piece weights in one pass (qgemm_tc2.cu; the line: two_piece_is_faster); from M = 9 on Q4_K with
+//   M <= 16           integer decode kernels in passes of up to eight tokens (qgemv.cu), or the tensor-core kernel of the
+//                     weights' integers in one pass (qgemm_unit.cu; the line: unit_pays); from M = 9 on Q4_K with
 //                     bf16 activations AND bf16 output takes the one-piece tensor-core kernels.  No workspace;
 //   M  > 16, Q4_K     tcgen05 tensor-core GEMM with in-kernel dequantisation, one piece (qgemm_tc2.cu while one round of CTAs
 //                     holds all 128-token tiles, qgemm_tc.cu beyond; bf16 activations and output, other types are
@@ -36,9 +36,9 @@ int q4k_gemm_mma(void* y, const void* x, const void* wq, int M, int N, int K, cu
 uint32_t oneshot_spin_limit();
 void* tensor_map_encoder();
 int q4k_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
-int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
-                  bool fresh, cudaStream_t s);
-bool two_piece_pays(int ggml_type, int M, int N, int K, bool x_f32);
+int gguf_gemm_unit(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
+                   bool fresh, cudaStream_t s);
+bool unit_pays(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32);
 int q8_0_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
 }  // namespace ub
 
@@ -219,28 +219,6 @@ __global__ void add_bf16_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Two to sixteen tokens: the tensor-core kernel with two-piece weights (one pass for all of them) or the decode kernels
-// (passes of up to eight).  Where the decode kernels run in one pass on rows they are made for they are the faster ones:
-// measured on B200, us, decode / two-piece, Q4_K four tokens 4096x4096 7.4 / 12, 27648x5120 33.6 / 75, 57344x8192 72 / 230, but
-// 4096x14336 135 / 30.6 and eight tokens 15360x5120 75 / 42; Q8_0 four tokens 6144x4096 9.2 / 20.5, four 6144x5120 76 / 25.
-// Where they need a second pass or fall back to the CUDA-core kernels, both are priced (two_piece_pays).
-// Error of f32 results (2-norm, f64): integer kernels, 15 bits of an activation, 2.8e-5; two pieces 2e-6 to 5e-6 with bf16
-// activations, 4e-6 to 1.2e-5 with f32 ones; CUDA-core kernels 1e-7 to 3e-6 (Q4_K while a row's activations fit its
-// shared memory 2e-5): where those run, f32 results stay with them.
-bool two_piece_is_faster(bool is_q4k, int M, int N, int K, bool x_f32, int out_dtype) {
-  const int pass = M < kDecodeOnePassM ? M : kDecodeOnePassM, nsb = K / UB_QK_K;
-  if (!is_q4k) {
-    const bool quads_fit = K % 2048 == 0 && (pass + 3) / 4 * (K / UB_QK8_0) <= 568;  // in qgemv_imma.cu's shared memory
-    if (quads_fit ? M <= kDecodeOnePassM : out_dtype == UB_DTYPE_F32 || K % UB_QK_K != 0) return false;
-  } else {
-    const bool made_for = K == 2048 || K == 4096 || (K == 8192 && M > 4);  // qgemv_mt.cu, qgemv_mc.cu
-    const bool pairs_fit = (pass + 1) / 2 * nsb <= 70;  // token pairs of a whole row in qgemv_imma.cu's shared memory
-    if (out_dtype == UB_DTYPE_F32 && !made_for && !pairs_fit) return false;
-    if (M <= kDecodeOnePassM && (made_for || (M <= 4 && pairs_fit))) return false;
-  }
-  return ub::two_piece_pays(is_q4k ? 12 : 8, M, N, K, x_f32);
-}
-
 inline size_t weight_bytes(bool is_q4k, int N, int K) {
   return is_q4k ? static_cast<size_t>(N) * (K / UB_QK_K) * UB_Q4K_BYTES
                 : static_cast<size_t>(N) * (K / UB_QK8_0) * UB_Q8_0_BYTES;
@@ -275,8 +253,14 @@ int qmatmul(bool is_q4k, int x_dtype, void* y, const void* x, const void* wq, in
     const int st = ub::q4k_gemm_tc(y, x, wq, M, N, K, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;  // unsupported shape or driver: the decode kernel below
   }
-  if (M >= 2 && M <= kDecodeMaxM && two_piece_is_faster(is_q4k, M, N, K, x_dtype == UB_DTYPE_F32, out_dtype)) {
-    const int st = ub::gguf_gemm_tc2(is_q4k ? 12 : 8, y, out_dtype, x, x_dtype == UB_DTYPE_F32, wq, M, N, K, fresh, s);
+  // Up to sixteen tokens: the tensor-core kernel of the integers (one pass for all of them, f32 rounding only: 1e-7 of a result,
+  // 2-norm) or the decode kernels (passes of up to eight; integer ones 2.8e-5, CUDA-core ones 1e-7 to 3e-5), whichever is the
+  // faster one.  One token of Q4_K, and of Q8_0 with rows of whole 2048 values, has kernels of its own.
+  if (M <= kDecodeMaxM && (M >= 2 || (!is_q4k && K % 2048 != 0)) && K % UB_QK_K == 0 &&
+      ub::unit_pays(is_q4k ? 12 : 8, M, N, K, x_dtype == UB_DTYPE_F32, out_dtype == UB_DTYPE_F32)) {
+    // what ran on CUDA cores before was never requested ahead of the dependency wait
+    const bool late = K % 2048 != 0 && (M == 1 || out_dtype == UB_DTYPE_F32);
+    const int st = ub::gguf_gemm_unit(is_q4k ? 12 : 8, y, out_dtype, x, x_dtype == UB_DTYPE_F32, wq, M, N, K, fresh || late, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   auto decode = [&]() {
