@@ -31,9 +31,12 @@
 //                 nibbles into the bf16 q * 2^-133 with one byte permute per pair, times d*sc minus dmin*m with
 //                 packed bf16 FMAs (rowblock.cuh); tcgen05.st; the stage is handed over (tcgen05.wait::st, mbarrier
 //                 arrive) after the next one's arithmetic
-//   warp 13       one lane issues all bulk copies: packed weight tiles ([128 rows][144 bytes], one 2-D
-//                 tensor-map copy per super-block column, two super-blocks ahead) and token tiles (one
-//                 copy per K step, as far ahead as the ring allows)
+//   warp 13       one lane copies packed weight tiles ([128 rows][144 bytes], one 2-D tensor-map copy per super-block column)
+//   warp 14       one lane copies token tiles (one copy per stage of 64 values)
+//   Both as far ahead as their rings allow.  One thread for both took 650 cycles for a stage (a wait of 200 per barrier, 50 per
+//   copy) and was what the grouped launches waited for.  With a thread for each, stages of the longest run's size instead of 128
+//   tokens, runs that end with their last live token and looks at barriers one stage ahead, the expert layer of 256 tokens
+//   (8 experts top-2, 4096 / 14336) takes 340 us instead of 399 (weights in one bf16 piece as in rowblock.cuh on both sides).
 //
 // Every mbarrier wait is bounded; on expiry the CTA sets a shared abort flag, records UB_ERR_TIMEOUT in
 // the device error word, all roles leave their loops, and TMEM is freed before the kernel returns.
@@ -48,7 +51,7 @@ namespace {
 using namespace ub;
 
 constexpr int kTcProducerWarps = 8;   // warps that dequantise a weight stage (128 rows x two 64-value groups)
-constexpr int kTcThreads = (5 + kTcProducerWarps + 1) * 32;
+constexpr int kTcThreads = (5 + kTcProducerWarps + 2) * 32;
 constexpr int kTcBK = 64;
 
 constexpr int kTcMaxStages = 8, kTcMaxAStages = 4;
@@ -85,6 +88,12 @@ struct TcGroup {
   int rows_per_expert;          // weight rows per expert in the packed tensor (2 I for mode 1, N for mode 2)
 };
 
+// Token tiles of one launch: dense, m[0] is the whole tile; grouped, m[i] is 32 (i + 1) tokens, so that a run of any length comes
+// by one copy per stage (the copying thread issues some 50 cycles apart and waits 200 for each barrier).
+struct TcXMaps {
+  CUtensorMap m[4];
+};
+
 struct TcRun {
   int e, m0, len;
 };
@@ -96,7 +105,7 @@ struct TcShared {
   unsigned long long wfull[kTcWStages], wempty[kTcWStages];
   uint32_t tmem_base;
   int abort_flag;
-  int nruns;
+  int nruns, longest;
 };
 
 // TOK: tokens per tile (UMMA N): 64, 128 or 256.  STAGES: ring depth (token tiles in shared memory and
@@ -114,14 +123,17 @@ struct TcShared {
 template <int TOK, int STAGES, int MODE, int CTAS, int WST, int FMT, int AST>
 __global__ void __launch_bounds__(kTcThreads, CTAS)
 qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err_word,
-                    const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
+                    const __grid_constant__ TcXMaps x_maps, const __grid_constant__ CUtensorMap w_map,
                     const TcGroup grp) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   __shared__ TcShared sh;
   __shared__ TcRun runs[MODE == 0 ? 1 : kTcMaxRuns];
   __shared__ float run_w[MODE == 2 ? TOK : 1];
   __shared__ int run_dst[MODE == 2 ? TOK : 1];
-  static_assert(STAGES <= kTcMaxStages, "barrier arrays");
+  // Looks at the next stage's barriers ahead of this one's work: the answer takes 200 cycles.  Grouped launches gain (below), with
+  // 256 tokens of one tile nobody waits for it (2048 tokens 14336x4096 208 / 211 us).
+  constexpr bool kLook = MODE != 0;
+  static_assert(STAGES <= kTcMaxStages && (MODE == 0 || TOK <= 256), "barrier arrays");
   constexpr uint32_t kBBytes = TOK * 128;              // TOK token rows x 64 bf16
   constexpr int kStageTok = tc_stage_tok(TOK, CTAS);   // tokens the output staging tile holds
   constexpr int kWStages = tc_wstages(TOK, CTAS, WST);
@@ -181,10 +193,26 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
           n++;
         }
       }
-      sh.nruns = n;
+      sh.nruns = n, sh.longest = 1;
+    }
+    __syncthreads();
+    // A run ends with its last live token, not with its last alignment block: what pads the block is neither read nor multiplied.
+    for (int r = warp; r < sh.nruns; r += kTcThreads / 32) {
+      int last = 0;
+      for (int i = lane; i < runs[r].len; i += 32) {
+        const int sid = grp.sorted_ids[runs[r].m0 + i];
+        if (sid >= 0 && sid < grp.num_valid) last = i + 1;
+      }
+      last = __reduce_max_sync(0xFFFFFFFFu, last);
+      if (lane == 0) runs[r].len = max(last, 1), atomicMax(&sh.longest, last);
     }
     __syncthreads();
   }
+  // Token stages are as large as the longest run needs, and as many as fit: how far the copies run ahead is what a step of such a
+  // launch waits for.
+  constexpr bool kFit = MODE != 0 && TOK <= 128;
+  const uint32_t x_stride = kFit ? static_cast<uint32_t>((sh.longest + 31) & ~31) * 128 : kBBytes;
+  const int nst = kFit ? min(kTcMaxStages, static_cast<int>(STAGES * kBBytes / x_stride)) : STAGES;
   const int ntiles = MODE == 0 ? w_tiles * t_tiles : sh.nruns * w_tiles;
   // tile -> (first token row of A, valid tokens, first weight row in the packed tensor, first output column)
   auto tile_info = [&](int tile, int& m0, int& valid, int& wrow0, int& n0) {
@@ -199,7 +227,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) {
+    for (int s = 0; s < kTcMaxStages; s++) {
       tc_mbar_init(full_bar(s), 1);
       tc_mbar_init(empty_bar(s), 1);
     }
@@ -234,7 +262,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
       int s = 0, as = 0;
       uint32_t phase = 0, aphase = 0, acc_phase = 0;
       int buf = 0;
-      bool ok = true;
+      bool ok = true, a_ready = false, x_ready = false;
       for (int tile = vblock; tile < ntiles && ok; tile += vgrid) {
         int m0_, valid, wrow0_, n0_;
         tile_info(tile, m0_, valid, wrow0_, n0_);
@@ -247,29 +275,30 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf) * kAccStride;
         for (int ks = 0; ks < ksteps; ks++) {
-          ok = tc_wait(afull_bar(as), aphase, abort_flag);
+          if (!a_ready) ok = tc_wait(afull_bar(as), aphase, abort_flag);
           const uint32_t a_tmem = tmem_base + kATmemCol + 64u * as;
+          const int as_next = as + 1 == AST ? 0 : as + 1;
+          const uint32_t aphase_next = as_next ? aphase : aphase ^ 1;
 #pragma unroll
           for (int g = 0; g < 2; g++) {
-            if (ok) ok = tc_wait(full_bar(s), phase, abort_flag);
+            if (ok && !x_ready) ok = tc_wait(full_bar(s), phase, abort_flag);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t b_desc = make_sw128_desc(smem_base + s * kBBytes);
+            // looks at the next stages, ahead of this one's MMAs
+            const int s_next = s + 1 == nst ? 0 : s + 1;
+            const uint32_t phase_next = s_next ? phase : phase ^ 1;
+            x_ready = kLook && tc_mbar_test(full_bar(s_next), phase_next);
+            if (kLook && g == 1) a_ready = tc_mbar_test(afull_bar(as_next), aphase_next);
+            const uint64_t b_desc = make_sw128_desc(smem_base + s * x_stride);
 #pragma unroll
             for (int j = 0; j < 4; j++)  // K = 16 per instruction: 8 TMEM columns of A, 32 bytes of a B row
               umma_bf16_ts(d_tmem, a_tmem + 32u * g + 8u * j, b_desc + 2 * j, idesc, (ks > 0 || g > 0 || j > 0) ? 1u : 0u);
             umma_commit(empty_bar(s));  // stage is free once these MMAs have read it
-            if (++s == STAGES) {
-              s = 0;
-              phase ^= 1;
-            }
+            s = s_next, phase = phase_next;
           }
           if (!ok) break;
           umma_commit(aempty_bar(as));
-          if (++as == AST) {
-            as = 0;
-            aphase ^= 1;
-          }
+          as = as_next, aphase = aphase_next;
         }
         if (!ok) break;
         umma_commit(tfull_bar(buf));  // accumulator complete
@@ -449,24 +478,22 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
     }
     hand_over();
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-  } else {
-    // ------------------------------------------------------------ bulk copies (one lane)
-    // Packed weight tiles run kWStages - 1 super-blocks ahead of the token tiles; token tiles run as far
-    // ahead of the MMA as the ring allows.
+  } else if (warp == 5 + kTcProducerWarps) {
+    // ------------------------------------------------------------ bulk copies of packed weights (one lane), as far ahead as
+    // their ring allows
     if (elect_one()) {
       const int nsb = K >> 8;
       const int my_tiles = vblock < ntiles ? (ntiles - vblock + vgrid - 1) / vgrid : 0;
       const int total_sb = my_tiles * nsb;
-      int s = 0, ws = 0;
-      uint32_t phase = 0, wphase = 0;
+      int ws = 0;
+      uint32_t wphase = 0;
       bool ok = true;
-      int wq_next = 0;  // next super-block (flat index) whose packed weights have not been requested
-      auto issue_w = [&]() {
-        const int ti = wq_next / nsb, sb = wq_next - ti * nsb;
+      for (int q = 0; q < total_sb && ok; q++) {
+        const int ti = q / nsb, sb = q - ti * nsb;
         int m0_, valid_, wrow0, n0_;
         tile_info(vblock + ti * vgrid, m0_, valid_, wrow0, n0_);
         ok = tc_wait(wempty_bar(ws), wphase ^ 1, abort_flag);
-        if (!ok) return;
+        if (!ok) break;
         const uint32_t bar = wfull_bar(ws);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTcWBytes) : "memory");
         asm volatile(
@@ -480,37 +507,55 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
                   "r"(smem_base + kWOff + ws * kTcWBytes + kTcWBytes / 2),
               "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(bar), "r"(sb * kWRow), "r"(wrow0 + N)
               : "memory");
-        wq_next++;
         if (++ws == kWStages) {
           ws = 0;
           wphase ^= 1;
         }
-      };
-      for (int i = 0; i < kWStages - 1 && wq_next < total_sb && ok; i++) issue_w();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ bulk copies of token tiles (one lane), as far ahead of the
+    // MMAs as their ring allows
+    if (elect_one()) {
+      const int nsb = K >> 8;
+      const int my_tiles = vblock < ntiles ? (ntiles - vblock + vgrid - 1) / vgrid : 0;
+      const int total_sb = my_tiles * nsb;
+      int s = 0;
+      uint32_t phase = 0;
+      bool ok = true, x_ready = false;
       for (int q = 0; q < total_sb && ok; q++) {
-        if (wq_next < total_sb) issue_w();
-        if (!ok) break;
         const int ti = q / nsb, sb = q - ti * nsb;
         int m0, valid, wrow0_, n0_;
         tile_info(vblock + ti * vgrid, m0, valid, wrow0_, n0_);
-        const int boxes = MODE == 0 ? 1 : (valid + 63) >> 6;  // grouped modes: boxes of 64 tokens, no more than the run has
+        const int box = MODE == 0 ? 0 : (valid - 1) >> 5;  // which map: no more tokens than the run has, in steps of 32
+        const CUtensorMap* const x_map = &x_maps.m[TOK > 128 && MODE != 0 ? 3 : box];
         for (int G = 0; G < 4; G++) {
-          ok = tc_wait(empty_bar(s), phase ^ 1, abort_flag);
+          if (!x_ready) ok = tc_wait(empty_bar(s), phase ^ 1, abort_flag);
           if (!ok) break;
+          const int s_next = s + 1 == nst ? 0 : s + 1;
+          const uint32_t phase_next = s_next ? phase : phase ^ 1;
+          x_ready = kLook && tc_mbar_test(empty_bar(s_next), phase_next ^ 1);
           const uint32_t bar = full_bar(s);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                       "r"(MODE == 0 ? kBBytes : static_cast<uint32_t>(boxes * 64 * 128))
-                       : "memory");
-          for (int b = 0; b < boxes; b++)
+          if (MODE != 0 && TOK > 128) {  // two boxes of 128 tokens at most
+            const int boxes = (valid + 127) >> 7;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(boxes * 128 * 128) : "memory");
+            for (int b = 0; b < boxes; b++)
+              asm volatile(
+                  "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
+                      "r"(smem_base + s * kBBytes + b * (128 * 128)),
+                  "l"(reinterpret_cast<uint64_t>(x_map)), "r"(bar), "r"((sb * 4 + G) * kTcBK), "r"(m0 + 128 * b)
+                  : "memory");
+          } else {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                         "r"(MODE == 0 ? kBBytes : static_cast<uint32_t>((box + 1) * 32 * 128))
+                         : "memory");
             asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
-                    "r"(smem_base + s * kBBytes + b * (64 * 128)),
-                "l"(reinterpret_cast<uint64_t>(&x_map)), "r"(bar), "r"((sb * 4 + G) * kTcBK), "r"(m0 + 64 * b)
+                    "r"(smem_base + s * x_stride),
+                "l"(reinterpret_cast<uint64_t>(x_map)), "r"(bar), "r"((sb * 4 + G) * kTcBK), "r"(m0)
                 : "memory");
-          if (++s == STAGES) {
-            s = 0;
-            phase ^= 1;
           }
+          s = s_next, phase = phase_next;
         }
       }
     }
@@ -557,17 +602,20 @@ int launch_tc(void* y, const void* x, const void* wq, int M, int N, int K, const
   }
   // token matrix as a 2-D tensor map: inner dimension K (bf16), outer M; box = 64 x TOK, 128-byte swizzle;
   // rows beyond M read as zeros
-  CUtensorMap map;
+  TcXMaps maps;
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return ub::fail(UB_ERR_UNSUPPORTED);
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(M)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(MODE == 0 ? TOK : 64)};
   const cuuint32_t estr[2] = {1, 1};
-  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return ub::fail(UB_ERR_UNSUPPORTED);
+  memset(&maps, 0, sizeof(maps));
+  for (int i = 0; i < (MODE == 0 ? 1 : 4); i++) {
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(MODE == 0 ? TOK : 32 * (i + 1))};
+    if (enc(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return ub::fail(UB_ERR_UNSUPPORTED);
+  }
   // packed weights as a 2-D byte tensor: inner dimension = one row's bytes, outer = all weight rows (of all
   // experts); box = one super-block (144 bytes) of 128 rows (64 for the gate/up halves of mode 1), no
   // swizzle; rows beyond the tensor read as zeros.  Q8_0: a box of eight blocks is 272 bytes, wider than the
@@ -589,10 +637,11 @@ int launch_tc(void* y, const void* x, const void* wq, int M, int N, int K, const
     return ub::fail(UB_ERR_CUDA);
   }
   return ub::launch_pdl_smem(kernel, dim3(grid), dim3(kTcThreads), smem, s, static_cast<__nv_bfloat16*>(y), M, N, K,
-                             ub::device_error_word(), map, wmap, grp);
+                             ub::device_error_word(), maps, wmap, grp);
 }
 
-// xg[i, :] = hidden[sorted_ids[i] / top_k, :] for the positions the alignment produced (zeros for padding)
+// xg[i, :] = hidden[sorted_ids[i] / top_k, :] for the positions the alignment produced (padding is left as it is: the GEMMs
+// store nothing of it)
 __global__ void __launch_bounds__(256) moe_gather_rows_kernel(__nv_bfloat16* __restrict__ xg,
                                                               const __nv_bfloat16* __restrict__ hidden,
                                                               const int32_t* __restrict__ sorted_ids,
@@ -603,10 +652,10 @@ __global__ void __launch_bounds__(256) moe_gather_rows_kernel(__nv_bfloat16* __r
   pdl_open();
   if (i >= *num_post_pad) return;
   const int sid = sorted_ids[i];
-  const bool live = sid >= 0 && sid < num_valid;
-  const uint4* src = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(live ? sid / top_k : 0) * H);
+  if (sid < 0 || sid >= num_valid) return;
+  const uint4* src = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(sid / top_k) * H);
   uint4* dst = reinterpret_cast<uint4*>(xg + static_cast<size_t>(i) * H);
-  for (int c = threadIdx.x; c < H / 8; c += blockDim.x) dst[c] = live ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+  for (int c = threadIdx.x; c < H / 8; c += blockDim.x) dst[c] = __ldg(src + c);
 }
 
 }  // namespace
