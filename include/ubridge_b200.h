@@ -155,8 +155,8 @@ int ub_repack_to_interleaved(void* interleaved, const void* split, size_t nblock
  * output and embedding matrices in it.  Blocks are interleaved as in a .gguf file, 2-byte aligned.
  * ub_dequant_q6k: the f32 value (d*scale)*(q-32) rounded once to out_dtype, bit-exact.
  * ub_qmatmul_q6k_*: y[M,N] = x[M,K] . W^T with W = N rows of K/256 blocks, f32 accumulation, a
- * weight-streaming decode kernel that takes the tokens four at a time (any M, no workspace), or, from three tokens on where
- * it is the faster one and as exact, a tensor-core kernel that takes them all.  With K a multiple of 2048 (up to 14336 for
+ * weight-streaming decode kernel that takes the tokens four at a time (any M, no workspace), or, from two tokens on (and for one
+ * in rows that are not whole 2048 values) where they are the faster ones and as exact, tensor-core kernels that take them all.  With K a multiple of 2048 (up to 14336 for
  * one token) and 16-byte aligned wq these kernels request their first weights before they wait for the kernel in front of
  * them on the stream: the precondition on the weights and UB_QMATMUL_WEIGHTS_FRESH (below, ORed into out_dtype) apply to
  * them as to ub_qmatmul_*. */
@@ -171,7 +171,7 @@ int ub_qmatmul_q6k_bf16(void* y, const void* x, const void* wq, int M, int N, in
  * matmul_* (kernels/matmul.cpp:1143-1184; small-M shape in
  * kernels/third_party/matmul_decoding.h:12-570).  The suffix names the activation type;
  * out_dtype is UB_DTYPE_F32 / UB_DTYPE_BF16 / UB_DTYPE_F16.  M <= 16 runs the
- * bandwidth-bound decode kernels or, where they would need a second pass, a tensor-core kernel of their
+ * bandwidth-bound decode kernels or, where it is the faster one, a tensor-core kernel of at least their
  * precision (Q4_K with bf16 activations and bf16 output: M <= 8), larger M
  * the tensor-core kernels — see ub_qmatmul_workspace_bytes for the scratch it needs when the
  * activation or output type is not bf16 (0 whenever M <= 16).  Q8_0 takes the tensor-core kernel when
@@ -230,8 +230,8 @@ int ub_qmatmul_q4k_f32_static(void* y, const void* x, const void* wq, int M, int
  * (kernels/quant.cpp:64-185) and ships kernels for Q8_0 and Q4_K; taken here: Q4_0 (2), Q8_0 (8), Q4_K (12),
  * Q5_K (13), Q6_K (14); other tags return UB_ERR_UNSUPPORTED.  x_dtype f32 / bf16; Q4_K with more than 16 tokens
  * and non-bf16 types needs ub_qmatmul_gguf_workspace_bytes of workspace, the other formats none.  Q4_0, Q5_K and
- * Q6_K with rows of whole 2048 values and 16-byte aligned blob and activations run kernels (up to four tokens: whole
- * rows staged by bulk copies; more: tensor cores) that request their first weights before they wait for the kernel in
+ * Q6_K with rows of whole 2048 values and 16-byte aligned blob and activations run kernels (few tokens: whole
+ * rows staged by bulk copies; else: tensor cores) that request their first weights before they wait for the kernel in
  * front of them on the stream: the precondition on the weights and UB_QMATMUL_WEIGHTS_FRESH (ORed into out_dtype)
  * apply to them as to ub_qmatmul_*. */
 int ub_gguf_block_values(int ggml_type);
