@@ -386,6 +386,16 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
     const int row = threadIdx.x - 256, wrow = tile_row(FMT, row);
     const uint32_t d_lane = tmem_base + (static_cast<uint32_t>(32 * (warp & 3)) << 16);
     const uint32_t ring = smem_base + kWOff + row * kPitch;
+    auto agree = [&](bool mine_ok) {  // the four warps take the same decision: nobody is left alone at a named barrier
+      uint32_t all_ok;
+      asm volatile(
+          "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, 128, q;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(all_ok)
+          : "r"(mine_ok ? 1u : 0u)
+          : "memory");
+      return all_ok != 0;
+    };
     int s = 0, ws = 0, xs = 0;
     uint32_t phase = 0, wphase = 0, xphase = 0;
     for (int tile = vblock; tile < ntiles && ok; tile += vgrid) {
@@ -488,6 +498,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
         if (++ws == WST) ws = 0, wphase ^= 1;
         if (FMT == kQ6K) skew = (skew + 210) & 15u;
       }
+      if (KS > 1) ok = agree(ok);  // a warp may have given up on its own; all four come here, once: one tile per CTA
       if (!ok) break;
       if (KS == 1) {
         if (n0 + wrow < N) {
@@ -517,14 +528,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
           *reinterpret_cast<float4*>(tiles + (at - smem_base) + q * own * 16) =
               make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
       }
-      uint32_t all_ok, my_ok = tc_wait_cluster(pfull, 0, abort_flag) ? 1u : 0u;
-      asm volatile(
-          "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, 128, q;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(all_ok)
-          : "r"(my_ok)
-          : "memory");
-      ok = all_ok != 0;
+      ok = agree(tc_wait_cluster(pfull, 0, abort_flag));
       if (!ok) break;
       for (int i = row; i < mine * (TT / 4); i += 128) {
         const int q = i / mine, l = i - q * mine, out = n0 + tile_row(FMT, first + l);
