@@ -199,7 +199,7 @@ int gguf_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int y
   constexpr int tag = FMT == 1 ? GGML_Q5_K : GGML_Q4_0;
   const bool y_f32 = y_dtype == UB_DTYPE_F32;
   if (ub::unit_takes(tag, M, N, K, x_f32, y_f32)) {
-    const int st = ub::gguf_gemm_unit(tag, y, y_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
+    const int st = ub::gguf_gemm_unit(tag, y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   } else if (M > 4 && (!y_f32 || (K % 2048 == 0 && K <= 4096))) {
     const int st = ub::gguf_gemm_tc2(tag, y, y_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);

@@ -400,6 +400,13 @@ qgemv_q6k_m1_kernel(const uint8_t* __restrict__ wq, const XT* __restrict__ x, vo
   if (!ok && lane == 0) report_device_error(err_word, UB_ERR_TIMEOUT);
 }
 
+// Bytes of a stage of weight rows and of MT tokens' limbs; a plan has at least two stages.
+inline size_t plan_stage_bytes(int K) { return kQ6W * static_cast<size_t>(K / UB_QK_K) * UB_Q6K_BYTES; }
+inline size_t plan_x_bytes(int MT, int K) {
+  return MT * (static_cast<size_t>(K / 16) * 32 + static_cast<size_t>(K / UB_QK_K) * 4);
+}
+inline bool plan_fits(int MT, int K) { return plan_x_bytes(MT, K) + 2 * plan_stage_bytes(K) <= kQ6DynBudgetOne; }
+
 // One to four tokens, K a multiple of 2048 (rows are then whole 16-byte pieces) while two stages fit beside the
 // tokens' limbs (one token: up to 14336), 16-byte aligned weights; UB_ERR_UNSUPPORTED for everything else.  Two CTAs per SM while two stages of eight rows fit beside the activation
 // limbs in half an SM's shared memory (K <= 4096), one CTA per SM with the whole of it beyond.
@@ -407,8 +414,7 @@ template <typename XT, int MT>
 int launch_q6k_m1(const uint8_t* w, const XT* x, void* y, int M, int N, int K, int out_dtype, bool fresh,
                   cudaStream_t s) {
   if (K % 2048 || (reinterpret_cast<uintptr_t>(w) & 15)) return UB_ERR_UNSUPPORTED;
-  const size_t row_bytes = static_cast<size_t>(K / UB_QK_K) * UB_Q6K_BYTES, stage_bytes = kQ6W * row_bytes;
-  const size_t xbytes = MT * (static_cast<size_t>(K / 16) * 32 + static_cast<size_t>(K / UB_QK_K) * 4);
+  const size_t stage_bytes = plan_stage_bytes(K), xbytes = plan_x_bytes(MT, K);
   int ctas = 2;
   int S = xbytes + 2 * stage_bytes <= kQ6DynBudget ? static_cast<int>((kQ6DynBudget - xbytes) / stage_bytes) : 0;
   if (S < 2) {
@@ -463,7 +469,7 @@ int q6k_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int ou
   constexpr bool x_f32 = std::is_same<XT, float>::value;
   const bool y_f32 = out_dtype == UB_DTYPE_F32;
   if (ub::unit_takes(14, M, N, K, x_f32, y_f32)) {
-    const int st = ub::gguf_gemm_unit(14, y, out_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
+    const int st = ub::gguf_gemm_unit(14, y, out_dtype, x, x_f32, wq, M, N, K, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   } else if (M > 4 && (!y_f32 || (K % 2048 == 0 && K <= 4096))) {
     const int st = ub::gguf_gemm_tc2(14, y, out_dtype, x, x_f32, wq, M, N, K, fresh || K % 2048 != 0, s);
@@ -499,6 +505,13 @@ int q6k_matmul(void* y, const XT* x, const void* wq, int M, int N, int K, int ou
 }
 
 }  // namespace
+
+namespace ub {
+
+// Does the staged kernel take M tokens of such rows (aligned ones)?
+bool q6k_staged_takes(int M, int K) { return K % 2048 == 0 && plan_fits(M > 2 ? 4 : M, K); }
+
+}  // namespace ub
 
 extern "C" {
 

@@ -41,6 +41,11 @@
 
 namespace ub {
 void* tensor_map_encoder();
+bool q4_0_staged_takes(int M, int K);
+bool q5k_staged_takes(int M, int K);
+bool q6k_staged_takes(int M, int K);
+bool q4k_imma_takes(int M, int K);
+bool q8_0_imma_takes(int M, int K);
 }
 
 namespace {
@@ -983,6 +988,23 @@ bool unit_takes(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32) {
   }
 }
 
+// May a launch request weights ahead of its dependency wait?  Only where every kernel that could have the call does: a caller
+// that writes weights with the kernel in front of a call which the plain launches take (CUDA-core kernels) needs no flag, and
+// keeps its order here.  The decode kernels' first pass decides; where they do not take it, 16-bit results of Q4_K, Q8_0 and, from
+// five tokens on, of the other formats were always requested ahead, except few tokens of Q8_0 rows that are not whole 2048
+// values, which either kind took.
+bool unit_early(int ggml_type, int M, int K, bool y_f32) {
+  const bool odd = K % 2048 != 0;
+  const int pass = ggml_type == 8 || ggml_type == 12 ? (M < 8 ? M : 8) : M < 4 ? M : 4;
+  switch (ggml_type) {
+    case 8: return q8_0_imma_takes(pass, K) || (!y_f32 && !(odd && (M <= 2 || M == 4)));
+    case 12: return K == 2048 || K == 4096 || (K == 8192 && M > 4) || q4k_imma_takes(pass, K) || !y_f32;
+    case 2: return !odd && (q4_0_staged_takes(pass, K) || (M > 4 && !y_f32));
+    case 13: return !odd && (q5k_staged_takes(pass, K) || (M > 4 && !y_f32));
+    default: return !odd && (q6k_staged_takes(pass, K) || (M > 4 && !y_f32));
+  }
+}
+
 // K % 256 == 0, x and wq 16-byte aligned; UB_ERR_UNSUPPORTED (nothing launched, nothing recorded) for the rest and for
 // formats and drivers it does not take.
 int gguf_gemm_unit(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
@@ -990,6 +1012,7 @@ int gguf_gemm_unit(int ggml_type, void* y, int y_dtype, const void* x, bool x_f3
   if (M <= 0 || N <= 0 || K <= 0 || K % UB_QK_K || (reinterpret_cast<uintptr_t>(wq) & 15) ||
       (reinterpret_cast<uintptr_t>(x) & 15))
     return UB_ERR_UNSUPPORTED;
+  if (!unit_early(ggml_type, M, K, y_dtype == UB_DTYPE_F32)) fresh = true;
   switch (ggml_type) {
     case 2: return by_type<kQ40>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
     case 8: return by_type<kQ8>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);

@@ -495,6 +495,15 @@ qgemv_q4k_imma_kernel(const uint8_t* __restrict__ wq, const XT* __restrict__ x, 
   if (!ok && lane == 0) report_device_error(err_word, UB_ERR_TIMEOUT);
 }
 
+// The shared-memory plan of MP token pairs: the fragments, two stages at least, and a ring that takes the partial sums.
+inline size_t imma_fixed(int MP, int nsb) { return static_cast<size_t>(MP) * nsb * (2048 + 64); }
+inline int imma_stages(int MP, const ImmaGeom& geo) {
+  const size_t fixed = imma_fixed(MP, geo.nsb), stage = geo.stage_bytes;
+  if (fixed + 2 * stage > kSmemBudget) return 0;
+  const int S = static_cast<int>((kSmemBudget - fixed) / stage), s = S < kMaxStages ? S : kMaxStages;
+  return s * stage < static_cast<size_t>(kCW) * imma_mt(MP) * MP * 32 * sizeof(float) ? 0 : s;
+}
+
 template <typename XT, int MP>
 int launch_imma(const uint8_t* wq, const XT* x, void* y, int M, int N, int K, int y_dtype, bool fresh, const ArParams& ar,
                 cudaStream_t s) {
@@ -518,12 +527,9 @@ int launch_imma(const uint8_t* wq, const XT* x, void* y, int M, int N, int K, in
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
   const ImmaGeom geo = imma_geom(K, use_tm);
-  const size_t fixed = static_cast<size_t>(MP) * geo.nsb * (2048 + 64);
-  if (fixed + 2 * static_cast<size_t>(geo.stage_bytes) > kSmemBudget) return UB_ERR_UNSUPPORTED;
-  int S = static_cast<int>((kSmemBudget - fixed) / geo.stage_bytes);
-  if (S > kMaxStages) S = kMaxStages;
-  const size_t red_bytes = static_cast<size_t>(kCW) * imma_mt(MP) * MP * 32 * sizeof(float);
-  if (static_cast<size_t>(S) * geo.stage_bytes < red_bytes) return UB_ERR_UNSUPPORTED;
+  const int S = imma_stages(MP, geo);
+  if (!S) return UB_ERR_UNSUPPORTED;
+  const size_t fixed = imma_fixed(MP, geo.nsb);
   const size_t smem = static_cast<size_t>(S) * geo.stage_bytes + fixed + 1024;
   auto kernel = qgemv_q4k_imma_kernel<XT, MP>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -777,21 +783,25 @@ qgemv_q8_0_imma_kernel(const XT* __restrict__ x, void* __restrict__ y, int M, in
   if (!ok && lane == 0) report_device_error(err_word, UB_ERR_TIMEOUT);
 }
 
+// The same for MQ token quads; rows of whole 64-block chunks (they are then whole 128-byte lines).
+inline size_t q8_imma_fixed(int MQ, int K) { return static_cast<size_t>(MQ) * (K / 32) * (256 + 16); }
+inline int q8_imma_stages(int MQ, int K) {
+  const size_t fixed = q8_imma_fixed(MQ, K), stage = kQ8StageBytes;
+  if (K % (32 * kQ8ChunkBlocks) != 0 || fixed + 2 * stage > kSmemBudget) return 0;
+  const int S = static_cast<int>((kSmemBudget - fixed) / stage), s = S < kMaxStages ? S : kMaxStages;
+  return s * stage < static_cast<size_t>(kCW) * 7 * MQ * 64 * sizeof(float) ? 0 : s;
+}
+
 template <typename XT, int MQ>
 int launch_q8_imma(const uint8_t* wq, const XT* x, void* y, int M, int N, int K, int y_dtype, bool fresh, cudaStream_t s) {
   typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(ub::tensor_map_encoder());
-  // whole 64-block chunks (rows are then whole 128-byte lines) and a 16-byte aligned base for the tensor map
-  if (!enc || K % (32 * kQ8ChunkBlocks) != 0 || (reinterpret_cast<uintptr_t>(wq) & 15)) return UB_ERR_UNSUPPORTED;
-  const int nblk = K / 32;
-  const size_t fixed = static_cast<size_t>(MQ) * nblk * (256 + 16);
-  if (fixed + 2 * static_cast<size_t>(kQ8StageBytes) > kSmemBudget) return UB_ERR_UNSUPPORTED;
-  int S = static_cast<int>((kSmemBudget - fixed) / kQ8StageBytes);
-  if (S > kMaxStages) S = kMaxStages;
-  const size_t red_bytes = static_cast<size_t>(kCW) * 7 * MQ * 64 * sizeof(float);
-  if (static_cast<size_t>(S) * kQ8StageBytes < red_bytes) return UB_ERR_UNSUPPORTED;
+  // a 16-byte aligned base for the tensor map
+  const int S = q8_imma_stages(MQ, K), nblk = K / 32;
+  if (!enc || !S || (reinterpret_cast<uintptr_t>(wq) & 15)) return UB_ERR_UNSUPPORTED;
+  const size_t fixed = q8_imma_fixed(MQ, K);
   CUtensorMap wmap;
   const cuuint64_t row_bytes = static_cast<cuuint64_t>(nblk) * UB_Q8_0_BYTES;
   const cuuint64_t dims[3] = {128, row_bytes / 128, static_cast<cuuint64_t>(N)};
@@ -845,6 +855,10 @@ int q4k_gemv_imma(const void* wq, const XT* x, void* y, int M, int N, int K, int
   if (M <= 4) return launch_imma<XT, 2>(w, x, y, M, N, K, y_dtype, fresh, a, s);
   return launch_imma<XT, 4>(w, x, y, M, N, K, y_dtype, fresh, a, s);
 }
+
+// Do the kernels of this file take 1 <= M <= 8 tokens of such rows (aligned ones)?
+bool q4k_imma_takes(int M, int K) { return imma_stages(M <= 2 ? 1 : M <= 4 ? 2 : 4, imma_geom(K, imma_tm_ok(K))) > 0; }
+bool q8_0_imma_takes(int M, int K) { return q8_imma_stages(M <= 4 ? 1 : 2, K) > 0; }
 
 // Q8_0 flavour, same contract.
 template <typename XT>

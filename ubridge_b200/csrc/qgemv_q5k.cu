@@ -248,10 +248,16 @@ qgemv_q5k_kernel(const uint8_t* __restrict__ wq, const XT* __restrict__ x, void*
   if (!ok && lane == 0) report_device_error(err_word, UB_ERR_TIMEOUT);
 }
 
+// Bytes of a stage of weight rows and of MT tokens' limbs; a plan has at least two stages.
+inline size_t plan_stage_bytes(int K) { return kW * static_cast<size_t>(K / UB_QK_K) * UB_Q5K_BYTES; }
+inline size_t plan_x_bytes(int MT, int K) {
+  return MT * (static_cast<size_t>(K / 16) * sizeof(XSlot) + static_cast<size_t>(K / UB_QK_K) * 4);
+}
+inline bool plan_fits(int MT, int K) { return plan_x_bytes(MT, K) + 2 * plan_stage_bytes(K) <= kDynBudgetOne; }
+
 template <typename XT, int MT>
 int launch_q5k(const uint8_t* w, const XT* x, void* y, int M, int N, int K, int out_dtype, bool fresh, cudaStream_t s) {
-  const size_t row_bytes = static_cast<size_t>(K / UB_QK_K) * UB_Q5K_BYTES, stage_bytes = kW * row_bytes;
-  const size_t xbytes = MT * (static_cast<size_t>(K / 16) * sizeof(XSlot) + static_cast<size_t>(K / UB_QK_K) * 4);
+  const size_t stage_bytes = plan_stage_bytes(K), xbytes = plan_x_bytes(MT, K);
   int ctas = 2;
   int S = xbytes + 2 * stage_bytes <= kDynBudget ? static_cast<int>((kDynBudget - xbytes) / stage_bytes) : 0;
   if (S < 2) {
@@ -287,6 +293,9 @@ int launch_q5k(const uint8_t* w, const XT* x, void* y, int M, int N, int K, int 
 }  // namespace
 
 namespace ub {
+
+// Does the staged kernel take M tokens of such rows (aligned ones)?
+bool q5k_staged_takes(int M, int K) { return K % 2048 == 0 && plan_fits(M > 2 ? 4 : M, K); }
 
 // y[M,N] = x[M,K] . dequant(Wq)^T for one to four tokens of Q5_K; UB_ERR_UNSUPPORTED (without touching the thread's
 // status) for what this kernel does not take: other M, K not a multiple of 2048 or too long for two stages beside

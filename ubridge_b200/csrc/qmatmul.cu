@@ -258,9 +258,7 @@ int qmatmul(bool is_q4k, int x_dtype, void* y, const void* x, const void* wq, in
   // faster one.  One token of Q4_K, and of Q8_0 with rows of whole 2048 values, has kernels of its own.
   if (M <= kDecodeMaxM && (M >= 2 || (!is_q4k && K % 2048 != 0)) && K % UB_QK_K == 0 &&
       ub::unit_pays(is_q4k ? 12 : 8, M, N, K, x_dtype == UB_DTYPE_F32, out_dtype == UB_DTYPE_F32)) {
-    // what ran on CUDA cores before was never requested ahead of the dependency wait
-    const bool late = K % 2048 != 0 && (M == 1 || out_dtype == UB_DTYPE_F32);
-    const int st = ub::gguf_gemm_unit(is_q4k ? 12 : 8, y, out_dtype, x, x_dtype == UB_DTYPE_F32, wq, M, N, K, fresh || late, s);
+    const int st = ub::gguf_gemm_unit(is_q4k ? 12 : 8, y, out_dtype, x, x_dtype == UB_DTYPE_F32, wq, M, N, K, fresh, s);
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   auto decode = [&]() {
