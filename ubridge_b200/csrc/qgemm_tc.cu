@@ -357,7 +357,7 @@ qgemm_q4k_tc_kernel(__nv_bfloat16* __restrict__ y, int M, int N, int K, int* err
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int j = 0; j < 32; j++) {
-            float f = __uint_as_float(v[j]) * one_piece_unscale(FMT ? kQ8 : kQ4K);
+            float f = __uint_as_float(v[j]);
             if (MODE == 2) f *= run_w[c0 + c + j];
             st_col[(c + j) * 128] = __float2bfloat16_rn(f);
           }

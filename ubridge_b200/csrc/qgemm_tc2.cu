@@ -111,7 +111,6 @@ qgemm_tc2_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ xf
   constexpr uint32_t kXBytes = TOK * 128, kStage = kXBytes * (XF || PIECES == 1 ? 2 : 1);
   constexpr uint32_t kPitch = slot_pitch(FMT), kWBytes = slot_bytes(FMT), kWOff = STAGES * kStage;
   static_assert(static_cast<uint32_t>(TOK) * 512 / 8 * 7 <= kWOff, "the ring takes the partial sums");
-  constexpr float kUnscale = PIECES == 1 ? one_piece_unscale(FMT) : 1.f;
   constexpr uint32_t kACol = TOK, kTmemCols = 512 / CTAS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_raw = static_cast<uint32_t>(__cvta_generic_to_shared(smem2));
@@ -236,8 +235,7 @@ qgemm_tc2_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ xf
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int j = 0; j < 32; j++)
-            if (live && c + j < valid) store_y(y, at0 + static_cast<size_t>(c + j) * N, y_dtype,
-                                                  __uint_as_float(v[j]) * kUnscale);
+            if (live && c + j < valid) store_y(y, at0 + static_cast<size_t>(c + j) * N, y_dtype, __uint_as_float(v[j]));
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -289,7 +287,7 @@ qgemm_tc2_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ xf
         }
 #pragma unroll
         for (int q = 0; q < 4; q++)
-          if (live && 4 * g + q < valid) store_y(y, at0 + static_cast<size_t>(4 * g + q) * N, y_dtype, f[q] * kUnscale);
+          if (live && 4 * g + q < valid) store_y(y, at0 + static_cast<size_t>(4 * g + q) * N, y_dtype, f[q]);
       }
       break;
     }

@@ -27,6 +27,14 @@ __device__ __forceinline__ uint32_t deq_pair(uint32_t w4, __nv_bfloat162 s, __nv
   return bf162_bits(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&n), s, c));
 }
 
+// The same with s of any size: the byte times 2^-6 first (exact), s carries 2^6.
+template <int SEL>
+__device__ __forceinline__ uint32_t deq_pair_wide(uint32_t w4, __nv_bfloat162 s, __nv_bfloat162 c) {
+  const uint32_t n = __byte_perm(w4, 0u, SEL), big = 0x7F007F00u;  // 2^127
+  const __nv_bfloat162 v = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&n), *reinterpret_cast<const __nv_bfloat162*>(&big));
+  return bf162_bits(__hfma2(v, s, c));
+}
+
 // Two signed bytes A and B of a word (given with their sign bits flipped: q + 128) -> packed bf16 (d * q): q 2^-6 from the bf16
 // n * 2^-133 in one exact step (2^127 n 2^-133 - 2), then d in two pieces, which carry 2^6: fma(q, dh, q dl) is d q rounded once.
 template <int SEL>
@@ -89,17 +97,20 @@ __device__ __forceinline__ int lds_s8(uint32_t a) {
 // pieces 2100.  It is the largest part of a launch of few tokens: 16 tokens through 28672x4096 26.4 -> 23.9 us, Q8_0 45 tokens
 // 14336x4096 24.8 -> 21.8 us.
 //
-// one_piece: values times 2^-one_piece_exp, which the kernels' epilogues take back from the f32 sums.  Q4_K: with 2^28 the
-// scale times 2^133 stays finite for every f16 super-block scale (65504 * 63 * 2^105 < 2^127), and the smallest (6e-8)
-// is 2e-16, nowhere near bf16's smallest normal number: every bit of the values is the same without it.
-constexpr int one_piece_exp(int f) { return f == kQ4K ? 28 : 0; }
-constexpr float one_piece_unscale(int f) { return f == kQ4K ? 0x1p28f : 1.f; }
+// One piece of Q4_K: low nibbles as q 2^-133, high ones as 16 q 2^-133, and a scale that carries the rest, finite in bf16 while a
+// super-block's d is below this (63 * 2^-11 * 2^133 < 2^128; trained weights have d of 1e-5 to 4e-4).  Where a row of the warp has a
+// larger one, the nibbles are multiplied by 2^127 first, exactly: two instructions more per four values.  Both give bf16(s q - m), s
+// and m rounded to bf16, and accumulators of ordinary size: with a factor on all weights instead, taken back from the sums, products of
+// activations below 2^-92 would be subnormal.  Low nibbles moved up by four bits would do until 2^-7: 0.7 % of an expert layer of
+// 256 tokens, 0.9 % of sixteen tokens through a wide block.
+constexpr float kOnePieceMaxD = 0x1p-11f;
 
 template <int FMT>
 struct RowBlock {
   uint32_t base;  // shared-memory address of the row's block: 16-byte aligned, Q6_K: 2-byte aligned
   uint32_t scw[2], mnw[2], fifth[8];
   float d, dmin;
+  bool wide;  // Q4_K: of any row of the warp
 
   __device__ __forceinline__ void open(uint32_t at) {
     base = at;
@@ -108,6 +119,7 @@ struct RowBlock {
       lds128(base, h);
       d = half_bits_to_f32(h[0]), dmin = half_bits_to_f32(h[0] >> 16);
       q4k_unpack_scales(h[1], h[2], h[3], scw[0], scw[1], mnw[0], mnw[1]);
+      if constexpr (FMT == kQ4K) wide = __any_sync(0xFFFFFFFFu, !(fabsf(d) < kOnePieceMaxD));
       if constexpr (FMT == kQ5K) lds128(base + 16, fifth), lds128(base + 32, fifth + 4);  // of all eight sub-blocks
     }
     if constexpr (FMT == kQ6K) d = half_bits_to_f32(lds32((base + 208) & ~3u) >> ((base & 2) * 8));
@@ -139,15 +151,26 @@ struct RowBlock {
       uint32_t q[8];
       lds128(base + 16 + 32 * G, q), lds128(base + 32 + 32 * G, q + 4);
 #pragma unroll
-      for (int h = 0; h < 2; h++) {  // upper nibbles stay where they are: 16 q
+      for (int h = 0; h < 2; h++) {
         float s, m;
         pair(2 * G + h, s, m);
-        const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 0x1p101f : 0x1p105f)), ndm = __float2bfloat162_rn(m * -0x1p-28f);
+        const __nv_bfloat162 ndm = __float2bfloat162_rn(-m);
+        if (!wide) {
+          const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 0x1p65f : 0x1p69f) * 0x1p64f);
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const uint32_t v = q[i] & (h ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
-          ot[16 * h + 2 * i] = deq_pair<0x4140>(v, dsc, ndm);
-          ot[16 * h + 2 * i + 1] = deq_pair<0x4342>(v, dsc, ndm);
+          for (int i = 0; i < 8; i++) {
+            const uint32_t v = q[i] & (h ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
+            ot[16 * h + 2 * i] = deq_pair<0x4140>(v, dsc, ndm);
+            ot[16 * h + 2 * i + 1] = deq_pair<0x4342>(v, dsc, ndm);
+          }
+        } else {
+          const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 4.f : 64.f));
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const uint32_t v = q[i] & (h ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
+            ot[16 * h + 2 * i] = deq_pair_wide<0x4140>(v, dsc, ndm);
+            ot[16 * h + 2 * i + 1] = deq_pair_wide<0x4342>(v, dsc, ndm);
+          }
         }
       }
     } else {
