@@ -66,9 +66,17 @@ constexpr uint32_t x_bytes(bool xf) { return kTok * x_vals(xf) * 2 * (xf ? 3 : 1
 constexpr int w_slots(int f) { return f == kQ4K || f == kQ40 ? 4 : f == kQ5K ? 3 : 2; }
 constexpr int threads_of(bool xf) { return (xf ? 17 : 16) * 32; }
 constexpr uint32_t kRecvBytes = (128 + 8) * kTok * 4;
+// Rounding.  A chain of n additions rounds n / 2 times as much as one.  Without an offset a stage of four groups is summed by itself,
+// then the stages of a super-block, then super-blocks.  Q6_K has twice the groups, and what an addition of a super-block
+// rounds off is summed beside it, in shared memory (in registers it would spill: 9 % of sixteen tokens, 13 % of eight in f32; so 1 to
+// 6 %).  Error of f32 results as a part of the CUDA-core kernels', bf16 activations: Q6_K 1200 rows of 1536 values 0.98 (1.20 in one
+// chain per super-block), 24000 rows of 4352 values 0.75 (1.14 without the rest), Q8_0 1024 values 0.97 (1.04 in one chain).
+constexpr bool keeps_stages(int f) { return f == kQ6K || f == kQ8; }
+constexpr bool keeps_rest(int f) { return f == kQ6K; }
+constexpr uint32_t rest_bytes(int f) { return keeps_rest(f) ? 128 * kTok * 4 : 0; }
 constexpr size_t smem_of(int f, bool xf) {
   return static_cast<size_t>(x_slots(xf)) * (x_bytes(xf) + x_vals(xf) * 2) + static_cast<size_t>(w_slots(f)) * slot_bytes(f) +
-         kRecvBytes + 1024;
+         kRecvBytes + rest_bytes(f) + 1024;
 }
 
 struct SharedU {
@@ -270,7 +278,9 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
   constexpr int kXVals = x_vals(XF), kPerSb = 256 / kSV, kPerX = kXVals / kSV;  // stages per super-block / activation slot
   constexpr uint32_t kXSlot = x_bytes(XF), kPiece = kTok * kXVals * 2, kSub = kTok * 128;  // kSub: 64 values
   constexpr uint32_t kPitch = slot_pitch(FMT), kWBytes = slot_bytes(FMT), kSums = kXVals * 2;
-  constexpr uint32_t kWOff = kXS * kXSlot, kSumOff = kWOff + WST * kWBytes, kRecvOff = kSumOff + kXS * kSums;
+  constexpr uint32_t kWOff = kXS * kXSlot, kSumOff = kWOff + WST * kWBytes, kRecvOff = kSumOff + kXS * kSums,
+                     kRestOff = kRecvOff + kRecvBytes;
+  constexpr bool kRest = keeps_rest(FMT), kOwn = keeps_stages(FMT);
   constexpr uint32_t kACol = kStages * 64;
   static_assert(kACol + kStages * (kSV / 2) <= kTmemCols && kXS <= kMaxX && WST <= kMaxW, "plan");
   static_assert(kWOff % 1024 == 0, "alignment");
@@ -401,6 +411,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
           : "memory");
       return all_ok != 0;
     };
+    float4* const rest = reinterpret_cast<float4*>(tiles + kRestOff) + row;  // this thread's own
     int s = 0, ws = 0, xs = 0;
     uint32_t phase = 0, wphase = 0, xphase = 0;
     for (int tile = vblock; tile < ntiles && ok; tile += vgrid) {
@@ -473,38 +484,64 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const int first_g = has_offset(FMT) ? 4 * i : 0;
-          constexpr int kAtOnce = TT > 8 ? 1 : TT > 4 ? 2 : 4;  // groups in registers
+          constexpr int kAtOnce = TT > 8 ? 1 : TT > 4 ? 2 : 4;          // groups in registers
+          constexpr int kChunk = kOwn && TT > 8 ? 8 : TT;  // tokens
 #pragma unroll
-          for (int g0 = 0; g0 < 4; g0 += kAtOnce) {
-            float v[kAtOnce][TT];
+          for (int t0 = 0; t0 < TT; t0 += kChunk) {
+            float own[kChunk];  // the stage's sums
 #pragma unroll
-            for (int g = 0; g < kAtOnce; g++) tmem_ld<TT>(d_lane + 64u * s + kTok * (g0 + g), v[g]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (g0 + kAtOnce == 4) {
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              __syncwarp();
-              if (lane == 0) tc_mbar_arrive(dempty + 8 * s);
-            }
+            for (int g0 = 0; g0 < 4; g0 += kAtOnce) {
+              float v[kAtOnce][kChunk];
 #pragma unroll
-            for (int g = 0; g < kAtOnce; g++)
-#pragma unroll
-              for (int t = 0; t < TT; t += 2) {
-                if (!has_offset(FMT) && i + g0 + g == 0)
-                  mul2(part[t], part[t + 1], v[g][t], v[g][t + 1], sg[first_g]);
-                else
-                  fma2(part[t], part[t + 1], v[g][t], v[g][t + 1], sg[first_g + g0 + g]);
+              for (int g = 0; g < kAtOnce; g++) tmem_ld<kChunk>(d_lane + 64u * s + kTok * (g0 + g) + t0, v[g]);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              if (t0 + kChunk == TT && g0 + kAtOnce == 4) {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc_mbar_arrive(dempty + 8 * s);
               }
+#pragma unroll
+              for (int g = 0; g < kAtOnce; g++)
+#pragma unroll
+                for (int t = 0; t < kChunk; t += 2) {
+                  float* const to = kOwn ? own + t : part + t0 + t;
+                  if (!has_offset(FMT) && (kOwn || i == 0) && g0 + g == 0)
+                    mul2(to[0], to[1], v[g][t], v[g][t + 1], sg[0]);
+                  else
+                    fma2(to[0], to[1], v[g][t], v[g][t + 1], sg[first_g + g0 + g]);
+                }
+            }
+            if constexpr (kOwn)
+#pragma unroll
+              for (int t = 0; t < kChunk; t++) part[t0 + t] = i == 0 ? own[t] : part[t0 + t] + own[t];
           }
           if (++s == kStages) s = 0, phase ^= 1;
         }
         if (!ok) break;
 #pragma unroll
-        for (int t = 0; t < TT; t++) acc[t] += part[t];
+        for (int t = 0; t < TT; t++) {
+          const float before = acc[t];
+          acc[t] += part[t];
+          if (kRest) part[t] -= acc[t] - before;  // what the addition has rounded off
+        }
+        if constexpr (kRest)
+#pragma unroll
+          for (int q = 0; q < TT / 4; q++) {
+            float4 r = sb ? rest[128 * q] : make_float4(0.f, 0.f, 0.f, 0.f);
+            r.x += part[4 * q], r.y += part[4 * q + 1], r.z += part[4 * q + 2], r.w += part[4 * q + 3];
+            rest[128 * q] = r;
+          }
         if (++ws == WST) ws = 0, wphase ^= 1;
         if (FMT == kQ6K) skew = (skew + 210) & 15u;
       }
       if (KS > 1) ok = agree(ok);  // a warp may have given up on its own; all four come here, once: one tile per CTA
       if (!ok) break;
+      if constexpr (kRest)
+#pragma unroll
+        for (int t = 0; t < TT; t++) {
+          const float r = reinterpret_cast<const float*>(rest + 128 * (t / 4))[t % 4];
+          if (fabsf(r) < INFINITY) acc[t] += r;  // not behind a sum that is infinite
+        }
       if (KS == 1) {
         if (n0 + wrow < N) {
 #pragma unroll
@@ -537,11 +574,22 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
       if (!ok) break;
       for (int i = row; i < mine * (TT / 4); i += 128) {
         const int q = i / mine, l = i - q * mine, out = n0 + tile_row(FMT, first + l);
-        float f[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int r = 0; r < KS; r++) {
-          const float4 p = *reinterpret_cast<const float4*>(tiles + kRecvOff + ((r * (TT / 4) + q) * own + l) * 16);
-          f[0] += p.x, f[1] += p.y, f[2] += p.z, f[3] += p.w;
+        auto rank = [&](int r) {
+          return *reinterpret_cast<const float4*>(tiles + kRecvOff + ((r * (TT / 4) + q) * own + l) * 16);
+        };
+        auto add = [](float4& a, const float4& b) { a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w; };
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < KS; r += 4) {  // pairs of pairs: a chain of eight would round more
+          float4 u = rank(r);
+          if (r + 1 < KS) add(u, rank(r + 1));
+          if (r + 2 < KS) {
+            float4 v = rank(r + 2);
+            if (r + 3 < KS) add(v, rank(r + 3));
+            add(u, v);
+          }
+          add(sum, u);
         }
+        const float f[4] = {sum.x, sum.y, sum.z, sum.w};
         if (out < N) {
 #pragma unroll
           for (int t = 0; t < 4; t++)
