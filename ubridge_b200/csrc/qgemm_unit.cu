@@ -104,6 +104,19 @@ __device__ __forceinline__ void store_one(void* y, size_t at, int dtype, float v
     static_cast<__half*>(y)[at] = __float2half_rn(v);
 }
 
+__device__ __forceinline__ float load_one(const void* y, size_t at, int dtype) {
+  if (dtype == UB_DTYPE_F32) return static_cast<const float*>(y)[at];
+  if (dtype == UB_DTYPE_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(y)[at]);
+  return __half2float(static_cast<const __half*>(y)[at]);
+}
+template <int N>
+__device__ __forceinline__ bool all_finite(const float (&v)[N]) {
+  float zero = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i++) zero = fmaf(v[i], 0.f, zero);
+  return zero == 0.f;
+}
+
 // Several barriers at once: one look at each costs some 200 cycles however long ago the phase ended, and the looks overlap.
 __device__ __forceinline__ bool wait2(uint32_t a, uint32_t pa, uint32_t b, uint32_t pb, volatile int* abort_flag) {
   const bool ra = tc_mbar_test(a, pa), rb = tc_mbar_test(b, pb);
@@ -263,13 +276,70 @@ struct UnitScale {
   }
 };
 
+// Value k of a weight row in global memory (2-byte aligned), by the formats' own arithmetic.
+template <int FMT>
+__device__ float weight_at(const uint8_t* row, int k) {
+  const int v = k & 255, l = v & 31, j = v >> 5;
+  auto half_at = [](const uint8_t* p) { return half_bits_to_f32(*reinterpret_cast<const unsigned short*>(p)); };
+  if constexpr (FMT == kQ8 || FMT == kQ40) {
+    const uint8_t* b = row + static_cast<size_t>(k >> 5) * (FMT == kQ8 ? 34 : 18);
+    if (FMT == kQ8) return half_at(b) * static_cast<float>(static_cast<signed char>(b[2 + l]));
+    return half_at(b) * static_cast<float>(((b[2 + (l & 15)] >> (l < 16 ? 0 : 4)) & 15) - 8);
+  } else {
+    const uint8_t* b = row + static_cast<size_t>(k >> 8) * row_sb_bytes(FMT);
+    if constexpr (FMT == kQ6K) {
+      const int h = j >> 2, p = j & 3;
+      const int q = ((b[64 * h + 32 * (p & 1) + l] >> (p < 2 ? 0 : 4)) & 15) | ((b[128 + 32 * h + l] >> (2 * p)) & 3) << 4;
+      return half_at(b + 208) * static_cast<float>(static_cast<signed char>(b[192 + (v >> 4)])) * static_cast<float>(q - 32);
+    } else {
+      const uint8_t* c = b + 4;  // 6-bit scales and mins
+      const int sc = j < 4 ? c[j] & 63 : (c[j + 4] & 15) | c[j - 4] >> 6 << 4;
+      const int mn = j < 4 ? c[j + 4] & 63 : c[j + 4] >> 4 | c[j] >> 6 << 4;
+      int q = (b[(FMT == kQ5K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1))) & 15;
+      if (FMT == kQ5K) q |= ((b[16 + l] >> j) & 1) << 4;
+      return half_at(b) * static_cast<float>(sc) * static_cast<float>(q) - half_at(b + 2) * static_cast<float>(mn);
+    }
+  }
+}
+
+// A result that came out as NaN although its token has infinities and no NaN.  The centred integer of a weight that is not zero
+// may be zero, its two terms may differ in sign, and the lower pieces of an f32 infinity are NaN; infinity times the weights has a sign
+// all the same, and finite activations do not change it.  False: the NaN stands.  (bf16 activations of formats without an offset
+// need none of this: infinity times the integer is the plain product.)
+template <int FMT, bool XF>
+__device__ __forceinline__ bool sum_of_infinities(const void* x, const uint8_t* w_row, int K, float& sum) {
+  bool any = false;
+  sum = 0.f;
+  for (int k = 0; k < K; k += 4) {
+    float f[4];
+    if (XF) {
+      const float4 v = *reinterpret_cast<const float4*>(static_cast<const float*>(x) + k);
+      f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+    } else {
+      const uint2 v = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(x) + k);
+      f[0] = __uint_as_float(v.x << 16), f[1] = __uint_as_float(v.x & 0xFFFF0000u);
+      f[2] = __uint_as_float(v.y << 16), f[3] = __uint_as_float(v.y & 0xFFFF0000u);
+    }
+#pragma unroll 1
+    for (int e = 0; e < 4; e++) {
+      const float v = e == 0 ? f[0] : e == 1 ? f[1] : e == 2 ? f[2] : f[3];
+      if (fabsf(v) < INFINITY) continue;
+      if (v != v) return false;
+      sum = fmaf(v, weight_at<FMT>(w_row, k + e), sum);
+      if (sum != sum) return false;  // zero weights, or infinities of both signs
+      any = true;
+    }
+  }
+  return any;
+}
+
 __host__ __device__ constexpr int tile_row(int f, int lane) { return f == kQ6K ? 8 * (lane & 15) + (lane >> 4) : lane; }
 
 // TT: tokens that the sums are kept of (4, 8, 16); the MMAs always take 16.
 template <int FMT, bool XF, int TT>
 __global__ void __launch_bounds__(threads_of(XF), 2)
-qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ xf, const uint8_t* __restrict__ wq, int M,
-                  int N, int K, int KS, int early, int* err_word, const __grid_constant__ CUtensorMap x_map,
+qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const void* __restrict__ x, const uint8_t* __restrict__ wq, int M, int N, int K,
+                  int KS, int early, int* err_word, const __grid_constant__ CUtensorMap x_map,
                   const __grid_constant__ CUtensorMap w_map) {
   extern __shared__ __align__(1024) unsigned char smem_u[];
   __shared__ SharedU sh;
@@ -280,7 +350,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
   constexpr uint32_t kPitch = slot_pitch(FMT), kWBytes = slot_bytes(FMT), kSums = kXVals * 2;
   constexpr uint32_t kWOff = kXS * kXSlot, kSumOff = kWOff + WST * kWBytes, kRecvOff = kSumOff + kXS * kSums,
                      kRestOff = kRecvOff + kRecvBytes;
-  constexpr bool kRest = keeps_rest(FMT), kOwn = keeps_stages(FMT);
+  constexpr bool kRest = keeps_rest(FMT), kOwn = keeps_stages(FMT), kLook = XF || has_offset(FMT);
   constexpr uint32_t kACol = kStages * 64;
   static_assert(kACol + kStages * (kSV / 2) <= kTmemCols && kXS <= kMaxX && WST <= kMaxW, "plan");
   static_assert(kWOff % 1024 == 0, "alignment");
@@ -410,6 +480,17 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
           : "r"(mine_ok ? 1u : 0u)
           : "memory");
       return all_ok != 0;
+    };
+    // Results that this thread has stored, of tokens first .. first + n - 1, when one of them is not finite.
+    auto look_again = [&](int first, int n, int out) {
+#pragma unroll 1
+      for (int m = first; m < first + n && m < M; m++) {
+        const size_t at = static_cast<size_t>(m) * N + out;
+        float sum = load_one(y, at, y_dtype);
+        if (sum != sum && sum_of_infinities<FMT, XF>(static_cast<const char*>(x) + static_cast<size_t>(m) * K * (XF ? 4 : 2),
+                                                     wq + static_cast<size_t>(out) * nsb_all * row_sb_bytes(FMT), K, sum))
+          store_one(y, at, y_dtype, sum);
+      }
     };
     float4* const rest = reinterpret_cast<float4*>(tiles + kRestOff) + row;  // this thread's own
     int s = 0, ws = 0, xs = 0;
@@ -547,6 +628,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
 #pragma unroll
           for (int t = 0; t < TT; t++)
             if (m0 + t < M) store_one(y, static_cast<size_t>(m0 + t) * N + n0 + wrow, y_dtype, acc[t]);
+          if (kLook && !all_finite(acc)) look_again(m0, TT, n0 + wrow);
         }
         continue;
       }
@@ -594,6 +676,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
 #pragma unroll
           for (int t = 0; t < 4; t++)
             if (m0 + 4 * q + t < M) store_one(y, static_cast<size_t>(m0 + 4 * q + t) * N + out, y_dtype, f[t]);
+          if (kLook && !all_finite(f)) look_again(m0 + 4 * q, 4, out);
         }
       }
     }
@@ -786,7 +869,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const float* __restrict__ x
       const int valid = min(kTok, M - m0);
       ok = __all_sync(0xFFFFFFFFu, tc_wait(xempty + 8 * xs, xphase ^ 1, abort_flag));
       if (!ok) break;
-      const float* src = xf + static_cast<size_t>(m0) * K + sb * 256 + (q & 1) * 128;
+      const float* src = static_cast<const float*>(x) + static_cast<size_t>(m0) * K + sb * 256 + (q & 1) * 128;
       unsigned char* const slot = tiles + xs * kXSlot;
       float* sums = reinterpret_cast<float*>(tiles + kSumOff + xs * kSums);
 #pragma unroll 2
@@ -899,7 +982,7 @@ int launch_unit(void* y, int y_dtype, const void* x, const void* wq, int M, int 
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = 2;
-    e = cudaLaunchKernelEx(&cfg, kernel, y, y_dtype, static_cast<const float*>(x), static_cast<const uint8_t*>(wq), M, N, K,
+    e = cudaLaunchKernelEx(&cfg, kernel, y, y_dtype, x, static_cast<const uint8_t*>(wq), M, N, K,
                            ks, fresh ? 0 : 1, ub::device_error_word(), xmap, wmap);
   }
   if (e != cudaSuccess) {
