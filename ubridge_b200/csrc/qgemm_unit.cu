@@ -109,11 +109,12 @@ __device__ __forceinline__ float load_one(const void* y, size_t at, int dtype) {
   if (dtype == UB_DTYPE_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(y)[at]);
   return __half2float(static_cast<const __half*>(y)[at]);
 }
+// of the first n
 template <int N>
-__device__ __forceinline__ bool all_finite(const float (&v)[N]) {
+__device__ __forceinline__ bool all_finite(const float (&v)[N], int n) {
   float zero = 0.f;
 #pragma unroll
-  for (int i = 0; i < N; i++) zero = fmaf(v[i], 0.f, zero);
+  for (int i = 0; i < N; i++) zero = fmaf(i < n ? v[i] : 0.f, 0.f, zero);
   return zero == 0.f;
 }
 
@@ -628,7 +629,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const void* __restrict__ x,
 #pragma unroll
           for (int t = 0; t < TT; t++)
             if (m0 + t < M) store_one(y, static_cast<size_t>(m0 + t) * N + n0 + wrow, y_dtype, acc[t]);
-          if (kLook && !all_finite(acc)) look_again(m0, TT, n0 + wrow);
+          if (kLook && !all_finite(acc, M - m0)) look_again(m0, TT, n0 + wrow);
         }
         continue;
       }
@@ -676,7 +677,7 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const void* __restrict__ x,
 #pragma unroll
           for (int t = 0; t < 4; t++)
             if (m0 + 4 * q + t < M) store_one(y, static_cast<size_t>(m0 + 4 * q + t) * N + out, y_dtype, f[t]);
-          if (kLook && !all_finite(f)) look_again(m0 + 4 * q, 4, out);
+          if (kLook && !all_finite(f, M - m0 - 4 * q)) look_again(m0 + 4 * q, 4, out);
         }
       }
     }
