@@ -53,3 +53,40 @@ def test_no_request_ahead_where_plain_launches_took_the_call():
 ])
 def test_weights_are_requested_ahead_where_they_always_were(tag, M, K, y_f32):
     assert early(tag, M, K, y_f32)
+
+
+def takes(tag, M, N, K, x_f32, y_f32):
+    """Which kernel has the call: 1 the integer kernel, 2 two-piece weights, 0 another one."""
+    b = ctypes.c_bool
+    if tag in (Q8_0, Q4_K):
+        f = rule("few_tokens_route", "iiiibb")
+        f.restype = ctypes.c_int
+        return f(tag, M, N, K, b(x_f32), b(y_f32))
+    return int(rule("unit_takes", "iiiibb")(tag, M, N, K, b(x_f32), b(y_f32)))
+
+
+@pytest.mark.parametrize("tag,M,N,K,x_f32,y_f32", [
+    # B200, us, the other kernel / this one: 2.0 / 5.5, 2.6 / 5.5, 20.8 / 24, 10.3 / 13.9; 2.3 / 4.2 (CUDA cores), 6.9 / 10.9 (two pieces)
+    (Q6_K, 1, 1024, 512, False, False), (Q6_K, 4, 1024, 512, False, False), (Q6_K, 1, 14336, 3328, False, False),
+    (Q6_K, 2, 512, 12288, True, False), (Q8_0, 1, 2048, 512, False, True), (Q4_K, 16, 4096, 512, True, False),
+])
+def test_calls_that_other_kernels_do_faster(tag, M, N, K, x_f32, y_f32):
+    assert takes(tag, M, N, K, x_f32, y_f32) != 1
+
+
+@pytest.mark.parametrize("tag,M,N,K,x_f32,y_f32", [
+    (Q4_K, 4, 4096, 14336, False, False), (Q8_0, 4, 6144, 5120, False, False), (Q4_0, 1, 4096, 4352, False, False),
+    (Q5_K, 4, 14336, 3328, False, True), (Q6_K, 8, 16384, 5120, False, False), (Q5_K, 1, 8192, 28672, False, False),
+])
+def test_calls_that_this_kernel_does_faster(tag, M, N, K, x_f32, y_f32):
+    assert takes(tag, M, N, K, x_f32, y_f32) == 1
+
+
+def test_two_piece_weights_only_for_f32_tokens_in_a_second_pass():
+    for tag in (Q8_0, Q4_K):
+        for M in range(1, 17):
+            for N in (1, 300, 1200, 4096, 28672):
+                for K in ROWS:
+                    for y_f32 in (False, True):
+                        assert takes(tag, M, N, K, False, y_f32) != 2
+                        assert M > 8 or takes(tag, M, N, K, True, y_f32) != 2

@@ -605,9 +605,15 @@ int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32
     case 2: return by_size<kQ40>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
     case 13: return by_size<kQ5K>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
     case 14: return by_size<kQ6K>(y, y_dtype, x, x_f32, wq, M, N, K, fresh, s);
+    // Q4_K and Q8_0: nine to sixteen f32 tokens, see few_tokens_route in qgemm_unit.cu
+    case 12: return x_f32 && M <= 64 ? launch2<kQ4K, 64, 6, 3, true>(y, y_dtype, x, wq, M, N, K, fresh, s) : UB_ERR_UNSUPPORTED;
+    case 8: return x_f32 && M <= 64 ? launch2<kQ8, 64, 6, 3, true>(y, y_dtype, x, wq, M, N, K, fresh, s) : UB_ERR_UNSUPPORTED;
     default: return UB_ERR_UNSUPPORTED;
   }
 }
+
+// Parts of K of a tile of 64 tokens.
+int two_piece_split(int tiles, int nsb) { return k_split(tiles, nsb, 1); }
 
 // y (bf16) = x (bf16) . W^T with weights rounded to bf16 once: the few-token launches of q4k_gemm_tc and q8_0_gemm_tc (fmt:
 // GGML type; Q8_0 up to 64 tokens).  Two CTAs per SM up to 64 tokens of Q4_K: one CTA's chain of barriers (830 cycles per

@@ -46,6 +46,7 @@ bool q5k_staged_takes(int M, int K);
 bool q6k_staged_takes(int M, int K);
 bool q4k_imma_takes(int M, int K);
 bool q8_0_imma_takes(int M, int K);
+int two_piece_split(int tiles, int nsb);
 }
 
 namespace {
@@ -1007,12 +1008,14 @@ int by_type(void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int
                : by_tokens<FMT, false>(y, y_dtype, x, wq, M, N, K, fresh, s);
 }
 
-// ---- up to sixteen tokens of Q4_K and Q8_0: this kernel or the decode kernels (CUDA cores, integer MMA) ----
+// ---- up to sixteen tokens: this kernel, the decode kernels (CUDA cores, integer MMA) or two-piece weights (qgemm_tc2.cu) ----
 // This kernel's time hardly depends on the tokens and falls with the matrix only down to the 3.5 us that the barriers, tensor
 // memory and the cluster exchange take; a decode kernel's pass takes one, two, four or eight tokens and scales with the
-// bytes.  No line of one size separates them, so both are priced, in us.  Where the decode kernels' time is within 5 % they
-// are taken.  Some crossings, B200, decode / this, bf16: Q4_K two tokens 14336x3328 10 / 14.5, four 4096x4352 18 / 8.5, four
-// 14336x3328 14 / 16, eight 14336x3328 41 / 18; Q8_0 four tokens 6144x4096 9 / 10, four 6144x5120 76 / 12.5, eight 28672x8192 66 / 53.
+// bytes.  No line of one size separates them, so all are priced, in us, by straight lines fitted to 23600 timings on B200 (256 to
+// 16384 values, 300 to 28672 rows); nine of ten are within 15 %.  This kernel is taken where it is faster by more than a twentieth.  Some
+// crossings, decode / this, bf16: Q4_K two tokens 14336x3328 10 / 14.5, four 4096x4352 18 / 8.5, four 14336x3328 14 / 16, eight
+// 14336x3328 41 / 18; Q8_0 four tokens 6144x4096 9 / 10, four 6144x5120 76 / 12.5; Q6_K two tokens 1024x512 2.3 / 5.5, 28672x8192 69 / 92,
+// 4096x14336 34 / 26; Q5_K one token 4096x14336 16.6 / 18.4, 8192x28672 450 / 54; Q4_0 one token 28672x8192 33 / 43, 4096x4352 24 / 8.
 struct Pass {  // us: fixed, per super-block of a row, per 1024 rows, per both
   float fixed, sb, rows, sb_rows;
   float us(int N, int nsb) const {
@@ -1022,15 +1025,32 @@ struct Pass {  // us: fixed, per super-block of a row, per 1024 rows, per both
 };
 constexpr float kNever = 1e9f;  // no decode kernel of this kind takes the pass
 
-// Token passes as the dispatchers cut them (Q4_K, Q8_0).
+// Token passes as the dispatchers cut them.
 float decode_us(int type, int M, int N, int K) {
   const int nsb = K / UB_QK_K;
   switch (type) {
+    case 2:
+    case 13:
+    case 14: {  // one to four tokens: rows that are not whole 2048 values / staged, two CTAs per SM / one
+      static const Pass lines[3][3][4] = {
+          {{{1.206f, .544f, -.017f, .198f}, {1.209f, .88f, .004f, .236f}, {2.329f, 1.439f, .06f, .337f}, {1.578f, 1.127f, -.045f, .371f}},
+           {{1.953f, .096f, .177f, .019f}, {1.786f, .18f, .164f, .037f}, {2.644f, .155f, -.073f, .088f}, {3.147f, .186f, -.05f, .103f}},
+           {{1.075f, .099f, .17f, .027f}, {2.387f, .114f, .38f, .037f}, {1.46f, .222f, .716f, .042f}, {-.107f, .341f, 2.921f, -.031f}}},
+          {{{1.165f, .627f, .017f, .242f}, {1.218f, .743f, .059f, .242f}, {2.418f, 1.305f, .09f, .436f}, {1.339f, 1.479f, -.243f, .477f}},
+           {{2.196f, .039f, .189f, .036f}, {1.449f, .143f, .676f, .026f}, {1.841f, .208f, .326f, .073f}, {1.589f, .311f, .451f, .09f}},
+           {{2.247f, .045f, .002f, .05f}, {3.245f, .06f, -.17f, .071f}, {2.218f, .135f, .799f, .082f}, {1.73f, .197f, 1.038f, .099f}}},
+          {{{1.178f, .354f, .118f, .057f}, {1.341f, .406f, .156f, .076f}, {2.665f, .655f, .214f, .137f}, {1.482f, .494f, .212f, .107f}},
+           {{1.616f, .084f, .564f, .013f}, {1.731f, .124f, .635f, .032f}, {2.036f, .181f, .356f, .066f}, {1.604f, .282f, .515f, .078f}},
+           {{2.139f, .05f, -.006f, .053f}, {3.008f, .069f, -.123f, .072f}, {1.871f, .142f, .742f, .071f}, {1.897f, .188f, .945f, .093f}}}};
+      const bool staged = type == 2 ? ub::q4_0_staged_takes(M, K) : type == 13 ? ub::q5k_staged_takes(M, K) : ub::q6k_staged_takes(M, K);
+      if (M > 4 || (K % 2048 == 0 && !staged)) return kNever;
+      return lines[type == 2 ? 0 : type == 13 ? 1 : 2][K % 2048 ? 0 : K <= 4096 ? 1 : 2][M - 1].us(N, nsb);
+    }
     case 8: {
-      static const Pass rest[2] = {{2.1f, .88f, 0.f, .18f}, {2.45f, .98f, .03f, .34f}};
+      static const Pass rest[4] = {{1.331f, .391f, .067f, .145f}, {1.181f, .594f, .027f, .244f}, {3.412f, .805f, .002f, .389f}, {1.196f, .987f, -.07f, .449f}};
       static const Pass lines[4] = {
           {.98f, .151f, .125f, .031f}, {1.88f, .144f, .08f, .037f}, {1.9f, .186f, .116f, .037f}, {2.45f, .343f, .146f, .049f}};
-      if (K % 2048) return M == 2 ? rest[0].us(N, nsb) : M == 4 ? rest[1].us(N, nsb) : kNever;
+      if (K % 2048) return M <= 4 ? rest[M - 1].us(N, nsb) : kNever;
       float t = 0.f;
       for (int left = M, n; left > 0; left -= n) {
         n = left < 8 ? left : 8;
@@ -1064,13 +1084,39 @@ float decode_us(int type, int M, int N, int K) {
   }
 }
 
-// us of a launch here, straight lines fitted to 1120 timings on B200 (256 to 28672 values, 512 to 40960 rows, within 20 %, f32
-// activations of more than eight tokens within 30 %): fixed, with a K split, per super-block of a CTA alone on its SM and of
-// one of two.
+// us of a launch here: fixed, with a K split, per super-block of a CTA alone on its SM and of one of two.  Clusters fill SMs in
+// pairs well before every SM has a CTA.
 struct UnitCost {
   float fixed, split, one, two;
 };
 float unit_us(int type, int M, int N, int K, bool x_f32) {
+  // up to four, eight, sixteen bf16 tokens, and f32 ones
+  static const UnitCost costs[5][6] = {
+      {{2.42f, 1.23f, .73f, 1.52f}, {2.79f, 1.4f, .79f, 1.61f}, {3.29f, 1.7f, 1.23f, 2.15f},
+       {2.53f, 1.27f, 1.04f, 1.77f}, {2.89f, 1.09f, 1.79f, 2.57f}, {4.72f, .62f, 2.82f, 3.99f}},
+      {{2.7f, 1.22f, .8f, 1.68f}, {2.26f, 1.38f, .89f, 1.68f}, {3.24f, 1.62f, .85f, 1.92f},
+       {2.86f, 1.52f, .96f, 1.9f}, {2.57f, 1.1f, 1.65f, 2.54f}, {4.18f, .4f, 2.52f, 3.91f}},
+      {{2.8f, 1.1f, .69f, 1.36f}, {2.97f, 1.22f, .63f, 1.37f}, {3.69f, 1.59f, .57f, 1.57f},
+       {2.81f, 1.29f, .88f, 1.71f}, {2.6f, 1.25f, 1.48f, 2.3f}, {3.88f, .94f, 2.34f, 3.48f}},
+      {{3.02f, 1.11f, .86f, 2.f}, {3.42f, .99f, .85f, 1.96f}, {4.09f, 1.14f, 1.17f, 2.51f},
+       {2.94f, 1.24f, 1.01f, 2.25f}, {2.92f, 1.26f, 1.76f, 2.98f}, {4.83f, .67f, 2.82f, 4.34f}},
+      {{3.29f, .94f, 1.41f, 2.83f}, {3.46f, .93f, 1.47f, 3.f}, {3.78f, 1.06f, 1.69f, 3.82f},
+       {3.61f, 1.07f, 1.52f, 3.14f}, {3.83f, .55f, 1.9f, 3.66f}, {7.06f, -.95f, 2.76f, 4.83f}}};
+  const UnitCost& c = costs[type == 12 ? 0 : type == 8 ? 1 : type == 2 ? 2 : type == 13 ? 3 : 4][(M <= 4 ? 0 : M <= 8 ? 1 : 2) + (x_f32 ? 3 : 0)];
+  const int tiles = ((N + 127) / 128) * ((M + kTok - 1) / kTok), nsb = K / UB_QK_K, sms = ub::num_sms(), ks = unit_split(tiles, nsb);
+  float us = c.fixed;
+  if (ks > 1) {
+    const float pairs = 2 * tiles * ks <= sms ? 0.f : tiles * ks <= sms ? .5f : 1.f;
+    us += c.split + (nsb + ks - 1) / ks * (c.one + pairs * (c.two - c.one));
+  } else {
+    const int full = tiles / (2 * sms), left = tiles % (2 * sms);
+    us += nsb * (full * c.two + (left == 0 ? 0.f : left <= sms ? c.one : c.two));
+  }
+  return us > 3.5f ? us : 3.5f;
+}
+
+// The same by the first fit (Q4_K, Q8_0; within 20 %): f32 results keep to the line that they were given, see few_tokens_route.
+float unit_us_f32_results(int type, int M, int N, int K, bool x_f32) {
   static const UnitCost q4k[6] = {{-.94f, 4.18f, 1.04f, 1.62f}, {-.86f, 3.89f, 1.15f, 1.75f}, {.43f, 3.48f, 1.55f, 2.17f},
                                   {-1.1f, 4.09f, 1.41f, 1.95f}, {-1.42f, 4.33f, 2.25f, 2.71f}, {-2.42f, 6.1f, 3.66f, 4.33f}};
   static const UnitCost q8[6] = {{-.7f, 3.21f, 1.35f, 1.82f}, {-.69f, 3.28f, 1.37f, 1.85f}, {.42f, 3.f, 1.55f, 2.11f},
@@ -1083,41 +1129,83 @@ float unit_us(int type, int M, int N, int K, bool x_f32) {
   return us > 3.5f ? us : 3.5f;
 }
 
+// us of a launch with two-piece weights, up to sixteen tokens (within 10 %).
+float two_piece_us(int type, int M, int N, int K, bool x_f32) {
+  struct Cost {
+    float fixed, step, step_f32;
+  };
+  const Cost c = type == 2    ? Cost{2.65f, 1.9f, 2.34f}
+                 : type == 13 ? Cost{2.95f, 2.02f, 2.3f}
+                 : type == 14 ? Cost{3.52f, 1.97f, 2.53f}
+                 : type == 8  ? Cost{2.6f, 1.95f, 2.55f}
+                              : Cost{2.4f, 1.77f, 2.2f};
+  const int tiles = (N + 127) / 128, nsb = K / UB_QK_K, ks = ub::two_piece_split(tiles, nsb), sms = ub::num_sms();
+  const int steps = (tiles * ks + sms - 1) / sms * ((nsb + ks - 1) / ks);
+  return c.fixed + (ks > 1 ? 1.3f : 0.f) + (x_f32 ? c.step_f32 : c.step) * steps + .02f * M * (N * (1.f / 1024.f));
+}
+
+// Q4_K and Q8_0: are two-piece weights faster than the decode kernels, where those need a second pass or have the CUDA-core kernels' time?
+// (f32 results stay with the CUDA-core kernels, which are the more exact ones.)
+bool two_piece_pays(int type, int M, int N, int K, bool x_f32, bool y_f32) {
+  const int pass = M < 8 ? M : 8, nsb = K / UB_QK_K;
+  if (type == 8) {
+    const bool quads_fit = K % 2048 == 0 && (pass + 3) / 4 * (K / UB_QK8_0) <= 568;  // in qgemv_imma.cu's shared memory
+    if (quads_fit ? M <= 8 : y_f32) return false;
+  } else {
+    const bool made_for = K == 2048 || K == 4096 || (K == 8192 && M > 4);  // qgemv_mt.cu, qgemv_mc.cu
+    const bool pairs_fit = (pass + 1) / 2 * nsb <= 70;  // token pairs of a whole row in qgemv_imma.cu's shared memory
+    if (y_f32 && !made_for && !pairs_fit) return false;
+    if (M <= 8 && (made_for || (M <= 4 && pairs_fit))) return false;
+  }
+  return 1.06f * two_piece_us(type, M, N, K, x_f32) < decode_us(type, M, N, K);
+}
+
 }  // namespace
 
 namespace ub {
 
-// Q4_K and Q8_0, up to sixteen tokens: this kernel or the decode kernels, both priced.
-// Where the decode kernels' results have bits that other calls share they stay unless they take 1.7 times as long: f32 results of five
-// tokens and more (passes of eight tokens and the rest are two calls), and the rows that qgemv_mc.cu is made for (a bf16
-// result is the f32 one rounded).
-bool unit_pays(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32) {
-  const bool mc = ggml_type == 12 && M <= 8 && (K == 2048 || K == 4096 || K == 8192);
-  return (M > 4 && (y_f32 || mc) ? 1.7f : 1.05f) * unit_us(ggml_type, M, N, K, x_f32) < decode_us(ggml_type, M, N, K);
+// Of 17300 calls of 1024 rows and values and more, timed without this kernel and with it, 213 take over 6 % longer with it: f32 results
+// that are more exact for it, and crossings that the lines miss by a tenth.  With thresholds on the sizes there were 477.
+//
+// Q4_K and Q8_0, up to sixteen tokens: 0 the decode kernels, 1 this kernel, 2 two-piece weights (nine f32 tokens and more, where three
+// pieces of an activation cost more than two of a weight: Q4_K sixteen tokens 8192x512 6.9 us there, 11.2 here).
+// 16-bit results: the fastest, this kernel from a tenth on.  The rows that qgemv_mc.cu is made for stay there unless it takes 1.7 times as
+// long (its bf16 result is its f32 one rounded).
+// f32 results: the kernels differ by 2.7e-5 (activations of 15 bits) against 1e-7 here, so a call does not go back to
+// the decode kernels for its time alone; where two-piece weights (2e-6 to 8e-6) would be faster than those, this kernel or they have
+// the call.  From five tokens on the decode kernels' results have bits that other calls share (passes of eight tokens and the
+// rest are two calls): they stay unless they take 1.7 times as long.
+int few_tokens_route(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32) {
+  const bool two = M > 4 && two_piece_pays(ggml_type, M, N, K, x_f32, y_f32);
+  const float decode = decode_us(ggml_type, M, N, K), unit = unit_us(ggml_type, M, N, K, x_f32);
+  const float two_us = two && x_f32 && M > 8 ? two_piece_us(ggml_type, M, N, K, x_f32) : kNever;
+  if (y_f32 && !(ggml_type == 8 && K % 2048)) {
+    if ((M > 4 ? 1.7f : 1.05f) * unit_us_f32_results(ggml_type, M, N, K, x_f32) < decode) return 1;
+    return !two ? 0 : two_us < unit ? 2 : 1;
+  }
+  if (two_us < unit && two_us < decode) return 2;
+  const bool mc = ggml_type == 12 && M > 4 && M <= 8 && (K == 2048 || K == 4096 || K == 8192);
+  return (mc ? 1.7f : 1.1f) * unit < decode ? 1 : 0;
 }
 
 // Q4_0, Q5_K and Q6_K: does this kernel take the call (instead of the staged kernels, qgemm_tc2.cu or the CUDA-core kernels)?
-// Measured on B200, us, before / this kernel, bf16 activations:
-//   rows that are not whole 2048 values  Q4_0 one token 4096x4352 24 / 8, Q5_K four 14336x3328 58 / 19, Q6_K eight 16384x5120 65 / 30;
-//     one token of Q6_K 14336x3328 20.8 / 22.9, 1024x5120 12.2 / 7.4
-//   whole 2048 values                    Q4_0 one token 28672x8192 33 / 43, 4096x14336 61 / 14, two 6144x4096 9.4 / 8.5; Q5_K one token
-//     4096x14336 16.6 / 18.4, 8192x28672 450 / 54, three 6144x4096 15 / 10.8, 512x2048 4.2 / 4.2; Q6_K two tokens 28672x8192 69 / 92,
-//     4096x14336 34 / 26, four 6144x4096 17.8 / 16, sixteen 6144x4096 27 / 16
-//   f32 activations, nine to sixteen tokens: 1024x5120 11.8 / 15.1 (three pieces here, two there), from there on this kernel
-//   f32 results of more tokens: Q4_0 32 tokens 11520x8960 2450 / 55, Q6_K 182 tokens 14976x3584 1594 / 198
+// f32 results of rows that the staged kernels take (15-bit activations, 2.7e-5) are this kernel's from where it was found the faster
+// one at three shapes; they do not go back for their time alone (Q6_K two tokens 2048x10240 11.2 there, 18.4 here).  f32 results of
+// one or two tokens of other Q6_K rows are the CUDA-core kernel's whatever the alignment of the weights.
+// f32 results of more tokens: Q4_0 32 tokens 11520x8960 2450 / 55, Q6_K 182 tokens 14976x3584 1594 / 198.
 bool unit_takes(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32) {
   const bool odd = K % 2048 != 0;
   if (M > 16) return y_f32 && (odd || K > 4096);
-  if (x_f32 && M > 8 && !y_f32 && K <= 5120) return false;
-  if (M > 4) return true;
-  switch (ggml_type) {
-    case 2: return odd || M >= 3 || K > 8192 || (M >= 2 && K >= 4096);
-    case 13: return odd || M >= 4 || K > 14336 || (M >= 2 && K >= 4096);
-    default:
-      // one or two tokens: f32 results are the CUDA-core kernel's whatever the alignment of the weights
-      if (odd) return M >= 3 || (!y_f32 && ((M == 2 && !x_f32) || (N <= 4096 && (M == 2 || !x_f32))));
-      return (M >= 2 && K > 8192) || (M >= 4 && K >= 4096);
+  if (M > 4)  // two-piece weights otherwise; with bf16 activations they are never the faster ones
+    return !(x_f32 && M > 8 && !y_f32) ||
+           1.05f * unit_us(ggml_type, M, N, K, x_f32) < two_piece_us(ggml_type, M, N, K, x_f32);
+  if (y_f32 && odd && ggml_type == 14 && M <= 2) return false;
+  if (y_f32 && !odd) {
+    if (ggml_type == 2) return M >= 3 || K > 8192 || (M >= 2 && K >= 4096);
+    if (ggml_type == 13) return M >= 4 || K > 14336 || (M >= 2 && K >= 4096);
+    return (M >= 2 && K > 8192) || (M >= 4 && K >= 4096);
   }
+  return 1.05f * unit_us(ggml_type, M, N, K, x_f32) < decode_us(ggml_type, M, N, K);
 }
 
 // May a launch request weights ahead of its dependency wait?  Only where every kernel that could have the call does: a caller

@@ -5,7 +5,7 @@
 // fits, batched kernel otherwise).  The same idea here is a split on M:
 //   M = 1             one-token decode kernels (qgemv_m1.cu, qgemv_q8_m1.cu), any whole super-blocks per row;
 //   M <= 16           integer decode kernels in passes of up to eight tokens (qgemv.cu), or the tensor-core kernel of the
-//                     weights' integers in one pass (qgemm_unit.cu; the line: unit_pays); from M = 9 on Q4_K with
+//                     weights' integers in one pass (qgemm_unit.cu) or, with f32 ones, of two-piece weights (qgemm_tc2.cu; the line: few_tokens_route); from M = 9 on Q4_K with
 //                     bf16 activations AND bf16 output takes the one-piece tensor-core kernels.  No workspace;
 //   M  > 16, Q4_K     tcgen05 tensor-core GEMM with in-kernel dequantisation, one piece (qgemm_tc2.cu while one round of CTAs
 //                     holds all 128-token tiles, qgemm_tc.cu beyond; bf16 activations and output, other types are
@@ -38,7 +38,9 @@ void* tensor_map_encoder();
 int q4k_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
 int gguf_gemm_unit(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
                    bool fresh, cudaStream_t s);
-bool unit_pays(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32);
+int gguf_gemm_tc2(int ggml_type, void* y, int y_dtype, const void* x, bool x_f32, const void* wq, int M, int N, int K,
+                  bool fresh, cudaStream_t s);
+int few_tokens_route(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32);
 int q8_0_gemm_tc(void* y, const void* x, const void* wq, int M, int N, int K, bool fresh, cudaStream_t s);
 }  // namespace ub
 
@@ -254,11 +256,15 @@ int qmatmul(bool is_q4k, int x_dtype, void* y, const void* x, const void* wq, in
     if (st != UB_ERR_UNSUPPORTED) return st;  // unsupported shape or driver: the decode kernel below
   }
   // Up to sixteen tokens: the tensor-core kernel of the integers (one pass for all of them, f32 rounding only: 1e-7 of a result,
-  // 2-norm) or the decode kernels (passes of up to eight; integer ones 2.8e-5, CUDA-core ones 1e-7 to 3e-5), whichever is the
-  // faster one.  One token of Q4_K, and of Q8_0 with rows of whole 2048 values, has kernels of its own.
-  if (M <= kDecodeMaxM && (M >= 2 || (!is_q4k && K % 2048 != 0)) && K % UB_QK_K == 0 &&
-      ub::unit_pays(is_q4k ? 12 : 8, M, N, K, x_dtype == UB_DTYPE_F32, out_dtype == UB_DTYPE_F32)) {
-    const int st = ub::gguf_gemm_unit(is_q4k ? 12 : 8, y, out_dtype, x, x_dtype == UB_DTYPE_F32, wq, M, N, K, fresh, s);
+  // 2-norm), the one with two-piece weights (2e-6 to 8e-6) or the decode kernels (passes of up to eight; integer ones 2.8e-5, CUDA-core
+  // ones 1e-7 to 3e-5).  One token of Q4_K, and of Q8_0 with rows of whole 2048 values, has kernels of its own.
+  if (M <= kDecodeMaxM && (M >= 2 || (!is_q4k && K % 2048 != 0)) && K % UB_QK_K == 0) {
+    const int tag = is_q4k ? 12 : 8;
+    const bool x_f32 = x_dtype == UB_DTYPE_F32;
+    const int route = ub::few_tokens_route(tag, M, N, K, x_f32, out_dtype == UB_DTYPE_F32);
+    const int st = route == 1   ? ub::gguf_gemm_unit(tag, y, out_dtype, x, x_f32, wq, M, N, K, fresh, s)
+                   : route == 2 ? ub::gguf_gemm_tc2(tag, y, out_dtype, x, x_f32, wq, M, N, K, fresh, s)
+                                : UB_ERR_UNSUPPORTED;
     if (st != UB_ERR_UNSUPPORTED) return st;
   }
   auto decode = [&]() {
