@@ -99,11 +99,12 @@ __device__ __forceinline__ int lds_s8(uint32_t a) {
 //
 // One piece of Q4_K: low nibbles as q 2^-133, high ones as 16 q 2^-133, and a scale that carries the rest, finite in bf16 while a
 // super-block's d is below this (63 * 2^-11 * 2^133 < 2^128; trained weights have d of 1e-5 to 4e-4).  Where a row of the warp has a
-// larger one, the nibbles are multiplied by 2^127 first, exactly: two instructions more per four values.  Both give bf16(s q - m), s
-// and m rounded to bf16, and accumulators of ordinary size: with a factor on all weights instead, taken back from the sums, products of
-// activations below 2^-92 would be subnormal.  Low nibbles moved up by four bits would do until 2^-7: 0.7 % of an expert layer of
-// 256 tokens, 0.9 % of sixteen tokens through a wide block.
-constexpr float kOnePieceMaxD = 0x1p-11f;
+// larger one, the nibbles are multiplied by 2^127 first, exactly: two instructions more per four values, up to 10 % of a launch.
+// Both give bf16(s q - m), s and m rounded to bf16, and accumulators of ordinary size: with a factor on all weights instead, taken back
+// from the sums, products of activations below 2^-92 would be subnormal.  The choice costs 0 to 1.5 % (expert layers of a few hundred
+// rows per expert most), and 3 % when made anew for each nibble half and from the f32 scale.  Low nibbles moved up by four bits
+// would do until 2^-7, for another 0.7 %.
+constexpr uint32_t kOnePieceMaxD = 0x1000;  // 2^-11 in f16
 
 template <int FMT>
 struct RowBlock {
@@ -119,7 +120,7 @@ struct RowBlock {
       lds128(base, h);
       d = half_bits_to_f32(h[0]), dmin = half_bits_to_f32(h[0] >> 16);
       q4k_unpack_scales(h[1], h[2], h[3], scw[0], scw[1], mnw[0], mnw[1]);
-      if constexpr (FMT == kQ4K) wide = __any_sync(0xFFFFFFFFu, !(fabsf(d) < kOnePieceMaxD));
+      if constexpr (FMT == kQ4K) wide = __any_sync(0xFFFFFFFFu, (h[0] & 0x7FFFu) >= kOnePieceMaxD);
       if constexpr (FMT == kQ5K) lds128(base + 16, fifth), lds128(base + 32, fifth + 4);  // of all eight sub-blocks
     }
     if constexpr (FMT == kQ6K) d = half_bits_to_f32(lds32((base + 208) & ~3u) >> ((base & 2) * 8));
@@ -150,21 +151,25 @@ struct RowBlock {
     if constexpr (FMT == kQ4K) {
       uint32_t q[8];
       lds128(base + 16 + 32 * G, q), lds128(base + 32 + 32 * G, q + 4);
+      if (__builtin_expect(!wide, 1)) {
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        float s, m;
-        pair(2 * G + h, s, m);
-        const __nv_bfloat162 ndm = __float2bfloat162_rn(-m);
-        if (!wide) {
-          const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 0x1p65f : 0x1p69f) * 0x1p64f);
+        for (int h = 0; h < 2; h++) {
+          float s, m;
+          pair(2 * G + h, s, m);
+          const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 0x1p65f : 0x1p69f) * 0x1p64f), ndm = __float2bfloat162_rn(-m);
 #pragma unroll
           for (int i = 0; i < 8; i++) {
             const uint32_t v = q[i] & (h ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
             ot[16 * h + 2 * i] = deq_pair<0x4140>(v, dsc, ndm);
             ot[16 * h + 2 * i + 1] = deq_pair<0x4342>(v, dsc, ndm);
           }
-        } else {
-          const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 4.f : 64.f));
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float s, m;
+          pair(2 * G + h, s, m);
+          const __nv_bfloat162 dsc = __float2bfloat162_rn(s * (h ? 4.f : 64.f)), ndm = __float2bfloat162_rn(-m);
 #pragma unroll
           for (int i = 0; i < 8; i++) {
             const uint32_t v = q[i] & (h ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
