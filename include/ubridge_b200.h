@@ -155,10 +155,9 @@ int ub_repack_to_interleaved(void* interleaved, const void* split, size_t nblock
  * output and embedding matrices in it.  Blocks are interleaved as in a .gguf file, 2-byte aligned.
  * ub_dequant_q6k: the f32 value (d*scale)*(q-32) rounded once to out_dtype, bit-exact.
  * ub_qmatmul_q6k_*: y[M,N] = x[M,K] . W^T with W = N rows of K/256 blocks, f32 accumulation, a
- * weight-streaming decode kernel that takes the tokens four at a time (any M, no workspace), or, from two tokens on (and for one
- * in rows that are not whole 2048 values) where they are the faster ones and as exact, tensor-core kernels that take them all.  With K a multiple of 2048 (up to 14336 for
- * one token) and 16-byte aligned wq these kernels request their first weights before they wait for the kernel in front of
- * them on the stream: the precondition on the weights and UB_QMATMUL_WEIGHTS_FRESH (below, ORed into out_dtype) apply to
+ * weight-streaming decode kernel that takes the tokens four at a time (any M, no workspace), or, where they are the faster ones and
+ * as exact, tensor-core kernels that take them all.  With K a multiple of 2048 (up to 14336 for one token) and 16-byte aligned
+ * wq these kernels request their first weights before they wait for the kernel in front of them on the stream: the precondition on the weights and UB_QMATMUL_WEIGHTS_FRESH (below, ORed into out_dtype) apply to
  * them as to ub_qmatmul_*. */
 int ub_dequant_q6k(void* out, const void* blocks, size_t numel, int out_dtype, void* stream);
 int ub_qmatmul_q6k_f32(void* y, const void* x, const void* wq, int M, int N, int K, int out_dtype, void* stream);
@@ -177,6 +176,10 @@ int ub_qmatmul_q6k_bf16(void* y, const void* x, const void* wq, int M, int N, in
  * activation or output type is not bf16 (0 whenever M <= 16).  Q8_0 takes the tensor-core kernel when
  * K % 256 == 0 and wq is 16-byte aligned; otherwise, or when called without the scratch, it runs the
  * decode kernel in passes of eight tokens (same result within the matmul tolerance, slower).
+ *
+ * Activations that are not finite: that token's results are not finite, other tokens are not touched.  f32 results that run on
+ * CUDA cores or on the tensor-core kernel of the weights' integers (rows that are not whole 2048 values among them) give an
+ * infinity with its sign where the plain sum does; fixed-point decode kernels (15-bit activations) and two-piece weights give NaN.
  *
  * Precondition on the weights.  The decode kernels (M <= 16) and the tensor-core kernel up to 64 tokens are
  * launched with programmatic dependent launch

@@ -7,8 +7,9 @@
 // s * u + b, u a small integer, s and b the group's own: the sum over the group is s * sum(u x) + b * sum(x).  The integers go
 // to the tensor cores as bf16 (exact), every group has an accumulator of its own, and s and b are applied in f32 to the
 // groups' sums.  Activations are exact too: bf16 ones come as they are, f32 ones in three bf16 pieces (24 bits), so results
-// carry f32 rounding only: 0.8e-7 to 1.2e-7 of a result as a 2-norm, 256 to 14336 values (CUDA-core kernels 0.7e-7 to 3.8e-7,
-// integer kernels with 15-bit activations 2.8e-5, two-piece weights 2e-6 to 2.6e-5).
+// carry f32 rounding only: 0.5e-7 to 1.2e-7 of a result as a 2-norm, 256 to 14336 values (CUDA-core kernels 0.6e-7 to 3.9e-7,
+// integer kernels with 15-bit activations 2.8e-5, two-piece weights 2e-6 to 2.6e-5).  An infinite activation gives what the plain
+// sum gives (sum_of_infinities), a NaN gives NaN.
 //
 // u is centred (Q4_K and Q4_0 q - 8, Q5_K q - 16, Q6_K q - 32, Q8_0 signed): small sums lose least when a result is small, and
 // Q4_0, Q6_K and Q8_0 have no second term.  The tensor cores get 2^-8 u, so that sums of large activations do not
@@ -27,11 +28,12 @@
 //
 // What bounds it: the sums' chain, 2100 cycles per super-block and CTA with four tokens (two barriers 500, scales and offsets
 // 600, two reads of tensor memory 700), two CTAs per SM, where the copies of a super-block take 790 cycles of an SM's share of
-// the memory and the integers 570.  Measured on B200, us, before / this kernel: Q4_K four tokens 4096x14336 30.6 / 15.1, Q8_0 four
-// 6144x5120 76 / 12.5, Q5_K ten tokens, f32 results, 2688x7680 284 / 13.8.
+// the memory and the integers 570.  The variants of sixteen tokens also spill registers (60 to 206 bytes a thread).
+// Measured on B200, us, before / this kernel: Q4_K four tokens 4096x14336 30.6 / 15.1, Q8_0 four 6144x5120 76 / 12.5, Q5_K ten
+// tokens, f32 results, 2688x7680 284 / 13.8.
 //
 // K split.  A tile may belong to a cluster of up to eight CTAs, each with a part of K.  Every CTA owns some of the 128 rows
-// and gets the others' partial sums of them (st.async, counted in bytes on a barrier of the owner); it adds them in rank
+// and gets the others' partial sums of them (st.async, counted in bytes on a barrier of the owner); it adds them in a fixed
 // order: deterministic.
 //
 // Every wait is bounded; on expiry the CTA records UB_ERR_TIMEOUT, all roles leave and TMEM is freed.

@@ -3,9 +3,11 @@
 // The reference picks a matmul variant per shape with AtenGemmTuner (src/gemm_tuner.rs:326-359,
 // small-M special cases :502-514) and kernels/matmul.cpp:1197-1208 (LHS-resident decode kernel when it
 // fits, batched kernel otherwise).  The same idea here is a split on M:
-//   M = 1             one-token decode kernels (qgemv_m1.cu, qgemv_q8_m1.cu), any whole super-blocks per row;
-//   M <= 16           integer decode kernels in passes of up to eight tokens (qgemv.cu), or the tensor-core kernel of the
-//                     weights' integers in one pass (qgemm_unit.cu) or, with f32 ones, of two-piece weights (qgemm_tc2.cu; the line: few_tokens_route); from M = 9 on Q4_K with
+//   M = 1             one-token decode kernels (qgemv_m1.cu, qgemv_q8_m1.cu), any whole super-blocks per row (Q8_0: rows of whole
+//                     2048 values; others as below);
+//   M <= 16           integer decode kernels in passes of up to eight tokens (qgemv.cu), the tensor-core kernel of the
+//                     weights' integers in one pass (qgemm_unit.cu) or, for nine f32 tokens and more, the one of two-piece weights
+//                     (qgemm_tc2.cu; the line: few_tokens_route); from M = 9 on Q4_K with
 //                     bf16 activations AND bf16 output takes the one-piece tensor-core kernels.  No workspace;
 //   M  > 16, Q4_K     tcgen05 tensor-core GEMM with in-kernel dequantisation, one piece (qgemm_tc2.cu while one round of CTAs
 //                     holds all 128-token tiles, qgemm_tc.cu beyond; bf16 activations and output, other types are
