@@ -71,9 +71,10 @@ constexpr int threads_of(bool xf) { return (xf ? 17 : 16) * 32; }
 constexpr uint32_t kRecvBytes = (128 + 8) * kTok * 4;
 // Rounding.  A chain of n additions rounds n / 2 times as much as one.  Without an offset a stage of four groups is summed by itself,
 // then the stages of a super-block, then super-blocks.  Q6_K has twice the groups, and what an addition of a super-block
-// rounds off is summed beside it, in shared memory (in registers it would spill: 9 % of sixteen tokens, 13 % of eight in f32; so 1 to
-// 6 %).  Error of f32 results as a part of the CUDA-core kernels', bf16 activations: Q6_K 1200 rows of 1536 values 0.98 (1.20 in one
-// chain per super-block), 24000 rows of 4352 values 0.75 (1.14 without the rest), Q8_0 1024 values 0.97 (1.04 in one chain).
+// rounds off is summed beside it, in shared memory (in registers it would spill more).  Q6_K takes longer for it: four tokens 1 %, eight
+// 3 to 5 %, sixteen 2 to 13 % (28672x5120 65.7 -> 70.7 us).  Error of f32 results as a part of the CUDA-core kernels', bf16
+// activations: Q6_K 1200 rows of 1536 values 0.98 (1.20 in one chain per super-block), 24000 rows of 4352 values 0.75 (1.14 without
+// the rest), Q8_0 1024 values 0.97 (1.04 in one chain).
 constexpr bool keeps_stages(int f) { return f == kQ6K || f == kQ8; }
 constexpr bool keeps_rest(int f) { return f == kQ6K; }
 constexpr uint32_t rest_bytes(int f) { return keeps_rest(f) ? 128 * kTok * 4 : 0; }
@@ -660,22 +661,21 @@ qgemm_unit_kernel(void* __restrict__ y, int y_dtype, const void* __restrict__ x,
       if (!ok) break;
       for (int i = row; i < mine * (TT / 4); i += 128) {
         const int q = i / mine, l = i - q * mine, out = n0 + tile_row(FMT, first + l);
-        auto rank = [&](int r) {
-          return *reinterpret_cast<const float4*>(tiles + kRecvOff + ((r * (TT / 4) + q) * own + l) * 16);
-        };
-        auto add = [](float4& a, const float4& b) { a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w; };
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int r = 0; r < KS; r += 4) {  // pairs of pairs: a chain of eight would round more
-          float4 u = rank(r);
-          if (r + 1 < KS) add(u, rank(r + 1));
-          if (r + 2 < KS) {
-            float4 v = rank(r + 2);
-            if (r + 3 < KS) add(v, rank(r + 3));
-            add(u, v);
+        // In rank order; Q6_K, where it shows, even and odd ranks by themselves (pairs of pairs in all formats took registers from the
+        // loop above: 28672x5120, sixteen tokens, Q4_K 44.3 -> 48.2 us, Q6_K 71 -> 77).
+        float f[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int r = 0; r < KS; r += kRest ? 2 : 1) {
+          const unsigned char* const part_r = tiles + kRecvOff + ((r * (TT / 4) + q) * own + l) * 16;
+          const float4 p = *reinterpret_cast<const float4*>(part_r);
+          f[0] += p.x, f[1] += p.y, f[2] += p.z, f[3] += p.w;
+          if (kRest && r + 1 < KS) {
+            const float4 p1 = *reinterpret_cast<const float4*>(part_r + (TT / 4) * own * 16);
+            odd[0] += p1.x, odd[1] += p1.y, odd[2] += p1.z, odd[3] += p1.w;
           }
-          add(sum, u);
         }
-        const float f[4] = {sum.x, sum.y, sum.z, sum.w};
+        if (kRest)
+#pragma unroll
+          for (int t = 0; t < 4; t++) f[t] += odd[t];
         if (out < N) {
 #pragma unroll
           for (int t = 0; t < 4; t++)
@@ -1166,7 +1166,7 @@ bool two_piece_pays(int type, int M, int N, int K, bool x_f32, bool y_f32) {
 
 namespace ub {
 
-// Of 17300 calls of 1024 rows and values and more, timed without this kernel and with it, 213 take over 6 % longer with it: f32 results
+// Of 17300 calls of 1024 rows and values and more, timed without this kernel and with it, 200 take over 6 % longer with it: f32 results
 // that are more exact for it, and crossings that the lines miss by a tenth.  With thresholds on the sizes there were 477.
 //
 // Q4_K and Q8_0, up to sixteen tokens: 0 the decode kernels, 1 this kernel, 2 two-piece weights (nine f32 tokens and more, where three
