@@ -29,8 +29,8 @@
 // What bounds it: the sums' chain, 2100 cycles per super-block and CTA with four tokens (two barriers 500, scales and offsets
 // 600, two reads of tensor memory 700), two CTAs per SM, where the copies of a super-block take 790 cycles of an SM's share of
 // the memory and the integers 570.  The variants of sixteen tokens also spill registers (60 to 206 bytes a thread).
-// Measured on B200, us, before / this kernel: Q4_K four tokens 4096x14336 30.6 / 15.1, Q8_0 four 6144x5120 76 / 12.5, Q5_K ten
-// tokens, f32 results, 2688x7680 284 / 13.8.
+// Measured on B200, us, before / this kernel: Q4_K four tokens 4096x14336 30.6 / 15.4, Q8_0 four 6144x5120 76 / 12.2, Q5_K ten
+// tokens, f32 results, 2688x7680 284 / 15.1.
 //
 // K split.  A tile may belong to a cluster of up to eight CTAs, each with a part of K.  Every CTA owns some of the 128 rows
 // and gets the others' partial sums of them (st.async, counted in bytes on a barrier of the owner); it adds them in a fixed
@@ -1192,9 +1192,9 @@ int few_tokens_route(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32)
 
 // Q4_0, Q5_K and Q6_K: does this kernel take the call (instead of the staged kernels, qgemm_tc2.cu or the CUDA-core kernels)?
 // f32 results of rows that the staged kernels take (15-bit activations, 2.7e-5) are this kernel's from where it was found the faster
-// one at three shapes; they do not go back for their time alone (Q6_K two tokens 2048x10240 11.2 there, 18.4 here).  f32 results of
+// one at three shapes; they do not go back for their time alone (Q6_K two tokens 2048x10240 11.2 there, 17.4 here).  f32 results of
 // one or two tokens of other Q6_K rows are the CUDA-core kernel's whatever the alignment of the weights.
-// f32 results of more tokens: Q4_0 32 tokens 11520x8960 2450 / 55, Q6_K 182 tokens 14976x3584 1594 / 198.
+// f32 results of more tokens: Q4_0 32 tokens 11520x8960 2450 / 55, Q6_K 182 tokens 14976x3584 1594 / 229.
 bool unit_takes(int ggml_type, int M, int N, int K, bool x_f32, bool y_f32) {
   const bool odd = K % 2048 != 0;
   if (M > 16) return y_f32 && (odd || K > 4096);
